@@ -392,6 +392,7 @@ meso_status meso_scene_load(meso_ctx* ctx, const char* path, uint64_t spare, mes
     return cuda_fail(e, "scene_load: upload");
   }
   meso_status rc = rebuild_macro(ctx, s, nullptr, 0, ctx->stream);
+  if (rc == MESO_OK) rc = rebuild_sub(ctx, s, n, ctx->stream);
   if (rc == MESO_OK) {
     e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) rc = cuda_fail(e, "scene_load: macro map");

@@ -83,6 +83,13 @@ struct meso_scene {
   uint8_t* d_macro2 = nullptr;
   // one byte per 64x64x64-brick cell (512^3 voxels), built like d_macro2 from it
   uint8_t* d_macro3 = nullptr;
+  // Derived maps of the raymarch's region walk (9 bytes per 4x4x4-brick cell
+  // and 8 per pool slot, under 1 % of the scene; not part of `bytes`, so that
+  // a budget admits what it did without them):
+  uint8_t* d_level = nullptr;  // per 4x4x4-brick cell: 0 if occupied, else log2 of the edge in voxels of the
+                               // largest aligned empty cube it is part of (5 .. 9)
+  uint64_t* d_mask = nullptr;  // per 4x4x4-brick cell: its occupied bricks, bit x + 4y + 16z
+  uint64_t* d_sub = nullptr;   // per pool slot: the non-empty 2x2x2-voxel blocks, bit x + 4y + 16z
   uint64_t capacity = 0;       // pool slots
   // allocator state (device): [0] bump (slots ever used), [1] free-stack top
   int64_t* d_alloc = nullptr;
@@ -112,13 +119,14 @@ inline cudaStream_t pick_stream(meso_ctx* ctx, void* s) {
 meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint64_t capacity,
                         meso_scene** out);
 void scene_release(meso_ctx* ctx, meso_scene* s);
-// Recomputes the macro-cell map of a scene from its pointer grid: all cells,
-// or the n cells listed in d_cells (linear macro-cell indices).
-// Recomputes the cell maps: every cell (lists null), or the listed cells of
-// 4^3, 16^3 and 64^3 bricks (each list sorted unique, children before parents).
+// Recomputes the cell maps (occupancy bytes, brick masks, level bytes): every
+// cell (lists null), or the listed cells of 4^3, 16^3 and 64^3 bricks (each
+// list sorted unique, children before parents).
 meso_status rebuild_macro(meso_ctx* ctx, meso_scene* s, const uint32_t* d_cells, uint32_t n, cudaStream_t st,
                           const uint32_t* d_cells2 = nullptr, uint32_t n2 = 0, const uint32_t* d_cells3 = nullptr,
                           uint32_t n3 = 0);
+// Recomputes d_sub of the first `slots` pool slots from their occupancy.
+meso_status rebuild_sub(meso_ctx* ctx, meso_scene* s, uint64_t slots, cudaStream_t st);
 
 // Kernel launchers (defined in the .cu files).
 // chunk_id_base: added to the list index in each quad's chunk field (the

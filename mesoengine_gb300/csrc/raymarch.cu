@@ -14,6 +14,7 @@
 // t = (b - o) * (1/d), with correctly rounded single operations
 // (__fsub_rn/__fmul_rn...) so the results are bit-identical to a host
 // evaluation of the same sequence.  Equal boundary times break x < y < z.
+#include <cmath>
 #include <cstring>
 
 #include "meso_internal.h"
@@ -24,9 +25,9 @@ struct RayView {
   const uint32_t* ptr;
   const uint64_t* occ;
   const uint16_t* mat;
-  const uint8_t* macro;   // per 4x4x4-brick cell: nonzero iff a brick of it is occupied
-  const uint8_t* macro2;  // per 16x16x16-brick cell: nonzero iff a 4x4x4 cell of it is, or it leaves the grid
-  const uint8_t* macro3;  // per 64x64x64-brick cell, likewise from the 16x16x16 cells
+  const uint8_t* level;  // per 4x4x4-brick cell: log2 of the edge (voxels) of the largest aligned empty cube it is part of, 0 if it is not empty
+  const uint64_t* mask;  // per 4x4x4-brick cell: its occupied bricks, bit x + 4y + 16z
+  const uint64_t* sub;   // per pool slot: the brick's non-empty 2x2x2-voxel blocks, bit x + 4y + 16z
   int32_t nx, ny, nz;
   int32_t cam_chunk[3];
   float o[3];
@@ -74,6 +75,7 @@ struct RayParams {
   unsigned long long* hash;  // checksum instantiation: partial sums per view (see launch_raymarch)
   uint32_t order_mul;  // CTA b takes block (b * order_mul) mod gridDim.x (0: block b)
   uint32_t cta_rows;   // 1: the output is host memory; write whole CTA rows (see the kernel)
+  float margin;        // region walk: distance (voxels) at which a position estimate settles a boundary; 0: step by step
 };
 
 struct Trav {
@@ -81,6 +83,7 @@ struct Trav {
   int vx, vy, vz;
   float t;
   int axis;
+  uint32_t slot;  // pool slot of the brick that was hit
   uint32_t coarse, fine;
   uint32_t fetches, bricks;  // pointer fetches and occupied bricks entered (statistics only)
 };
@@ -91,209 +94,75 @@ __device__ __forceinline__ float bound_time(int b, float o, float inv) {
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
-// Brick steps the two-level DDA takes along a non-exit axis (sign s, brick
-// B, next brick boundary nb) while it crosses an empty cell of (mask+1)^3
-// bricks, up to the step that leaves the cell through another axis at time
-// tE (c_first: this axis wins ties with the exit axis).  The DDA takes its
-// boundary events in (time, axis x<y<z) order and one axis's events come at
-// strictly increasing times, so these steps are the interior boundaries that
-// precede the exit in that order: a prefix.  Its length is estimated from the
-// position at tE and settled by exact boundary-time comparisons.
-__device__ __forceinline__ int cell_steps(int s, int B, int mask, int nb, float o, float d, float inv, float tE,
-                                          bool c_first) {
-  if (s == 0) return 0;
-  const int inner = s > 0 ? mask - (B & mask) : (B & mask);
-  if (inner == 0) return 0;
-  const float pos = __fmaf_rn(d, tE, o);  // an estimate only
-  const float q = s > 0 ? __fsub_rn(pos, __int2float_rn(nb)) : __fsub_rn(__int2float_rn(nb), pos);
-  int k = clampi((int)ceilf(__fmul_rn(q, 0.125f)), 0, inner);
-  while (k > 0) {
-    const float tj = bound_time(nb + 8 * s * (k - 1), o, inv);
-    if (tj < tE || (tj == tE && c_first)) break;
-    k--;
-  }
-  while (k < inner) {
-    const float tj = bound_time(nb + 8 * s * k, o, inv);
-    if (!(tj < tE || (tj == tE && c_first))) break;
-    k++;
-  }
-  return k;
-}
-
-// Empty-cell level of brick B: 3 if its 64^3-brick cell is empty, 2 if its
-// 16^3-brick cell is, 1 if its 4^3-brick cell is, else 0 (the three bytes
-// are fetched together).
-__device__ __forceinline__ int cell_level(const RayView& V, int Bx, int By, int Bz, int MX, int MY, int MX2, int MY2,
-                                          int MX3, int MY3) {
-  const uint8_t m3 = __ldg(V.macro3 + (Bx >> 6) + MX3 * ((By >> 6) + MY3 * (Bz >> 6)));
-  const uint8_t m2 = __ldg(V.macro2 + (Bx >> 4) + MX2 * ((By >> 4) + MY2 * (Bz >> 4)));
-  const uint8_t m1 = __ldg(V.macro + (Bx >> 2) + MX * ((By >> 2) + MY * (Bz >> 2)));
-  return m3 == 0 ? 3 : (m2 == 0 ? 2 : (m1 == 0 ? 1 : 0));
-}
-
-// Walks from voxel (vx,vy,vz) (absolute, inside the grid) at time t, entered
-// through axis ea (-1 none).  Ray coordinates are relative to the absolute
-// voxel (bx0,by0,bz0); ix, iy, iz are 1/d per axis (0 where d is 0).
-//
-// The walk is the same sequence of float operations as a step-by-step
-// recomputation, organised for issue efficiency: a boundary time is only
-// recomputed for the axis that stepped (the others are unchanged values),
-// the entry voxel of a brick is derived only when an occupied brick is
-// reached, the pointer index is stepped incrementally, and the occupancy
-// word of the current z layer stays in a register.
+// ------------------------------------------------------- step by step
+// The walk as it is defined, from voxel (vx,vy,vz) (absolute, inside the
+// grid) at time t, entered through axis ea (-1 none).  Ray coordinates are
+// relative to the absolute voxel (bx0,by0,bz0); ix, iy, iz are 1/d per axis
+// (0 where d is 0).  A step cap ends the walk of a ray that makes no
+// progress (a direction of zeros or NaNs).  The statistics instantiation
+// takes this path to count its fetches, and so does any ray whose values lie
+// outside what the region walk below was proven for.
 template <bool kStats>
-__device__ __forceinline__ void traverse(const RayView& V, int bx0, int by0, int bz0, float ox, float oy, float oz,
-                                         float dx, float dy, float dz, float ix, float iy, float iz, int vx, int vy,
-                                         int vz, float t, int ea, Trav& r) {
+__device__ __noinline__ void walk_steps(const RayView& V, int bx0, int by0, int bz0, float ox, float oy, float oz,
+                                        float dx, float dy, float dz, float ix, float iy, float iz, int vx, int vy,
+                                        int vz, float t, int ea, Trav& r) {
   uint32_t n_fetch = 0, n_brick = 0;
   const int sx = dx > 0.0f ? 1 : (dx < 0.0f ? -1 : 0);
   const int sy = dy > 0.0f ? 1 : (dy < 0.0f ? -1 : 0);
   const int sz = dz > 0.0f ? 1 : (dz < 0.0f ? -1 : 0);
   const int px = sx > 0 ? 1 : 0, py = sy > 0 ? 1 : 0, pz = sz > 0 ? 1 : 0;
   const int NBx = V.nx >> 3, NBy = V.ny >> 3, NBz = V.nz >> 3;
-  const int MX = NBx >> 2, MY = NBy >> 2;                  // cells of 4x4x4 bricks
-  const int MX2 = (NBx + 15) >> 4, MY2 = (NBy + 15) >> 4;  // cells of 16x16x16 bricks
-  const int MX3 = (NBx + 63) >> 6, MY3 = (NBy + 63) >> 6;  // cells of 64x64x64 bricks
-  const uint32_t strideY = (uint32_t)NBx, strideZ = (uint32_t)NBx * (uint32_t)NBy;
-  // signed index increments of one step along each axis
-  const uint32_t dIx = (uint32_t)sx, dIy = (uint32_t)(sy * (int)strideY), dIz = (uint32_t)(sz * (int)strideZ);
   int Bx = vx >> 3, By = vy >> 3, Bz = vz >> 3;
-  uint32_t idx = (uint32_t)Bx + strideY * (uint32_t)By + strideZ * (uint32_t)Bz;
   uint32_t cs = 0, fs = 0;
   const uint32_t cap = (uint32_t)(4 * (V.nx + V.ny + V.nz) + 64);
+  uint32_t p = MESO_EMPTY_BRICK;
   r.hit = 0;
   for (;;) {
     if (cs + fs > cap) break;
-    uint32_t p = __ldg(V.ptr + idx);
+    p = __ldg(V.ptr + (uint32_t)Bx + (uint32_t)NBx * ((uint32_t)By + (uint32_t)NBy * (uint32_t)Bz));
     if (kStats) {
       n_fetch++;
       n_brick += p != MESO_EMPTY_BRICK;
     }
-    if (p == MESO_EMPTY_BRICK) {
-      // ---- coarse: one step per empty brick; nb* = next brick boundary
-      // (relative voxel coordinate) along each axis.  A cell of 4x4x4 empty
-      // bricks is crossed in one jump (the timed kernel; the statistics
-      // instantiation takes every brick step to count the fetches).
-      int nbx = (Bx + px) * 8 - bx0, nby = (By + py) * 8 - by0, nbz = (Bz + pz) * 8 - bz0;
-      float tx = sx ? bound_time(nbx, ox, ix) : kInf;
-      float ty = sy ? bound_time(nby, oy, iy) : kInf;
-      float tz = sz ? bound_time(nbz, oz, iz) : kInf;
-      bool out = false;
-      int a = ea;
-      // cell level at the current brick: 3 / 2 / 1 = its 64^3- / 16^3- /
-      // 4^3-brick cell is empty (the largest such), 0 = take brick steps
-      int lvl = 0;
-      if (!kStats) lvl = cell_level(V, Bx, By, Bz, MX, MY, MX2, MY2, MX3, MY3);
-      bool stale = false;
-      for (;;) {
-        if (lvl) {
-          const int sh = 2 * lvl, mask = (1 << sh) - 1;
-          const float Tx = sx ? bound_time((((Bx >> sh) + px) << (sh + 3)) - bx0, ox, ix) : kInf;
-          const float Ty = sy ? bound_time((((By >> sh) + py) << (sh + 3)) - by0, oy, iy) : kInf;
-          const float Tz = sz ? bound_time((((Bz >> sh) + pz) << (sh + 3)) - bz0, oz, iz) : kInf;
-          const bool my = Ty < Tx;
-          float tE = my ? Ty : Tx;
-          const bool mz = Tz < tE;
-          tE = mz ? Tz : tE;
-          const int aE = mz ? 2 : (my ? 1 : 0);
-          // along the exit axis every brick up to the face, then the exit step
-          const int Be = aE == 0 ? Bx : (aE == 1 ? By : Bz), se = aE == 0 ? sx : (aE == 1 ? sy : sz);
-          const int ke = (se > 0 ? mask - (Be & mask) : (Be & mask)) + 1;
-          const int kx = aE == 0 ? ke : cell_steps(sx, Bx, mask, nbx, ox, dx, ix, tE, true);
-          const int ky = aE == 1 ? ke : cell_steps(sy, By, mask, nby, oy, dy, iy, tE, aE == 2);
-          const int kz = aE == 2 ? ke : cell_steps(sz, Bz, mask, nbz, oz, dz, iz, tE, false);
-          const uint32_t k = (uint32_t)(kx + ky + kz);
-          if (cs + fs + k <= cap) {
-            cs += k;
-            t = tE;
-            a = aE;
-            Bx += sx * kx;
-            By += sy * ky;
-            Bz += sz * kz;
-            idx += dIx * (uint32_t)kx + dIy * (uint32_t)ky + dIz * (uint32_t)kz;
-            nbx += 8 * sx * kx;
-            nby += 8 * sy * ky;
-            nbz += 8 * sz * kz;
-            stale = true;  // brick boundary times: recomputed if a brick step follows
-            out = ((unsigned)Bx >= (unsigned)NBx) | ((unsigned)By >= (unsigned)NBy) | ((unsigned)Bz >= (unsigned)NBz);
-            if (out || cs + fs > cap) break;
-            p = __ldg(V.ptr + idx);
-            lvl = cell_level(V, Bx, By, Bz, MX, MY, MX2, MY2, MX3, MY3);
-            if (p != MESO_EMPTY_BRICK) break;
-            continue;
-          }
-          lvl = 0;  // the jump would pass the step cap: take brick steps
-        }
-        if (stale) {
-          tx = sx ? bound_time(nbx, ox, ix) : kInf;
-          ty = sy ? bound_time(nby, oy, iy) : kInf;
-          tz = sz ? bound_time(nbz, oz, iz) : kInf;
-          stale = false;
-        }
-        const bool cy = ty < tx;
-        float tm = cy ? ty : tx;
-        const bool cz = tz < tm;
-        tm = cz ? tz : tm;
-        a = cz ? 2 : (cy ? 1 : 0);
-        cs++;
-        t = tm;
-        const bool a0 = a == 0, a1 = a == 1, a2 = a == 2;
-        Bx += a0 ? sx : 0;
-        By += a1 ? sy : 0;
-        Bz += a2 ? sz : 0;
-        idx += a0 ? dIx : (a1 ? dIy : dIz);
-        out = ((unsigned)Bx >= (unsigned)NBx) | ((unsigned)By >= (unsigned)NBy) | ((unsigned)Bz >= (unsigned)NBz);
-        if (out || cs + fs > cap) break;
-        p = __ldg(V.ptr + idx);
-        if (kStats) {
-          n_fetch++;
-          n_brick += p != MESO_EMPTY_BRICK;
-        } else {
-          // entering a new cell: is it empty?
-          const int cnew = a0 ? Bx : (a1 ? By : Bz);
-          const int snew = a0 ? sx : (a1 ? sy : sz);
-          if ((cnew & 3) == (snew > 0 ? 0 : 3)) lvl = cell_level(V, Bx, By, Bz, MX, MY, MX2, MY2, MX3, MY3);
-        }
-        // the next boundary time is computed while the pointer load is in
-        // flight; an occupied brick recomputes its times from scratch
-        nbx += a0 ? 8 * sx : 0;
-        nby += a1 ? 8 * sy : 0;
-        nbz += a2 ? 8 * sz : 0;
-        const int nb = a0 ? nbx : (a1 ? nby : nbz);
-        const float oo = a0 ? ox : (a1 ? oy : oz);
-        const float ii = a0 ? ix : (a1 ? iy : iz);
-        const float tn = bound_time(nb, oo, ii);
-        tx = a0 ? tn : tx;
-        ty = a1 ? tn : ty;
-        tz = a2 ? tn : tz;
-        if (p != MESO_EMPTY_BRICK) break;
-      }
+    const bool coarse = p == MESO_EMPTY_BRICK;
+    if (coarse) {
+      // one step per empty brick
+      const float tx = sx ? bound_time((Bx + px) * 8 - bx0, ox, ix) : kInf;
+      const float ty = sy ? bound_time((By + py) * 8 - by0, oy, iy) : kInf;
+      const float tz = sz ? bound_time((Bz + pz) * 8 - bz0, oz, iz) : kInf;
+      const bool cy = ty < tx;
+      float tm = cy ? ty : tx;
+      const bool cz = tz < tm;
+      tm = cz ? tz : tm;
+      const int a = cz ? 2 : (cy ? 1 : 0);
+      cs++;
+      t = tm;
       ea = a;
-      if (out || p == MESO_EMPTY_BRICK) break;
-      // entry voxel of the occupied brick: exact along the stepped axis,
-      // floor of the entry point (clamped into the brick) along the others
+      Bx += a == 0 ? sx : 0;
+      By += a == 1 ? sy : 0;
+      Bz += a == 2 ? sz : 0;
+      if (((unsigned)Bx >= (unsigned)NBx) | ((unsigned)By >= (unsigned)NBy) | ((unsigned)Bz >= (unsigned)NBz)) break;
+      // the voxel entered: exact along the stepped axis, floor of the entry
+      // point (clamped into the brick) along the others
       const int fx = clampi((int)floorf(__fadd_rn(ox, __fmul_rn(dx, t))) + bx0, Bx * 8, Bx * 8 + 7);
       const int fy = clampi((int)floorf(__fadd_rn(oy, __fmul_rn(dy, t))) + by0, By * 8, By * 8 + 7);
       const int fz = clampi((int)floorf(__fadd_rn(oz, __fmul_rn(dz, t))) + bz0, Bz * 8, Bz * 8 + 7);
       vx = a == 0 ? (sx > 0 ? Bx * 8 : Bx * 8 + 7) : fx;
       vy = a == 1 ? (sy > 0 ? By * 8 : By * 8 + 7) : fy;
       vz = a == 2 ? (sz > 0 ? Bz * 8 : Bz * 8 + 7) : fz;
+      continue;
     }
-    // ---- fine: voxel steps inside occupied brick p; nv* = next voxel
-    // boundary (relative) along each axis
-    if (cs + fs > cap) break;
+    // voxel steps inside occupied brick p
     const uint64_t* occ = V.occ + (size_t)p * 8;
-    uint64_t w = __ldg(occ + (vz & 7));
-    int nvx = vx + px - bx0, nvy = vy + py - by0, nvz = vz + pz - bz0;
-    float tx = sx ? bound_time(nvx, ox, ix) : kInf;
-    float ty = sy ? bound_time(nvy, oy, iy) : kInf;
-    float tz = sz ? bound_time(nvz, oz, iz) : kInf;
-    bool left = false, exit_brick = false;
+    bool left = false;
     for (;;) {
-      if ((w >> ((vx & 7) + 8 * (vy & 7))) & 1ull) {
+      if ((__ldg(occ + (vz & 7)) >> ((vx & 7) + 8 * (vy & 7))) & 1ull) {
         r.hit = 1;
         break;
       }
+      const float tx = sx ? bound_time(vx + px - bx0, ox, ix) : kInf;
+      const float ty = sy ? bound_time(vy + py - by0, oy, iy) : kInf;
+      const float tz = sz ? bound_time(vz + pz - bz0, oz, iz) : kInf;
       const bool cy = ty < tx;
       float tm = cy ? ty : tx;
       const bool cz = tz < tm;
@@ -302,34 +171,18 @@ __device__ __forceinline__ void traverse(const RayView& V, int bx0, int by0, int
       fs++;
       t = tm;
       ea = a;
-      const bool a0 = a == 0, a1 = a == 1, a2 = a == 2;
-      vx += a0 ? sx : 0;
-      vy += a1 ? sy : 0;
-      vz += a2 ? sz : 0;
-      // next z layer's word, in flight during the bookkeeping below (on a
-      // brick exit it wraps within this brick's 8 words and is unused)
-      if (a2) w = __ldg(occ + (vz & 7));
-      const int c = a0 ? vx : (a1 ? vy : vz);
-      const int cb = a0 ? Bx : (a1 ? By : Bz);
-      exit_brick = (c >> 3) != cb;
-      if (exit_brick) {
+      vx += a == 0 ? sx : 0;
+      vy += a == 1 ? sy : 0;
+      vz += a == 2 ? sz : 0;
+      const int c = a == 0 ? vx : (a == 1 ? vy : vz);
+      const int cb = a == 0 ? Bx : (a == 1 ? By : Bz);
+      if ((c >> 3) != cb) {
         Bx = vx >> 3;
         By = vy >> 3;
         Bz = vz >> 3;
-        idx += a0 ? dIx : (a1 ? dIy : dIz);
         left = ((unsigned)Bx >= (unsigned)NBx) | ((unsigned)By >= (unsigned)NBy) | ((unsigned)Bz >= (unsigned)NBz);
         break;
       }
-      nvx += a0 ? sx : 0;
-      nvy += a1 ? sy : 0;
-      nvz += a2 ? sz : 0;
-      const int nv = a0 ? nvx : (a1 ? nvy : nvz);
-      const float oo = a0 ? ox : (a1 ? oy : oz);
-      const float ii = a0 ? ix : (a1 ? iy : iz);
-      const float tn = bound_time(nv, oo, ii);
-      tx = a0 ? tn : tx;
-      ty = a1 ? tn : ty;
-      tz = a2 ? tn : tz;
       if (cs + fs > cap) {
         left = true;
         break;
@@ -342,10 +195,223 @@ __device__ __forceinline__ void traverse(const RayView& V, int bx0, int by0, int
   r.vz = vz;
   r.t = t;
   r.axis = ea;
+  r.slot = p;
   r.coarse = cs;
   r.fine = fs;
   r.fetches = n_fetch;
   r.bricks = n_brick;
+}
+
+// ---------------------------------------------------------- region walk
+// The same walk, taken a region at a time, with the same results bit for bit.
+//
+// A region is an aligned empty cube of 2^l voxels around the ray's position:
+// l = 5..9 cells of 4^3 .. 64^3 bricks (a level byte per 4^3-brick cell),
+// l = 3, 4 one brick or 2^3 bricks (the cell's 64-bit mask of its bricks),
+// l = 1, 2 blocks of 2^3 or 4^3 voxels of an occupied brick (a 64-bit mask of
+// its 2^3-voxel blocks), l = 0 one voxel.  Every kind is left by one and the
+// same piece of code, so the lanes of a warp stay together whatever each is
+// crossing; the former loops for cell jumps, brick steps and voxel steps ran
+// one after the other with half of the lanes idle.
+//
+// Why it is the same walk.  Each axis's boundary times never decrease along
+// the ray, and the walk takes all axes' boundaries merged in (time, axis x<y<z)
+// order.  So it leaves a region through the face with the smallest (time,
+// axis); the boundaries of another axis that it takes before are those whose
+// (time, axis) precede the face's, a prefix; and the steps it makes are the
+// voxels (inside a brick) or bricks it moves by, whatever their order, so they
+// are counted from the positions where a run of either kind begins and ends.
+//
+// The position along the other axes.  A boundary at relative coordinate b is
+// taken iff its computed time (b - o) * (1/d) precedes the face's time tE.
+// The computed time differs from the real (b - o) / d by at most 3 roundings,
+// the position o + d * tE below by a few more: less than 8 * 2^-24 of the
+// largest coordinate R in all.  Where the position lies further than twice
+// that (margin = R * 2^-20) from a boundary, the boundary's side of it
+// decides; else the boundary's own time is computed and compared.
+//
+// Directions are mirrored so that every ray moves up: an axis with d < 0
+// counts voxels as ~v and uses -o, -d and -1/d, which rounds the same way
+// and keeps the regions' alignment.  An axis with d = 0 gets an infinite
+// 1/d, so its faces lie at infinite time and are never chosen.
+//
+struct RayAxis {
+  float o, d, i;  // mirrored origin, |d| and 1/|d| (infinite for d = 0)
+  float a;        // o plus the base voxel: absolute origin, for estimates
+  int b;          // mirrored base voxel
+  int m;          // -1 for a mirrored axis, else 0
+};
+
+__device__ __forceinline__ RayAxis ray_axis(int b0, float o, float d, float inv) {
+  RayAxis A;
+  A.m = d < 0.0f ? -1 : 0;
+  A.o = d < 0.0f ? -o : o;
+  A.d = fabsf(d);
+  A.i = d == 0.0f ? kInf : fabsf(inv);
+  A.b = d < 0.0f ? -b0 : b0;
+  A.a = A.o + __int2float_rn(A.b);
+  return A;
+}
+
+// d is 0, or of a size at which 1/d and the boundary times are normal numbers
+__device__ __forceinline__ bool regular_axis(float d) {
+  const float m = fabsf(d);
+  return m == 0.0f || (m > 1e-30f && m < 1e30f);
+}
+
+// Time of the mirrored absolute boundary f.
+__device__ __forceinline__ float face_time(const RayAxis& A, int f) {
+  return __fmul_rn(__fsub_rn(__int2float_rn(f - A.b), A.o), A.i);
+}
+
+// Voxel (mirrored) at time t along an axis that was not stepped, by the
+// definition's own operations: floor(o + d*t).
+__device__ __forceinline__ int entry_voxel(const RayAxis& A, float t) {
+  const float x = __fadd_rn(A.o, __fmul_rn(A.d, t));
+  return (__float2int_rd(A.m ? -x : x) ^ A.m) + A.b;
+}
+
+constexpr float kRoundMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to the nearest integer
+
+// Units (2^ush voxels) along one axis at time t: index of the unit that the
+// position estimate lies in, and how far the estimate is from a unit's middle.
+__device__ __forceinline__ int estimate(const RayAxis& A, float t, float inv_unit, int ush, float& off) {
+  const float q = __fmaf_rn(__fmaf_rn(A.d, t, A.a), inv_unit, -0.5f);
+  const float s = __fadd_rn(q, kRoundMagic);
+  off = __fsub_rn(q, __fsub_rn(s, kRoundMagic));
+  return (__float_as_int(s) - 0x4B400000) << ush;
+}
+
+// An estimate too close to a unit boundary: the boundary's own time decides
+// on which side of it the ray is at tE (`first`: this axis wins ties).
+__device__ __forceinline__ int settle(float o, float i, int b, int e, int ush, float off, float tE, bool first) {
+  const int bd = off > 0.0f ? e + (1 << ush) : e;  // the boundary next to the estimate
+  const float tb = __fmul_rn(__fsub_rn(__int2float_rn(bd - b), o), i);
+  return (tb < tE || (tb == tE && first)) ? bd : bd - (1 << ush);
+}
+
+__device__ __forceinline__ void walk_regions(const RayView& V, const RayAxis& X, const RayAxis& Y, const RayAxis& Z,
+                                             float margin, int vx, int vy, int vz, float t, int ea, Trav& r) {
+  const int CX = V.nx >> 5, CY = V.ny >> 5;  // cells of 4x4x4 bricks
+  int x = vx ^ X.m, y = vy ^ Y.m, z = vz ^ Z.m;  // mirrored position
+  // steps: += position where a run of its kind ends, -= where it begins
+  int cs = 0, fs = -(x + y + z);
+  bool fine = true;   // in an occupied brick (the first position counts as one until looked up)
+  bool look = true;   // the brick at the position has not been looked up
+  uint32_t p = 0;
+  uint64_t blocks = 0;  // 2^3-voxel blocks of the current brick
+  r.hit = 0;
+  for (;;) {
+    const int ux = x ^ X.m, uy = y ^ Y.m, uz = z ^ Z.m;
+    int l = 0;
+    if (look) {
+      if (((unsigned)ux >= (unsigned)V.nx) | ((unsigned)uy >= (unsigned)V.ny) | ((unsigned)uz >= (unsigned)V.nz)) break;
+      const uint32_t c = (uint32_t)(ux >> 5) + (uint32_t)CX * ((uint32_t)(uy >> 5) + (uint32_t)CY * (uint32_t)(uz >> 5));
+      const uint32_t lev = __ldg(V.level + c);
+      const uint64_t bricks = __ldg(V.mask + c);
+      const int k = ((ux >> 3) & 3) | ((uy >> 1) & 12) | ((uz << 1) & 48);
+      if ((bricks >> k) & 1ull) {
+        p = __ldg(V.ptr + (uint32_t)(ux >> 3) +
+                  (uint32_t)(V.nx >> 3) * ((uint32_t)(uy >> 3) + (uint32_t)(V.ny >> 3) * (uint32_t)(uz >> 3)));
+        blocks = __ldg(V.sub + p);
+        if (!fine) {
+          cs += (x >> 3) + (y >> 3) + (z >> 3);
+          // exact along the stepped axis (x, y or z is its brick's first
+          // voxel already), floor of the entry point along the others
+          if (ea != 0) x = clampi(entry_voxel(X, t), x & ~7, x | 7);
+          if (ea != 1) y = clampi(entry_voxel(Y, t), y & ~7, y | 7);
+          if (ea != 2) z = clampi(entry_voxel(Z, t), z & ~7, z | 7);
+          fs -= x + y + z;
+          fine = true;
+        }
+      } else {
+        if (fine) {
+          fs += x + y + z;
+          cs -= (x >> 3) + (y >> 3) + (z >> 3);
+          fine = false;
+        }
+        l = lev ? (int)lev : (((bricks >> (k & 42)) & 0x330033ull) ? 3 : 4);
+      }
+    }
+    if (fine) {
+      const int wx = x ^ X.m, wy = y ^ Y.m, wz = z ^ Z.m;
+      const int k = ((wx >> 1) & 3) | ((wy << 1) & 12) | ((wz << 3) & 48);
+      if (!((blocks >> (k & 42)) & 0x330033ull)) {
+        l = 2;
+      } else if (!((blocks >> k) & 1ull)) {
+        l = 1;
+      } else {
+        const uint64_t w = __ldg(V.occ + (size_t)p * 8 + (wz & 7));
+        if ((w >> ((wx & 7) + 8 * (wy & 7))) & 1ull) {
+          r.hit = 1;
+          break;
+        }
+        l = 0;
+      }
+    }
+    // ---- leave the region of 2^l voxels
+    const int in = (1 << l) - 1;
+    const int fx = (x | in) + 1, fy = (y | in) + 1, fz = (z | in) + 1;
+    const float tx = face_time(X, fx), ty = face_time(Y, fy), tz = face_time(Z, fz);
+    const bool cy = ty < tx;
+    float tE = cy ? ty : tx;
+    const bool cz = tz < tE;
+    tE = cz ? tz : tE;
+    const bool az = cz, ay = cy && !cz, ax = !cy && !cz;
+    const int ush = l >= 3 ? 3 : 0;
+    const float inv_unit = l >= 3 ? 0.125f : 1.0f;
+    // a voxel has no boundary inside it to be unsure of
+    const float lim = l == 0 ? 1.0f : __fmaf_rn(-margin, inv_unit, 0.5f);
+    float gx, gy, gz;
+    int nx = estimate(X, tE, inv_unit, ush, gx), ny = estimate(Y, tE, inv_unit, ush, gy),
+        nz = estimate(Z, tE, inv_unit, ush, gz);
+    const bool qx = !ax && fabsf(gx) > lim, qy = !ay && fabsf(gy) > lim, qz = !az && fabsf(gz) > lim;
+    if (qx | qy | qz) {
+      if (qx) nx = settle(X.o, X.i, X.b, nx, ush, gx, tE, true);
+      if (qy) ny = settle(Y.o, Y.i, Y.b, ny, ush, gy, tE, az);
+      if (qz) nz = settle(Z.o, Z.i, Z.b, nz, ush, gz, tE, false);
+    }
+    x = ax ? fx : max(x, min(x | in, nx));
+    y = ay ? fy : max(y, min(y | in, ny));
+    z = az ? fz : max(z, min(z | in, nz));
+    t = tE;
+    ea = az ? 2 : (ay ? 1 : 0);
+    look = !fine || ((ax ? fx : (ay ? fy : fz)) & 7) == 0;
+  }
+  if (fine) fs += x + y + z;
+  else cs += (x >> 3) + (y >> 3) + (z >> 3);
+  // a mirrored boundary that passes through the origin: (b - o) * (1/d) is
+  // minus zero there
+  if (t == 0.0f && ea >= 0) {
+    const int f = ea == 0 ? x - X.b : (ea == 1 ? y - Y.b : z - Z.b), m = ea == 0 ? X.m : (ea == 1 ? Y.m : Z.m);
+    const float o = ea == 0 ? X.o : (ea == 1 ? Y.o : Z.o);
+    if (m && __int2float_rn(f) == o) t = -0.0f;
+  }
+  r.vx = x ^ X.m;
+  r.vy = y ^ Y.m;
+  r.vz = z ^ Z.m;
+  r.t = t;
+  r.axis = ea;
+  r.slot = p;
+  r.coarse = (uint32_t)cs;
+  r.fine = (uint32_t)fs;
+}
+
+// Traces a ray by regions where its values allow, else step by step.
+template <bool kStats>
+__device__ __forceinline__ void trace(const RayView& V, float margin, int bx0, int by0, int bz0, float ox, float oy,
+                                      float oz, float dx, float dy, float dz, float ix, float iy, float iz, int vx,
+                                      int vy, int vz, float t, int ea, Trav& r) {
+  const bool regions = !kStats && margin > 0.0f && regular_axis(dx) && regular_axis(dy) && regular_axis(dz) &&
+                       (dx != 0.0f || dy != 0.0f || dz != 0.0f);
+  if (regions) {
+    const RayAxis X = ray_axis(bx0, ox, dx, ix), Y = ray_axis(by0, oy, dy, iy), Z = ray_axis(bz0, oz, dz, iz);
+    walk_regions(V, X, Y, Z, margin, vx, vy, vz, t, ea, r);
+  } else {
+    Trav q;
+    walk_steps<kStats>(V, bx0, by0, bz0, ox, oy, oz, dx, dy, dz, ix, iy, iz, vx, vy, vz, t, ea, q);
+    r = q;
+  }
 }
 
 __device__ __forceinline__ void camera_ray(const RayView& V, uint32_t px, uint32_t py, float& dx, float& dy,
@@ -448,48 +514,58 @@ __device__ __forceinline__ void trace_pixel(const RayView& V, uint32_t px, uint3
     vy = clampi((int)floorf(oy) + by0, 0, V.ny - 1);
     vz = clampi((int)floorf(oz) + bz0, 0, V.nz - 1);
   }
-  Trav r;
-  traverse<kStats>(V, bx0, by0, bz0, ox, oy, oz, dx, dy, dz, ix, iy, iz, vx, vy, vz, t0, ea, r);
-  h.steps = r.fine | (r.coarse << 16);
-  if (kStats) {
-    st[0] += r.fetches;
-    st[1] += r.bricks;
-    st[3] += 1;
+  // pass 0 the primary ray, pass 1 the shadow ray of a hit: one copy of the
+  // walk's code for both
+  int base_x = bx0, base_y = by0, base_z = bz0;
+  float rox = ox, roy = oy, roz = oz, rdx = dx, rdy = dy, rdz = dz, rix = ix, riy = iy, riz = iz;
+#pragma unroll 1
+  for (int pass = 0;; pass++) {
+    Trav r;
+    trace<kStats>(V, P.margin, base_x, base_y, base_z, rox, roy, roz, rdx, rdy, rdz, rix, riy, riz, vx, vy, vz, t0, ea,
+                  r);
+    if (kStats) {
+      st[0] += r.fetches;
+      st[1] += r.bricks;
+      st[3] += 1;
+    }
+    if (pass) {
+      h.shadow = (uint8_t)(r.hit ? 1 : 0);
+      h.shadow_steps = r.fine | (r.coarse << 16);
+      return;
+    }
+    h.steps = r.fine | (r.coarse << 16);
+    if (!r.hit) return;
+    if (kStats) st[2] += 1;
+    h.voxel = (uint64_t)r.vx + (uint64_t)V.nx * ((uint64_t)r.vy + (uint64_t)V.ny * (uint64_t)r.vz);
+    h.t = r.t;
+    h.material = __ldg(V.mat + (size_t)r.slot * 512 + (r.vx & 7) + 8 * (r.vy & 7) + 64 * (r.vz & 7));
+    if (r.axis < 0) return;
+    const float da = r.axis == 0 ? rdx : (r.axis == 1 ? rdy : rdz);
+    const int sa = da > 0.0f ? 1 : (da < 0.0f ? -1 : 0);
+    h.face = (uint8_t)(2 * r.axis + (sa > 0 ? 1 : 0));
+    if (!P.shadow) return;
+    // the shadow ray starts at the centre of the empty voxel across the face
+    vx = r.vx - (r.axis == 0 ? sa : 0);
+    vy = r.vy - (r.axis == 1 ? sa : 0);
+    vz = r.vz - (r.axis == 2 ? sa : 0);
+    if (((unsigned)vx >= (unsigned)V.nx) | ((unsigned)vy >= (unsigned)V.ny) | ((unsigned)vz >= (unsigned)V.nz)) {
+      h.shadow = 0;
+      return;
+    }
+    base_x = vx;
+    base_y = vy;
+    base_z = vz;
+    rox = roy = roz = 0.5f;
+    rdx = P.light[0];
+    rdy = P.light[1];
+    rdz = P.light[2];
+    rix = P.inv_light[0];
+    riy = P.inv_light[1];
+    riz = P.inv_light[2];
+    t0 = 0.0f;
+    ea = -1;
   }
-  if (!r.hit) return;
-  if (kStats) st[2] += 1;
-  h.voxel = (uint64_t)r.vx + (uint64_t)V.nx * ((uint64_t)r.vy + (uint64_t)V.ny * (uint64_t)r.vz);
-  h.t = r.t;
-  {
-    const uint32_t p =
-        __ldg(V.ptr + (size_t)(r.vx >> 3) + (size_t)(V.nx >> 3) * ((size_t)(r.vy >> 3) + (size_t)(V.ny >> 3) * (r.vz >> 3)));
-    h.material = __ldg(V.mat + (size_t)p * 512 + (r.vx & 7) + 8 * (r.vy & 7) + 64 * (r.vz & 7));
-  }
-  if (r.axis < 0) return;
-  const int sa = r.axis == 0 ? sx : (r.axis == 1 ? sy : sz);
-  h.face = (uint8_t)(2 * r.axis + (sa > 0 ? 1 : 0));
-  if (!P.shadow) return;
-  int Sx = r.vx, Sy = r.vy, Sz = r.vz;
-  bool outside;
-  if (r.axis == 0) { Sx -= sx; outside = Sx < 0 || Sx >= V.nx; }
-  else if (r.axis == 1) { Sy -= sy; outside = Sy < 0 || Sy >= V.ny; }
-  else { Sz -= sz; outside = Sz < 0 || Sz >= V.nz; }
-  if (outside) {
-    h.shadow = 0;
-    return;
-  }
-  Trav sr;
-  traverse<kStats>(V, Sx, Sy, Sz, 0.5f, 0.5f, 0.5f, P.light[0], P.light[1], P.light[2], P.inv_light[0],
-                   P.inv_light[1], P.inv_light[2], Sx, Sy, Sz, 0.0f, -1, sr);
-  if (kStats) {
-    st[0] += sr.fetches;
-    st[1] += sr.bricks;
-    st[3] += 1;
-  }
-  h.shadow = (uint8_t)(sr.hit ? 1 : 0);
-  h.shadow_steps = sr.fine | (sr.coarse << 16);
 }
-
 
 // kMode: kPlain; kStatsMode also accumulates {pointer fetches, occupied
 // bricks entered, hits, rays} into P.stats; kHashMode also adds each view's
@@ -636,9 +712,9 @@ static void fill_views(const meso_scene* const* scenes, const meso_camera* cams,
     RayView& V = out[v];
     memset(&V, 0, sizeof(V));
     V.ptr = s->d_ptr;
-    V.macro = s->d_macro;
-    V.macro2 = s->d_macro2;
-    V.macro3 = s->d_macro3;
+    V.level = s->d_level;
+    V.mask = s->d_mask;
+    V.sub = s->d_sub;
     V.occ = s->d_occ;
     V.mat = s->d_mat;
     V.nx = s->nx;
@@ -662,6 +738,22 @@ static void fill_views(const meso_scene* const* scenes, const meso_camera* cams,
     tiles += (uint64_t)V.tiles_x * tiles_y;
     hits += (uint64_t)c.width * c.height;
   }
+}
+
+// The region walk's margin for a launch: 2^-20 of the largest coordinate a
+// ray of the views reaches (twice the error bound derived at walk_regions),
+// or 0 (every ray step by step) where a view lies outside what that bound was
+// derived for: coordinates beyond 2^17 voxels, an origin that is not finite.
+static float region_margin(const meso_scene* const* scenes, const meso_camera* cams, uint32_t n_views) {
+  float R = 0.0f;
+  for (uint32_t v = 0; v < n_views; v++)
+    for (int a = 0; a < 3; a++) {
+      const int n = a == 0 ? scenes[v]->nx : (a == 1 ? scenes[v]->ny : scenes[v]->nz);
+      const float c = 32.0f * fabsf((float)cams[v].origin_chunk[a]) + (float)n + fabsf(cams[v].origin_frac[a]) + 64.0f;
+      if (!(c < 131072.0f)) return 0.0f;
+      R = c > R ? c : R;
+    }
+  return R * 9.5367431640625e-7f;
 }
 
 }  // namespace meso
@@ -734,6 +826,7 @@ meso_status launch_raymarch(meso_ctx* ctx, const meso_scene* const* scenes, cons
   P.tile_w = tw;
   P.tile_h = th;
   P.shadow = (flags & MESO_RAY_SHADOW) ? 1u : 0u;
+  P.margin = region_margin(scenes, cams, n_views);
   if (light)
     for (int a = 0; a < 3; a++) {
       P.light[a] = light[a];
@@ -866,6 +959,7 @@ extern "C" meso_status meso_raymarch_noalloc(meso_ctx* ctx, const meso_scene* co
   P.tile_w = tw;
   P.tile_h = th;
   P.shadow = (flags & MESO_RAY_SHADOW) ? 1u : 0u;
+  P.margin = region_margin(scenes, h_cams, n_views);
   if (light)
     for (int a = 0; a < 3; a++) {
       P.light[a] = light[a];

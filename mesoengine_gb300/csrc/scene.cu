@@ -78,6 +78,26 @@ __global__ void column_max_kernel(TerrainDev T, const float* heights, float* hma
   hmax[i] = m;
 }
 
+// The non-empty 2x2x2-voxel blocks of a brick (bit x + 4y + 16z) from its
+// occupancy as 16 words of 32 voxels (word k: z = k/2, rows y = 4(k mod 2) ..
+// +3 of 8 bits each).
+__device__ __forceinline__ uint64_t sub_mask(const uint32_t (&w)[16]) {
+  uint64_t m = 0;
+#pragma unroll
+  for (int z = 0; z < 4; z++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      uint32_t v = w[4 * z + h] | w[4 * z + 2 + h];  // both layers
+      v |= v >> 8;                                   // both rows: bytes 0 and 2
+      v |= v >> 1;                                   // both columns: even bits
+      v &= 0x00550055u;
+      v = (v | v >> 1) & 0x00330033u;
+      v = (v | v >> 2) & 0x000F000Fu;
+      m |= (uint64_t)((v | v >> 12) & 0xFFu) << (16 * z + 8 * h);
+    }
+  return m;
+}
+
 // One warp per brick; lane covers voxels lane + 32k (x = i&7, y = (i>>3)&7, z = i>>6).
 template <bool kFill>
 __global__ void terrain_brick_kernel(TerrainDev T, const float* heights, const float* hmax, uint8_t* flags,
@@ -333,6 +353,7 @@ struct EditParams {
   uint32_t* ptr;
   uint64_t* occ;
   uint16_t* mat;
+  uint64_t* sub;
   uint16_t* temp;          // 512 per touched brick
   uint8_t* state;          // per touched brick: bit0 present, bit1 nonempty
   uint32_t* free_stack;
@@ -368,11 +389,14 @@ __global__ void edit_compute_kernel(EditParams P) {
   for (int k = 0; k < 16; k++) any |= v[k] != 0;
   const bool nonempty = __any_sync(kFull, any);
   if (present && nonempty) {
+    uint32_t w[16];
+#pragma unroll
     for (int k = 0; k < 16; k++) {
       P.mat[(size_t)slot * 512 + lane + 32 * k] = v[k];
-      const uint32_t bits = __ballot_sync(kFull, v[k] != 0);
-      if (lane == 0) reinterpret_cast<uint32_t*>(P.occ + (size_t)slot * 8)[k] = bits;
+      w[k] = __ballot_sync(kFull, v[k] != 0);
+      if (lane == 0) reinterpret_cast<uint32_t*>(P.occ + (size_t)slot * 8)[k] = w[k];
     }
+    if (lane == 0) P.sub[slot] = sub_mask(w);
   } else if (present && !nonempty) {
     if (lane == 0) {
       P.ptr[b] = MESO_EMPTY_BRICK;
@@ -410,13 +434,18 @@ __global__ void edit_alloc_kernel(EditParams P) {
   slot = __shfl_sync(kFull, slot, 0);
   if (!ok) return;
   const uint32_t b = P.bricks[wi];
+  uint32_t w[16];
+#pragma unroll
   for (int k = 0; k < 16; k++) {
     const uint16_t m = P.temp[(size_t)wi * 512 + lane + 32 * k];
     P.mat[(size_t)slot * 512 + lane + 32 * k] = m;
-    const uint32_t bits = __ballot_sync(kFull, m != 0);
-    if (lane == 0) reinterpret_cast<uint32_t*>(P.occ + (size_t)slot * 8)[k] = bits;
+    w[k] = __ballot_sync(kFull, m != 0);
+    if (lane == 0) reinterpret_cast<uint32_t*>(P.occ + (size_t)slot * 8)[k] = w[k];
   }
-  if (lane == 0) P.ptr[b] = slot;
+  if (lane == 0) {
+    P.ptr[b] = slot;
+    P.sub[slot] = sub_mask(w);
+  }
 }
 
 __global__ void edit_fix_kernel(int32_t* alloc, uint32_t capacity) {
@@ -453,22 +482,24 @@ unsigned grid_for(uint64_t warps, int threads = 256) {
 
 }  // namespace
 
-// One warp per macro cell (4x4x4 bricks): any occupied brick -> 1.
-__global__ void macro_kernel(const uint32_t* ptr, int bx, int by, uint8_t* macro, const uint32_t* cells,
-                             uint64_t n) {
+// One warp per macro cell (4x4x4 bricks): the mask of its occupied bricks
+// (bit x + 4y + 16z), and a byte that says whether there are any.
+__global__ void macro_kernel(const uint32_t* ptr, int bx, int by, uint8_t* macro, uint64_t* mask,
+                             const uint32_t* cells, uint64_t n) {
   const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (w >= n) return;
   const uint32_t m = cells ? cells[w] : (uint32_t)w;
   const int mx = bx >> 2, my = by >> 2;
   const int cx = (int)(m % (uint32_t)mx), cy = (int)((m / (uint32_t)mx) % (uint32_t)my), cz = (int)(m / ((uint32_t)mx * my));
-  bool any = false;
-  for (int k = lane; k < 64; k += 32) {
-    const int x = cx * 4 + (k & 3), y = cy * 4 + ((k >> 2) & 3), z = cz * 4 + (k >> 4);
-    any |= ptr[(uint64_t)x + (uint64_t)bx * ((uint64_t)y + (uint64_t)by * z)] != MESO_EMPTY_BRICK;
+  const int x = cx * 4 + (lane & 3), y = cy * 4 + ((lane >> 2) & 3), z = cz * 4 + (lane >> 4);
+  const uint64_t i = (uint64_t)x + (uint64_t)bx * ((uint64_t)y + (uint64_t)by * z);
+  const uint32_t lo = __ballot_sync(0xFFFFFFFFu, ptr[i] != MESO_EMPTY_BRICK);
+  const uint32_t hi = __ballot_sync(0xFFFFFFFFu, ptr[i + 2ull * bx * by] != MESO_EMPTY_BRICK);
+  if (lane == 0) {
+    macro[m] = (lo | hi) != 0 ? 1 : 0;
+    mask[m] = (uint64_t)hi << 32 | lo;
   }
-  const bool occupied = __any_sync(0xFFFFFFFFu, any);
-  if (lane == 0) macro[m] = occupied ? 1 : 0;
 }
 
 // One warp per 16x16x16-brick cell: any occupied 4x4x4-brick child -> 1 (its
@@ -516,6 +547,70 @@ __global__ void macro3_kernel(const uint8_t* macro2, int bx, int by, int bz, uin
   if (lane == 0) macro3[i] = set ? 1 : 0;
 }
 
+// Level bytes: per 4x4x4-brick cell log2 of the edge, in voxels, of the
+// largest aligned cube of empty space that the cell is part of and that lies
+// in the grid (9: 64^3 bricks, 8: 32^3, 7: 16^3, 6: 8^3, 5: the cell), 0 if
+// the cell is occupied.  The cells of one 64^3-brick cell depend on nothing
+// outside it, so an edit recomputes those of the 64^3-brick cells it touches
+// (list; 4096 threads each), a build all of them.
+__global__ void level_kernel(const uint8_t* macro, const uint8_t* macro2, const uint8_t* macro3, int bx, int by,
+                             int bz, uint8_t* level, const uint32_t* list, uint64_t n) {
+  const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (w >= n) return;
+  const int mx = bx / 4, my = by / 4, mz = bz / 4;
+  const int m2x = (bx + 15) / 16, m2y = (by + 15) / 16, m2z = (bz + 15) / 16;
+  const int m3x = (bx + 63) / 64, m3y = (by + 63) / 64;
+  int cx, cy, cz;
+  if (list) {
+    const uint32_t r = list[w >> 12], k = (uint32_t)w & 4095u;
+    cx = (int)(r % (uint32_t)m3x) * 16 + (int)(k & 15u);
+    cy = (int)((r / (uint32_t)m3x) % (uint32_t)m3y) * 16 + (int)((k >> 4) & 15u);
+    cz = (int)(r / ((uint32_t)m3x * m3y)) * 16 + (int)(k >> 8);
+    if (cx >= mx || cy >= my || cz >= mz) return;
+  } else {
+    cx = (int)(w % (uint32_t)mx);
+    cy = (int)((w / (uint32_t)mx) % (uint32_t)my);
+    cz = (int)(w / ((uint32_t)mx * my));
+  }
+  // all 2x2x2 cells (aligned) around (x, y, z) of a map of nx x ny x nz cells in the grid and zero
+  auto block_empty = [](const uint8_t* m, int x, int y, int z, int nx, int ny, int nz) {
+    x &= ~1;
+    y &= ~1;
+    z &= ~1;
+    if (x + 1 >= nx || y + 1 >= ny || z + 1 >= nz) return false;
+    uint32_t any = 0;
+    for (int k = 0; k < 8; k++)
+      any |= m[(uint32_t)(x + (k & 1)) + (uint32_t)nx * ((uint32_t)(y + ((k >> 1) & 1)) + (uint32_t)ny * (uint32_t)(z + (k >> 2)))];
+    return any == 0;
+  };
+  const uint32_t i = (uint32_t)cx + (uint32_t)mx * ((uint32_t)cy + (uint32_t)my * (uint32_t)cz);
+  int l;
+  if (macro[i]) l = 0;
+  else if (!macro3[(uint32_t)(cx >> 4) + (uint32_t)m3x * ((uint32_t)(cy >> 4) + (uint32_t)m3y * (uint32_t)(cz >> 4))]) l = 9;
+  else if (block_empty(macro2, cx >> 2, cy >> 2, cz >> 2, m2x, m2y, m2z)) l = 8;
+  else if (!macro2[(uint32_t)(cx >> 2) + (uint32_t)m2x * ((uint32_t)(cy >> 2) + (uint32_t)m2y * (uint32_t)(cz >> 2))]) l = 7;
+  else if (block_empty(macro, cx, cy, cz, mx, my, mz)) l = 6;
+  else l = 5;
+  level[i] = (uint8_t)l;
+}
+
+// d_sub of `slots` consecutive pool slots, one thread each.
+__global__ void sub_kernel(const uint64_t* occ, uint64_t slots, uint64_t* sub) {
+  const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= slots) return;
+  const uint4* src = reinterpret_cast<const uint4*>(occ + p * 8);
+  uint32_t w[16];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const uint4 v = src[k];
+    w[4 * k] = v.x;
+    w[4 * k + 1] = v.y;
+    w[4 * k + 2] = v.z;
+    w[4 * k + 3] = v.w;
+  }
+  sub[p] = sub_mask(w);
+}
+
 // ---------------------------------------------------------------- scene API
 
 meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint64_t capacity, meso_scene** out) {
@@ -533,17 +628,32 @@ meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint6
     delete s;
     return fail(MESO_ERR_OVER_BUDGET, "scene exceeds the HBM budget");
   }
+  // one allocation for the cell maps and one for the pool's small arrays
+  const uint64_t nm = std::max<uint64_t>(n_macro_of(s), 1), nm2 = std::max<uint64_t>(n_macro2_of(s), 1),
+                 nm3 = std::max<uint64_t>(n_macro3_of(s), 1), nslot = std::max<uint64_t>(capacity, 1);
+  uint8_t* maps = nullptr;
+  uint8_t* small = nullptr;
   cudaError_t e = cudaMalloc(&s->d_ptr, nb * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&s->d_macro, std::max<uint64_t>(nb / 64, 1));
-  if (e == cudaSuccess) e = cudaMemset(s->d_macro, 0, std::max<uint64_t>(nb / 64, 1));
-  if (e == cudaSuccess) e = cudaMalloc(&s->d_macro2, std::max<uint64_t>(n_macro2_of(s), 1));
-  if (e == cudaSuccess) e = cudaMemset(s->d_macro2, 1, std::max<uint64_t>(n_macro2_of(s), 1));
-  if (e == cudaSuccess) e = cudaMalloc(&s->d_macro3, std::max<uint64_t>(n_macro3_of(s), 1));
-  if (e == cudaSuccess) e = cudaMemset(s->d_macro3, 1, std::max<uint64_t>(n_macro3_of(s), 1));
-  if (e == cudaSuccess) e = cudaMalloc(&s->d_occ, std::max<uint64_t>(capacity, 1) * 64);
-  if (e == cudaSuccess) e = cudaMalloc(&s->d_mat, std::max<uint64_t>(capacity, 1) * 1024);
-  if (e == cudaSuccess) e = cudaMalloc(&s->d_free, std::max<uint64_t>(capacity, 1) * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&s->d_alloc, 16);
+  if (e == cudaSuccess) e = cudaMalloc(&maps, nm * 10 + nm2 + nm3);
+  if (e == cudaSuccess) {
+    s->d_mask = reinterpret_cast<uint64_t*>(maps);
+    s->d_level = maps + nm * 8;
+    s->d_macro = s->d_level + nm;
+    s->d_macro2 = s->d_macro + nm;
+    s->d_macro3 = s->d_macro2 + nm2;
+    // until the maps are built nothing is known to be empty
+    e = cudaMemset(maps, 0xFF, nm * 8);
+  }
+  if (e == cudaSuccess) e = cudaMemset(s->d_level, 0, nm * 2);
+  if (e == cudaSuccess) e = cudaMemset(s->d_macro2, 1, nm2 + nm3);
+  if (e == cudaSuccess) e = cudaMalloc(&s->d_occ, nslot * 64);
+  if (e == cudaSuccess) e = cudaMalloc(&s->d_mat, nslot * 1024);
+  if (e == cudaSuccess) e = cudaMalloc(&small, nslot * 12 + 16);
+  if (e == cudaSuccess) {
+    s->d_sub = reinterpret_cast<uint64_t*>(small);
+    s->d_alloc = reinterpret_cast<int64_t*>(small + nslot * 8);
+    s->d_free = reinterpret_cast<uint32_t*>(small + nslot * 8 + 16);
+  }
   if (e != cudaSuccess) {
     scene_release(ctx, s);
     cudaGetLastError();
@@ -559,13 +669,10 @@ meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint6
 void scene_release(meso_ctx* ctx, meso_scene* s) {
   if (!s) return;
   cudaFree(s->d_ptr);
-  cudaFree(s->d_macro);
-  cudaFree(s->d_macro2);
-  cudaFree(s->d_macro3);
+  cudaFree(s->d_mask);  // the base of the cell maps
   cudaFree(s->d_occ);
   cudaFree(s->d_mat);
-  cudaFree(s->d_free);
-  cudaFree(s->d_alloc);
+  cudaFree(s->d_sub);  // the base of the pool's small arrays
   if (s->bytes) ctx->scene_bytes.fetch_sub(s->bytes);
   delete s;
 }
@@ -574,8 +681,8 @@ meso_status rebuild_macro(meso_ctx* ctx, meso_scene* s, const uint32_t* d_cells,
                           const uint32_t* d_cells2, uint32_t n2, const uint32_t* d_cells3, uint32_t n3) {
   const uint64_t cells = d_cells ? n : n_macro_of(s);
   if (cells == 0) return MESO_OK;
-  macro_kernel<<<(unsigned)((cells * 32 + 255) / 256), 256, 0, st>>>(s->d_ptr, s->bx, s->by, s->d_macro, d_cells,
-                                                                     cells);
+  macro_kernel<<<(unsigned)((cells * 32 + 255) / 256), 256, 0, st>>>(s->d_ptr, s->bx, s->by, s->d_macro, s->d_mask,
+                                                                     d_cells, cells);
   const uint64_t cells2 = d_cells2 ? n2 : n_macro2_of(s);
   if (cells2)
     macro2_kernel<<<(unsigned)((cells2 * 32 + 255) / 256), 256, 0, st>>>(s->d_macro, s->bx, s->by, s->bz,
@@ -584,13 +691,26 @@ meso_status rebuild_macro(meso_ctx* ctx, meso_scene* s, const uint32_t* d_cells,
   if (cells3)
     macro3_kernel<<<(unsigned)((cells3 * 32 + 255) / 256), 256, 0, st>>>(s->d_macro2, s->bx, s->by, s->bz,
                                                                           s->d_macro3, d_cells3, n3);
-  ctx->launches.fetch_add(3);
+  const uint64_t levels = d_cells3 ? (uint64_t)n3 << 12 : n_macro_of(s);
+  if (levels)
+    level_kernel<<<(unsigned)((levels + 255) / 256), 256, 0, st>>>(s->d_macro, s->d_macro2, s->d_macro3, s->bx, s->by,
+                                                                    s->bz, s->d_level, d_cells3, levels);
+  ctx->launches.fetch_add(4);
+  MESO_CUDA_TRY(cudaGetLastError());
+  return MESO_OK;
+}
+
+meso_status rebuild_sub(meso_ctx* ctx, meso_scene* s, uint64_t slots, cudaStream_t st) {
+  if (slots == 0) return MESO_OK;
+  sub_kernel<<<(unsigned)((slots + 127) / 128), 128, 0, st>>>(s->d_occ, slots, s->d_sub);
+  ctx->launches.fetch_add(1);
   MESO_CUDA_TRY(cudaGetLastError());
   return MESO_OK;
 }
 
 static meso_status finish_pools(meso_ctx* ctx, meso_scene* s, uint64_t count, cudaStream_t st) {
   MESO_TRY(rebuild_macro(ctx, s, nullptr, 0, st));
+  MESO_TRY(rebuild_sub(ctx, s, count, st));
   int32_t init[4] = {(int32_t)count, 0, 0, 0};
   MESO_CUDA_TRY(cudaMemcpyAsync(s->d_alloc, init, 16, cudaMemcpyHostToDevice, st));
   MESO_CUDA_TRY(cudaStreamSynchronize(st));
@@ -961,6 +1081,7 @@ meso_status edit_spheres(meso_ctx* ctx, meso_scene* s, const meso_sphere_edit* h
   P.ptr = s->d_ptr;
   P.occ = s->d_occ;
   P.mat = s->d_mat;
+  P.sub = s->d_sub;
   P.temp = d_temp;
   P.state = d_state;
   P.free_stack = s->d_free;

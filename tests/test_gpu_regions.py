@@ -1,0 +1,124 @@
+"""The raymarch's region walk against the oracle's step-by-step walk.
+
+The kernel leaves aligned empty cubes of 1 to 512 voxels on a side in one
+step each and counts the steps it passed over from the positions; every field
+of every hit, t included, has to be the same bytes as the oracle's, for every
+direction octant, for directions with zero components, for origins on voxel,
+brick and chunk boundaries (boundary times that tie), for grids whose sides
+are no multiple of a cell, after edits and after a load, and for the values
+that take the step-by-step path instead (far cameras, a light without a
+direction).
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+import mesoengine_gb300 as meso
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def same(got, ref):
+    bad = np.nonzero((got.view(np.uint8).reshape(-1, 24) != ref.view(np.uint8).reshape(-1, 24)).any(1))[0]
+    assert bad.size == 0, f"{bad.size} of {got.size} hits differ, first {got[bad[:3]]} vs {ref[bad[:3]]}"
+
+
+def sparse(dims, seed, n_points, n_boxes):
+    """A mostly empty grid: single voxels, and boxes of a few voxels to a few bricks."""
+    rng = np.random.default_rng(seed)
+    nx, ny, nz = dims
+    g = np.zeros((nz, ny, nx), dtype=np.uint16)
+    for _ in range(n_points):
+        g[rng.integers(nz), rng.integers(ny), rng.integers(nx)] = rng.integers(1, 65536)
+    for _ in range(n_boxes):
+        x, y, z = (int(rng.integers(0, n)) for n in dims)
+        w, h, d = (int(v) for v in rng.integers(1, 20, 3))
+        g[z:z + d, y:y + h, x:x + w] = rng.integers(1, 65536)
+    return g
+
+
+@pytest.fixture(scope="module", params=[((32, 32, 32), 60, 2), ((96, 160, 64), 60, 12), ((544, 288, 320), 80, 60),
+                                        ((1024, 64, 576), 60, 40)], ids=lambda p: "x".join(map(str, p[0])))
+def grid(ctx, request):
+    dims, points, boxes = request.param
+    g = sparse(dims, sum(dims), points, boxes)
+    scene = ctx.scene_from_dense(g)
+    yield dims, scene, oracle.HostBrickMap.from_dense(g)
+    scene.destroy()
+
+
+def both(ctx, scene, bm, o, target, w=56, h=37, light=None):
+    same(ctx.raymarch(scene, meso.camera(o, target, w, h), light=light),
+         oracle.raymarch(bm, oracle.camera(o, target, w, h), light=light))
+
+
+def test_every_octant(ctx, grid):
+    dims, scene, bm = grid
+    c = [n / 2.0 + 0.37 for n in dims]
+    for k in range(8):
+        s = [1 if (k >> a) & 1 else -1 for a in range(3)]
+        out = [c[a] - s[a] * (0.6 * dims[a] + 21.3) for a in range(3)]
+        into = [c[a] + s[a] * (0.4 * dims[a] + 5.1) for a in range(3)]
+        both(ctx, scene, bm, out, c)   # from outside
+        both(ctx, scene, bm, c, into)  # from inside
+        light = np.array([0.3 * s[0], 0.5 * s[1], 0.8 * s[2]], dtype=np.float32)
+        both(ctx, scene, bm, out, c, light=light)
+
+
+def test_ties_and_axis_aligned_rays(ctx, grid):
+    dims, scene, bm = grid
+    nx, ny, nz = dims
+    # an odd image size puts rays exactly along the axis through its middle
+    for o, target in [((nx / 2, ny / 2, nz + 40.0), (nx / 2, ny / 2, 0.0)), ((-33.0, ny / 2, nz / 2), (nx, ny / 2, nz / 2)),
+                      ((nx / 2, ny + 8.0, nz / 2), (nx / 2, 0.0, nz / 2)), ((0.0, 0.0, 0.0), (nx, ny, nz)),
+                      ((float(nx), float(ny), float(nz)), (0.0, 0.0, 0.0)), ((-32.0, -32.0, -32.0), (32.0, 32.0, 32.0)),
+                      ((nx - 0.5, 0.5, 0.5), (nx - 33.5, 33.5, 33.5)), ((nx / 2, ny / 2, nz / 2), (nx / 2 + 8, ny / 2 + 8, nz / 2))]:
+        for w, h in ((33, 33), (32, 32)):
+            both(ctx, scene, bm, o, target, w, h)
+    for light in ((0.0, 0.0, 1.0), (1.0, 0.0, 0.0), (0.0, -1.0, 0.0), (1.0, 1.0, 1.0), (-0.5, 0.0, 0.5), (1e3, 2e3, 1e3)):
+        both(ctx, scene, bm, (-31.0, -17.0, nz + 25.0), (nx / 2, ny / 2, nz / 2), light=np.array(light, np.float32))
+
+
+def test_values_off_the_region_path(ctx, grid):
+    dims, scene, bm = grid
+    nx, ny, nz = dims
+    mid = (nx / 2, ny / 2, nz / 2)
+    both(ctx, scene, bm, (-140000.0, ny / 2 + 3.0, nz / 2 + 1.0), mid, 16, 9)  # beyond the region path's coordinates
+    both(ctx, scene, bm, (-100000.0, ny / 2 + 3.0, nz / 2 + 1.0), mid, 16, 9)  # within them
+    for light in ((0.0, 0.0, 0.0), (1e-32, 0.0, 1.0), (0.0, 1e-36, 0.0), (1e31, 1e31, 1e31)):
+        both(ctx, scene, bm, (-31.0, -17.0, nz + 25.0), mid, 24, 17, light=np.array(light, np.float32))
+    # a view that needs the step-by-step path beside one that does not
+    cams = [((-31.0, -17.0, nz + 25.0), mid), ((-140000.0, ny / 2 + 3.0, nz / 2 + 1.0), mid)]
+    got = ctx.raymarch(scene, [meso.camera(o, t, 20, 11) for o, t in cams])
+    same(got, oracle.raymarch(bm, [oracle.camera(o, t, 20, 11) for o, t in cams]))
+
+
+def _edits(rng, dims, n, radius):
+    return [(tuple(int(rng.integers(0, d)) for d in dims), int(rng.integers(0, radius + 1)),
+             0 if rng.random() < 0.4 else int(rng.integers(1, 65536))) for _ in range(n)]
+
+
+@pytest.mark.parametrize("radius", [0, 1, 3, 40])
+def test_maps_follow_edits(ctx, radius, tmp_path):
+    # single voxels and small spheres (blocks inside bricks), large ones
+    # (cells of every level emptied and filled); then the same scene from a file
+    dims = (544, 288, 320)
+    g = sparse(dims, 7, 200, 30)
+    scene, bm = ctx.scene_from_dense(g, spare_bricks=20000), oracle.HostBrickMap.from_dense(g)
+    rng = np.random.default_rng(radius)
+    poses = [((-60.0, -80.0, 400.0), (270.0, 140.0, 100.0)), ((600.0, 350.0, -40.0), (200.0, 100.0, 200.0))]
+    for _ in range(3):
+        e = _edits(rng, dims, 24, radius)
+        scene.edit([meso.SphereEdit((ctypes.c_int32 * 3)(*c), r, m, 0) for c, r, m in e])
+        bm.edit([oracle.Sphere((ctypes.c_int32 * 3)(*c), r, m, 0) for c, r, m in e])
+        for o, t in poses:
+            both(ctx, scene, bm, o, t, 120, 80)
+    path = str(tmp_path / "scene.bin")
+    scene.save(path)
+    again = ctx.scene_load(path)
+    for o, t in poses:
+        both(ctx, again, bm, o, t, 120, 80)
+    again.destroy()
+    scene.destroy()
