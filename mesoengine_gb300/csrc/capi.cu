@@ -163,6 +163,14 @@ meso_status meso_ctx_create(const meso_config* cfg, meso_ctx** out) {
     if (e == cudaSuccess) e = cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &cur);
     if (e == cudaSuccess && cur < keep) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
+  if (e == cudaSuccess) {
+    cudaMemPoolProps props;
+    memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = c.device;
+    e = cudaMemPoolCreate(&ctx->scene_pool, &props);
+  }
   if (e != cudaSuccess) {
     if (ctx->d_tickets) cudaFree(ctx->d_tickets);
     if (ctx->d_scratch) cudaFree(ctx->d_scratch);
@@ -180,6 +188,7 @@ void meso_ctx_destroy(meso_ctx* ctx) {
   cudaStreamSynchronize(ctx->stream);
   cudaFree(ctx->d_scratch);
   cudaFree(ctx->d_tickets);
+  cudaMemPoolDestroy(ctx->scene_pool);  // memory of scenes that still live goes with them
   cudaStreamDestroy(ctx->stream);
   delete ctx;
 }

@@ -382,7 +382,10 @@ meso_status meso_scene_load(meso_ctx* ctx, const char* path, uint64_t spare, mes
     if (ptr[b] != MESO_EMPTY_BRICK && ptr[b] >= n) return fail(MESO_ERR_INVALID_ARG, "scene_load: bad brick pointer");
   meso_scene* s = nullptr;
   MESO_TRY(scene_alloc(ctx, nx, ny, nz, n + spare, &s));
-  cudaError_t e = cudaMemcpy(s->d_ptr, ptr.data(), nb * 4, cudaMemcpyHostToDevice);
+  // the arrays are ordered after ctx->stream's allocation, the copies below
+  // are on the default stream
+  cudaError_t e = cudaStreamSynchronize(ctx->stream);
+  if (e == cudaSuccess) e = cudaMemcpy(s->d_ptr, ptr.data(), nb * 4, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && n) e = cudaMemcpy(s->d_occ, occ.data(), n * 64, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && n) e = cudaMemcpy(s->d_mat, mat.data(), n * 1024, cudaMemcpyHostToDevice);
   const int32_t alloc[4] = {(int32_t)n, 0, 0, 0};

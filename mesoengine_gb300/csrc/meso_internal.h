@@ -67,6 +67,10 @@ struct meso_ctx {
   uint32_t* d_tickets = nullptr;
   std::atomic<uint32_t> next_ticket{0};
   std::mutex mu;
+  // the scenes' device memory (see scene_alloc)
+  cudaMemPool_t scene_pool = nullptr;
+  uint64_t scene_pool_live = 0;  // bytes of live scenes, under scene_pool_mu
+  std::mutex scene_pool_mu;
 };
 
 struct meso_scene {
@@ -95,6 +99,7 @@ struct meso_scene {
   int64_t* d_alloc = nullptr;
   uint32_t* d_free = nullptr;  // free stack, capacity entries
   uint64_t bytes = 0;
+  uint64_t pool_bytes = 0;  // taken from the context's scene pool
   uint64_t live_bricks_host = 0;  // as of the last build/edit sync
 };
 
@@ -115,7 +120,10 @@ inline cudaStream_t pick_stream(meso_ctx* ctx, void* s) {
   return s ? (cudaStream_t)s : ctx->stream;
 }
 
-// Scene-layer helpers shared by the edit and serving code.
+// Scene-layer helpers shared by the edit and serving code.  A scene's arrays
+// are allocated and freed in the order of ctx->stream: work on another stream
+// must be ordered after the former (the build entry points wait for it) and
+// finished before scene_release.
 meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint64_t capacity,
                         meso_scene** out);
 void scene_release(meso_ctx* ctx, meso_scene* s);
