@@ -87,11 +87,11 @@ struct meso_scene {
   uint8_t* d_macro2 = nullptr;
   // one byte per 64x64x64-brick cell (512^3 voxels), built like d_macro2 from it
   uint8_t* d_macro3 = nullptr;
-  // Derived maps of the raymarch's region walk (9 bytes per 4x4x4-brick cell
-  // and 8 per pool slot, under 1 % of the scene; not part of `bytes`, so that
-  // a budget admits what it did without them):
-  uint8_t* d_level = nullptr;  // per 4x4x4-brick cell: 0 if occupied, else log2 of the edge in voxels of the
-                               // largest aligned empty cube it is part of (5 .. 9)
+  // Derived maps of the raymarch's region walk (a byte per brick, 8 per
+  // 4x4x4-brick cell and 8 per pool slot, a few percent of the scene at most;
+  // not part of `bytes`, so that a budget admits what it did without them):
+  uint8_t* d_level = nullptr;  // per brick: 0 if occupied, else log2 of the edge in voxels of the largest
+                               // aligned empty cube it is part of (3 .. 9)
   uint64_t* d_mask = nullptr;  // per 4x4x4-brick cell: its occupied bricks, bit x + 4y + 16z
   uint64_t* d_sub = nullptr;   // per pool slot: the non-empty 2x2x2-voxel blocks, bit x + 4y + 16z
   uint64_t capacity = 0;       // pool slots

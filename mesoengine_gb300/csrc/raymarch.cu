@@ -10,10 +10,20 @@
 // Traversal (Amanatides & Woo 1987, at two levels): bricks whose pointer is
 // empty are crossed in one coarse step; inside an occupied brick every voxel
 // advance is a fine step over the brick's 8x8x8 occupancy bits.  Boundary
-// times are recomputed from integer coordinates at every step,
-// t = (b - o) * (1/d), with correctly rounded single operations
-// (__fsub_rn/__fmul_rn...) so the results are bit-identical to a host
-// evaluation of the same sequence.  Equal boundary times break x < y < z.
+// times are computed from integer coordinates, t = (b - o) * (1/d), with
+// correctly rounded single operations (__fsub_rn/__fmul_rn...) so the results
+// are bit-identical to a host evaluation of the same sequence.  Equal boundary
+// times break x < y < z.  walk_steps is that definition; walk_regions, which
+// nearly all rays take, crosses empty space of any size in one turn of one
+// loop and gives the same bytes.
+//
+// What bounds it: the instructions of the loop (141 per warp and turn, 45 % of
+// them on the half-rate ALU pipe) and, for small images and at the end of a
+// launch, the longest ray's chain of up to about 100 turns of some 0.3 us.
+// 1920x1080, primary and shadow rays, 1024^3 terrain: 112 M warp instructions
+// with 24.4 of 32 lanes active in 142 us, where separate loops for cell jumps,
+// brick steps and voxel steps took 290 M with 16.6 lanes in 384 us; DRAM is
+// idle (1 %).
 #include <cmath>
 #include <cstring>
 
@@ -25,8 +35,7 @@ struct RayView {
   const uint32_t* ptr;
   const uint64_t* occ;
   const uint16_t* mat;
-  const uint8_t* level;  // per 4x4x4-brick cell: log2 of the edge (voxels) of the largest aligned empty cube it is part of, 0 if it is not empty
-  const uint64_t* mask;  // per 4x4x4-brick cell: its occupied bricks, bit x + 4y + 16z
+  const uint8_t* level;  // per brick: log2 of the edge (voxels) of the largest aligned empty cube it is part of, 0 if it is occupied
   const uint64_t* sub;   // per pool slot: the brick's non-empty 2x2x2-voxel blocks, bit x + 4y + 16z
   int32_t nx, ny, nz;
   int32_t cam_chunk[3];
@@ -35,8 +44,8 @@ struct RayView {
   float tan_half;
   float aspect;  // width / height, correctly rounded
   uint32_t width, height;
-  uint32_t tiles_x;
-  uint32_t tile_start;
+  float margin;          // region walk: distance (voxels) at which a position estimate settles a boundary; 0: step by step
+  uint32_t block_start;  // the launch's first block of this view
   meso_hit* out;  // this view's width*height hit records, row major
 };
 
@@ -59,15 +68,19 @@ __device__ __forceinline__ uint64_t mix64(uint64_t x) {
   return x;
 }
 
-struct InlineViews {
-  RayView v[kInlineViews];
+// The views of a launch as kernel parameters (one entry and no use where the
+// descriptors come from a device table).
+template <int kViews>
+struct Views {
+  RayView v[kViews];
 };
 
 struct RayParams {
   const RayView* table;  // device table (n_views > kInlineViews) or null
   uint32_t n_views;
-  uint32_t total_tiles;
   uint32_t tile_w, tile_h;
+  uint32_t tile_shift;   // log2 of tile_w
+  uint32_t block_shift;  // log2 of a block's tiles side by side
   float light[3];
   float inv_light[3];  // 1 / light per axis, correctly rounded (0 for a zero component)
   uint32_t shadow;
@@ -75,7 +88,6 @@ struct RayParams {
   unsigned long long* hash;  // checksum instantiation: partial sums per view (see launch_raymarch)
   uint32_t order_mul;  // CTA b takes block (b * order_mul) mod gridDim.x (0: block b)
   uint32_t cta_rows;   // 1: the output is host memory; write whole CTA rows (see the kernel)
-  float margin;        // region walk: distance (voxels) at which a position estimate settles a boundary; 0: step by step
 };
 
 struct Trav {
@@ -206,9 +218,7 @@ __device__ __noinline__ void walk_steps(const RayView& V, int bx0, int by0, int 
 // The same walk, taken a region at a time, with the same results bit for bit.
 //
 // A region is an aligned empty cube of 2^l voxels around the ray's position:
-// l = 5..9 cells of 4^3 .. 64^3 bricks (a level byte per 4^3-brick cell),
-// l = 3, 4 one brick or 2^3 bricks (the cell's 64-bit mask of its bricks),
-// l = 1, 2 blocks of 2^3 or 4^3 voxels of an occupied brick (a 64-bit mask of
+// l = 3..9 one brick to 64^3 bricks (a level byte per brick), l = 1, 2 blocks of 2^3 or 4^3 voxels of an occupied brick (a 64-bit mask of
 // its 2^3-voxel blocks), l = 0 one voxel.  Every kind is left by one and the
 // same piece of code, so the lanes of a warp stay together whatever each is
 // crossing; the former loops for cell jumps, brick steps and voxel steps ran
@@ -235,21 +245,27 @@ __device__ __noinline__ void walk_steps(const RayView& V, int bx0, int by0, int 
 // and keeps the regions' alignment.  An axis with d = 0 gets an infinite
 // 1/d, so its faces lie at infinite time and are never chosen.
 //
+constexpr float kRoundMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to the nearest integer
+constexpr int kRoundBits = 0x4B400000;      // its bits
+
 struct RayAxis {
   float o, d, i;  // mirrored origin, |d| and 1/|d| (infinite for d = 0)
   float a;        // o plus the base voxel: absolute origin, for estimates
-  int b;          // mirrored base voxel
+  int b1;         // 1 - mirrored base voxel, plus kRoundBits
   int m;          // -1 for a mirrored axis, else 0
+  int end;        // first mirrored voxel beyond the grid
 };
 
-__device__ __forceinline__ RayAxis ray_axis(int b0, float o, float d, float inv) {
+__device__ __forceinline__ RayAxis ray_axis(int b0, float o, float d, float inv, int n) {
   RayAxis A;
   A.m = d < 0.0f ? -1 : 0;
   A.o = d < 0.0f ? -o : o;
   A.d = fabsf(d);
   A.i = d == 0.0f ? kInf : fabsf(inv);
-  A.b = d < 0.0f ? -b0 : b0;
-  A.a = A.o + __int2float_rn(A.b);
+  const int b = d < 0.0f ? -b0 : b0;
+  A.a = A.o + __int2float_rn(b);
+  A.b1 = kRoundBits + 1 - b;
+  A.end = d < 0.0f ? 0 : n;
   return A;
 }
 
@@ -259,90 +275,97 @@ __device__ __forceinline__ bool regular_axis(float d) {
   return m == 0.0f || (m > 1e-30f && m < 1e30f);
 }
 
-// Time of the mirrored absolute boundary f.
-__device__ __forceinline__ float face_time(const RayAxis& A, int f) {
-  return __fmul_rn(__fsub_rn(__int2float_rn(f - A.b), A.o), A.i);
+// Time of the mirrored absolute boundary last + 1.  The conversion to float
+// (exact: the coordinate is below 2^22) is an addition in a float whose unit
+// is one, which takes the FMA pipe and 4 cycles where the convert instruction
+// takes a quarter-rate pipe.
+__device__ __forceinline__ float face_time(const RayAxis& A, int last) {
+  const float b = __fsub_rn(__int_as_float(last + A.b1), kRoundMagic);
+  return __fmul_rn(__fsub_rn(b, A.o), A.i);
 }
 
 // Voxel (mirrored) at time t along an axis that was not stepped, by the
 // definition's own operations: floor(o + d*t).
 __device__ __forceinline__ int entry_voxel(const RayAxis& A, float t) {
   const float x = __fadd_rn(A.o, __fmul_rn(A.d, t));
-  return (__float2int_rd(A.m ? -x : x) ^ A.m) + A.b;
+  return (__float2int_rd(A.m ? -x : x) ^ A.m) + kRoundBits + 1 - A.b1;
 }
 
-constexpr float kRoundMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to the nearest integer
-
-// Units (2^ush voxels) along one axis at time t: index of the unit that the
-// position estimate lies in, and how far the estimate is from a unit's middle.
-__device__ __forceinline__ int estimate(const RayAxis& A, float t, float inv_unit, int ush, float& off) {
+// Position along one axis at time t in units of 1 / inv_unit voxels: the unit
+// that the estimate lies in (its first voxel), and how far the estimate is
+// from that unit's middle.
+__device__ __forceinline__ int estimate(const RayAxis& A, float t, float inv_unit, uint32_t unit, uint32_t bias,
+                                       float& off) {
   const float q = __fmaf_rn(__fmaf_rn(A.d, t, A.a), inv_unit, -0.5f);
   const float s = __fadd_rn(q, kRoundMagic);
   off = __fsub_rn(q, __fsub_rn(s, kRoundMagic));
-  return (__float_as_int(s) - 0x4B400000) << ush;
+  return (int)((uint32_t)__float_as_int(s) * unit + bias);
 }
 
 // An estimate too close to a unit boundary: the boundary's own time decides
 // on which side of it the ray is at tE (`first`: this axis wins ties).
-__device__ __forceinline__ int settle(float o, float i, int b, int e, int ush, float off, float tE, bool first) {
-  const int bd = off > 0.0f ? e + (1 << ush) : e;  // the boundary next to the estimate
-  const float tb = __fmul_rn(__fsub_rn(__int2float_rn(bd - b), o), i);
-  return (tb < tE || (tb == tE && first)) ? bd : bd - (1 << ush);
+__device__ __forceinline__ int settle(const RayAxis& A, int e, int unit, float off, float tE, bool first) {
+  const int b = off > 0.0f ? e + unit : e;  // the boundary next to the estimate
+  const float tb = face_time(A, b - 1);
+  return (tb < tE || (tb == tE && first)) ? b : b - unit;
 }
 
 __device__ __forceinline__ void walk_regions(const RayView& V, const RayAxis& X, const RayAxis& Y, const RayAxis& Z,
                                              float margin, int vx, int vy, int vz, float t, int ea, Trav& r) {
-  const int CX = V.nx >> 5, CY = V.ny >> 5;  // cells of 4x4x4 bricks
-  int x = vx ^ X.m, y = vy ^ Y.m, z = vz ^ Z.m;  // mirrored position
+  const uint32_t NBX = (uint32_t)V.nx >> 3, NBY = (uint32_t)V.ny >> 3;
+  const uint32_t flip = (X.m & 7) | (Y.m & 56) | (Z.m & 448);  // the same, of a voxel's 3+3+3 bits in its brick
+  int x = vx ^ X.m, y = vy ^ Y.m, z = vz ^ Z.m;            // mirrored position
   // steps: += position where a run of its kind ends, -= where it begins
   int cs = 0, fs = -(x + y + z);
+  // the unit of the position estimates (a voxel in an occupied brick, a brick
+  // elsewhere), kept and not derived from l: 6 instructions of each turn
+  float inv_unit = 1.0f;
+  uint32_t unit = 1u, bias = 0u - (uint32_t)kRoundBits;
   bool fine = true;   // in an occupied brick (the first position counts as one until looked up)
   bool look = true;   // the brick at the position has not been looked up
   uint32_t p = 0;
-  uint64_t blocks = 0;  // 2^3-voxel blocks of the current brick
+  uint2 blocks = make_uint2(0u, 0u);  // 2^3-voxel blocks of the current brick
   r.hit = 0;
   for (;;) {
-    const int ux = x ^ X.m, uy = y ^ Y.m, uz = z ^ Z.m;
     int l = 0;
     if (look) {
-      if (((unsigned)ux >= (unsigned)V.nx) | ((unsigned)uy >= (unsigned)V.ny) | ((unsigned)uz >= (unsigned)V.nz)) break;
-      const uint32_t c = (uint32_t)(ux >> 5) + (uint32_t)CX * ((uint32_t)(uy >> 5) + (uint32_t)CY * (uint32_t)(uz >> 5));
-      const uint32_t lev = __ldg(V.level + c);
-      const uint64_t bricks = __ldg(V.mask + c);
-      const int k = ((ux >> 3) & 3) | ((uy >> 1) & 12) | ((uz << 1) & 48);
-      if ((bricks >> k) & 1ull) {
-        p = __ldg(V.ptr + (uint32_t)(ux >> 3) +
-                  (uint32_t)(V.nx >> 3) * ((uint32_t)(uy >> 3) + (uint32_t)(V.ny >> 3) * (uint32_t)(uz >> 3)));
-        blocks = __ldg(V.sub + p);
+      if ((x >= X.end) | (y >= Y.end) | (z >= Z.end)) break;
+      const uint32_t brick = (uint32_t)((x ^ X.m) >> 3) +
+                             NBX * ((uint32_t)((y ^ Y.m) >> 3) + NBY * (uint32_t)((z ^ Z.m) >> 3));
+      l = __ldg(V.level + brick);
+      p = __ldg(V.ptr + brick);  // fetched beside the level: one latency instead of two where it is needed
+      if (l == 0) {
+        blocks = __ldg(reinterpret_cast<const uint2*>(V.sub) + p);
         if (!fine) {
           cs += (x >> 3) + (y >> 3) + (z >> 3);
-          // exact along the stepped axis (x, y or z is its brick's first
-          // voxel already), floor of the entry point along the others
-          if (ea != 0) x = clampi(entry_voxel(X, t), x & ~7, x | 7);
-          if (ea != 1) y = clampi(entry_voxel(Y, t), y & ~7, y | 7);
-          if (ea != 2) z = clampi(entry_voxel(Z, t), z & ~7, z | 7);
+          // floor of the entry point, in the brick (along the stepped axis
+          // that is the brick's first voxel: the point lies on its face)
+          x = clampi(entry_voxel(X, t), x & ~7, x | 7);
+          y = clampi(entry_voxel(Y, t), y & ~7, y | 7);
+          z = clampi(entry_voxel(Z, t), z & ~7, z | 7);
           fs -= x + y + z;
           fine = true;
+          inv_unit = 1.0f;
+          unit = 1u;
+          bias = 0u - (uint32_t)kRoundBits;
         }
-      } else {
-        if (fine) {
-          fs += x + y + z;
-          cs -= (x >> 3) + (y >> 3) + (z >> 3);
-          fine = false;
-        }
-        l = lev ? (int)lev : (((bricks >> (k & 42)) & 0x330033ull) ? 3 : 4);
+      } else if (fine) {
+        fs += x + y + z;
+        cs -= (x >> 3) + (y >> 3) + (z >> 3);
+        fine = false;
+        inv_unit = 0.125f;
+        unit = 8u;
+        bias = 0u - 8u * (uint32_t)kRoundBits;
       }
     }
     if (fine) {
-      const int wx = x ^ X.m, wy = y ^ Y.m, wz = z ^ Z.m;
-      const int k = ((wx >> 1) & 3) | ((wy << 1) & 12) | ((wz << 3) & 48);
-      if (!((blocks >> (k & 42)) & 0x330033ull)) {
-        l = 2;
-      } else if (!((blocks >> k) & 1ull)) {
-        l = 1;
-      } else {
-        const uint64_t w = __ldg(V.occ + (size_t)p * 8 + (wz & 7));
-        if ((w >> ((wx & 7) + 8 * (wy & 7))) & 1ull) {
+      const uint32_t v = ((x & 7) | ((y << 3) & 56) | ((z << 6) & 448)) ^ flip;  // voxel of the brick
+      const uint32_t k = ((v >> 1) & 3u) | ((v >> 2) & 12u) | ((v >> 3) & 16u);  // its block, of half the brick
+      const uint32_t half = v & 256u ? blocks.y : blocks.x;
+      l = ((half >> (k & 10u)) & 0x330033u) == 0 ? 2 : 1;
+      if ((half >> (k & 31u)) & 1u) {
+        const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(V.occ) + ((size_t)p * 16 + (v >> 5)));
+        if ((w >> (v & 31u)) & 1u) {
           r.hit = 1;
           break;
         }
@@ -351,41 +374,41 @@ __device__ __forceinline__ void walk_regions(const RayView& V, const RayAxis& X,
     }
     // ---- leave the region of 2^l voxels
     const int in = (1 << l) - 1;
-    const int fx = (x | in) + 1, fy = (y | in) + 1, fz = (z | in) + 1;
-    const float tx = face_time(X, fx), ty = face_time(Y, fy), tz = face_time(Z, fz);
-    const bool cy = ty < tx;
-    float tE = cy ? ty : tx;
-    const bool cz = tz < tE;
-    tE = cz ? tz : tE;
-    const bool az = cz, ay = cy && !cz, ax = !cy && !cz;
-    const int ush = l >= 3 ? 3 : 0;
-    const float inv_unit = l >= 3 ? 0.125f : 1.0f;
-    // a voxel has no boundary inside it to be unsure of
-    const float lim = l == 0 ? 1.0f : __fmaf_rn(-margin, inv_unit, 0.5f);
+    const int lx = x | in, ly = y | in, lz = z | in;  // the region's last voxels
+    const float tx = face_time(X, lx), ty = face_time(Y, ly), tz = face_time(Z, lz);
+    const float txy = fminf(tx, ty);
+    const bool az = tz < txy, ay = ty < tx && !az, ax = !az && !(ty < tx);
+    const float tE = fminf(txy, tz);
+    const float lim = __fmaf_rn(-margin, inv_unit, 0.5f);
     float gx, gy, gz;
-    int nx = estimate(X, tE, inv_unit, ush, gx), ny = estimate(Y, tE, inv_unit, ush, gy),
-        nz = estimate(Z, tE, inv_unit, ush, gz);
+    int nx = estimate(X, tE, inv_unit, unit, bias, gx), ny = estimate(Y, tE, inv_unit, unit, bias, gy),
+        nz = estimate(Z, tE, inv_unit, unit, bias, gz);
     const bool qx = !ax && fabsf(gx) > lim, qy = !ay && fabsf(gy) > lim, qz = !az && fabsf(gz) > lim;
     if (qx | qy | qz) {
-      if (qx) nx = settle(X.o, X.i, X.b, nx, ush, gx, tE, true);
-      if (qy) ny = settle(Y.o, Y.i, Y.b, ny, ush, gy, tE, az);
-      if (qz) nz = settle(Z.o, Z.i, Z.b, nz, ush, gz, tE, false);
+      if (qx) nx = settle(X, nx, (int)unit, gx, tE, true);
+      if (qy) ny = settle(Y, ny, (int)unit, gy, tE, az);
+      if (qz) nz = settle(Z, nz, (int)unit, gz, tE, false);
     }
-    x = ax ? fx : max(x, min(x | in, nx));
-    y = ay ? fy : max(y, min(y | in, ny));
-    z = az ? fz : max(z, min(z | in, nz));
+    if (ax) nx = lx + 1;
+    if (ay) ny = ly + 1;
+    if (az) nz = lz + 1;
+    // an entry point rounded up may lie ahead of the estimate; past the
+    // region's face it cannot be, as that face's own time is not before tE
+    x = max(x, nx);
+    y = max(y, ny);
+    z = max(z, nz);
     t = tE;
     ea = az ? 2 : (ay ? 1 : 0);
-    look = !fine || ((ax ? fx : (ay ? fy : fz)) & 7) == 0;
+    look = !fine || ((az ? lz : (ay ? ly : lx)) & 7) == 7;
   }
   if (fine) fs += x + y + z;
   else cs += (x >> 3) + (y >> 3) + (z >> 3);
   // a mirrored boundary that passes through the origin: (b - o) * (1/d) is
   // minus zero there
   if (t == 0.0f && ea >= 0) {
-    const int f = ea == 0 ? x - X.b : (ea == 1 ? y - Y.b : z - Z.b), m = ea == 0 ? X.m : (ea == 1 ? Y.m : Z.m);
+    const int f = (ea == 0 ? x + X.b1 : (ea == 1 ? y + Y.b1 : z + Z.b1)) - kRoundBits, m = ea == 0 ? X.m : (ea == 1 ? Y.m : Z.m);
     const float o = ea == 0 ? X.o : (ea == 1 ? Y.o : Z.o);
-    if (m && __int2float_rn(f) == o) t = -0.0f;
+    if (m && __int2float_rn(f - 1) == o) t = -0.0f;
   }
   r.vx = x ^ X.m;
   r.vy = y ^ Y.m;
@@ -405,7 +428,8 @@ __device__ __forceinline__ void trace(const RayView& V, float margin, int bx0, i
   const bool regions = !kStats && margin > 0.0f && regular_axis(dx) && regular_axis(dy) && regular_axis(dz) &&
                        (dx != 0.0f || dy != 0.0f || dz != 0.0f);
   if (regions) {
-    const RayAxis X = ray_axis(bx0, ox, dx, ix), Y = ray_axis(by0, oy, dy, iy), Z = ray_axis(bz0, oz, dz, iz);
+    const RayAxis X = ray_axis(bx0, ox, dx, ix, V.nx), Y = ray_axis(by0, oy, dy, iy, V.ny),
+                  Z = ray_axis(bz0, oz, dz, iz, V.nz);
     walk_regions(V, X, Y, Z, margin, vx, vy, vz, t, ea, r);
   } else {
     Trav q;
@@ -416,18 +440,16 @@ __device__ __forceinline__ void trace(const RayView& V, float margin, int bx0, i
 
 __device__ __forceinline__ void camera_ray(const RayView& V, uint32_t px, uint32_t py, float& dx, float& dy,
                                            float& dz) {
-  const float fw = __uint2float_rn(V.width), fh = __uint2float_rn(V.height);
-  const float aspect = V.aspect;
-  float sxv = __fdiv_rn(__uint2float_rn(2u * px + 1u), fw);
+  float sxv = __fdiv_rn(__uint2float_rn(2u * px + 1u), __uint2float_rn(V.width));
   sxv = __fsub_rn(sxv, 1.0f);
   sxv = __fmul_rn(sxv, V.tan_half);
-  sxv = __fmul_rn(sxv, aspect);
-  float syv = __fdiv_rn(__uint2float_rn(2u * py + 1u), fh);
+  sxv = __fmul_rn(sxv, V.aspect);
+  float syv = __fdiv_rn(__uint2float_rn(2u * py + 1u), __uint2float_rn(V.height));
   syv = __fsub_rn(1.0f, syv);
   syv = __fmul_rn(syv, V.tan_half);
-  float d0 = __fadd_rn(__fadd_rn(V.fwd[0], __fmul_rn(V.right[0], sxv)), __fmul_rn(V.up[0], syv));
-  float d1 = __fadd_rn(__fadd_rn(V.fwd[1], __fmul_rn(V.right[1], sxv)), __fmul_rn(V.up[1], syv));
-  float d2 = __fadd_rn(__fadd_rn(V.fwd[2], __fmul_rn(V.right[2], sxv)), __fmul_rn(V.up[2], syv));
+  const float d0 = __fadd_rn(__fadd_rn(V.fwd[0], __fmul_rn(V.right[0], sxv)), __fmul_rn(V.up[0], syv));
+  const float d1 = __fadd_rn(__fadd_rn(V.fwd[1], __fmul_rn(V.right[1], sxv)), __fmul_rn(V.up[1], syv));
+  const float d2 = __fadd_rn(__fadd_rn(V.fwd[2], __fmul_rn(V.right[2], sxv)), __fmul_rn(V.up[2], syv));
   float n2 = __fmul_rn(d0, d0);
   n2 = __fadd_rn(n2, __fmul_rn(d1, d1));
   n2 = __fadd_rn(n2, __fmul_rn(d2, d2));
@@ -454,9 +476,9 @@ __device__ __forceinline__ void trace_pixel(const RayView& V, uint32_t px, uint3
   const int sx = dx > 0.0f ? 1 : (dx < 0.0f ? -1 : 0);
   const int sy = dy > 0.0f ? 1 : (dy < 0.0f ? -1 : 0);
   const int sz = dz > 0.0f ? 1 : (dz < 0.0f ? -1 : 0);
-  const float ix = sx ? __fdiv_rn(1.0f, dx) : 0.0f;
-  const float iy = sy ? __fdiv_rn(1.0f, dy) : 0.0f;
-  const float iz = sz ? __fdiv_rn(1.0f, dz) : 0.0f;
+  const float ix = sx ? __frcp_rn(dx) : 0.0f;
+  const float iy = sy ? __frcp_rn(dy) : 0.0f;
+  const float iz = sz ? __frcp_rn(dz) : 0.0f;
   // slab test against [-base, N - base)
   float tnear = -kInf, tfar = kInf;
   int ea = -1;
@@ -521,7 +543,7 @@ __device__ __forceinline__ void trace_pixel(const RayView& V, uint32_t px, uint3
 #pragma unroll 1
   for (int pass = 0;; pass++) {
     Trav r;
-    trace<kStats>(V, P.margin, base_x, base_y, base_z, rox, roy, roz, rdx, rdy, rdz, rix, riy, riz, vx, vy, vz, t0, ea,
+    trace<kStats>(V, V.margin, base_x, base_y, base_z, rox, roy, roz, rdx, rdy, rdz, rix, riy, riz, vx, vy, vz, t0, ea,
                   r);
     if (kStats) {
       st[0] += r.fetches;
@@ -572,30 +594,44 @@ __device__ __forceinline__ void trace_pixel(const RayView& V, uint32_t px, uint3
 // order-sensitive hit checksum and its traced shadow rays into P.hash (the
 // serving loop's per-request summary, so the hits need not be read again).
 // Each is a separate instantiation; the timed path has none of it.
-// At most 128 threads per CTA; 8 resident CTAs per SM cap registers at 64,
-// which measured faster than the uncapped 73 (more warps to hide latency).
-template <bool kInline, int kMode>
-__global__ void __launch_bounds__(128, 8) raymarch_kernel(const RayParams P, const __grid_constant__ InlineViews iv) {
+// At most 128 threads per CTA; 8 resident CTAs per SM cap registers at 64
+// (1080p frame 149 us; 7 CTAs 154, 6 152, 9 with 56 registers 151).
+// kViews: 1 = one view and 32 = up to 32 views as kernel parameters, 0 = a
+// device table.  A block belongs to one view (a view's last block may have
+// idle warps), so the descriptor's index depends on the block alone and its
+// fields are read through the uniform path; one view's are operands in the
+// parameter bank, with no load at all.
+template <int kViews, int kMode>
+__global__ void __launch_bounds__(128, 8)
+    raymarch_kernel(const RayParams P, const __grid_constant__ Views<kViews ? kViews : 1> iv) {
   constexpr bool kStats = kMode == kStatsMode;
   const uint32_t warps = blockDim.x >> 5;
-  const uint32_t bid = P.order_mul ? (uint32_t)(((uint64_t)blockIdx.x * P.order_mul) % gridDim.x) : blockIdx.x;
-  const uint32_t tile = bid * warps + (threadIdx.x >> 5);
-  if (tile >= P.total_tiles) return;
-  const int lane = threadIdx.x & 31;
-  const RayView* views = kInline ? iv.v : P.table;
-  // view lookup: last view whose tile_start <= tile
-  uint32_t lo = 0, hi = P.n_views;
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (views[mid].tile_start <= tile) lo = mid;
-    else hi = mid;
+  const uint32_t bid = P.order_mul ? (blockIdx.x * P.order_mul) % gridDim.x : blockIdx.x;
+  const RayView* views = kViews ? iv.v : P.table;
+  uint32_t lo = 0;
+  if constexpr (kViews != 1) {
+    // view lookup: last view whose block_start <= bid
+    uint32_t hi = P.n_views;
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (views[mid].block_start <= bid) lo = mid;
+      else hi = mid;
+    }
   }
-  const RayView& V = views[lo];
-  const uint32_t lt = tile - V.tile_start;
-  const uint32_t tx = lt % V.tiles_x, ty = lt / V.tiles_x;
+  const RayView& V = kViews == 1 ? iv.v[0] : views[lo];
+  const uint32_t lb = bid - V.block_start;
+  const uint32_t warp = threadIdx.x >> 5;
+  const uint32_t tiles_x = (V.width + P.tile_w - 1u) >> P.tile_shift;
+  const uint32_t tiles_y = (V.height + P.tile_h - 1u) >> (5u - P.tile_shift);
+  const uint32_t blocks_x = (tiles_x + (1u << P.block_shift) - 1u) >> P.block_shift;
+  const uint32_t by = lb / blocks_x, bx = lb - by * blocks_x;
+  const uint32_t tx = (bx << P.block_shift) + (warp & ((1u << P.block_shift) - 1u));
+  const uint32_t ty = by * (warps >> P.block_shift) + (warp >> P.block_shift);
+  if (tx >= tiles_x || ty >= tiles_y) return;
+  const int lane = threadIdx.x & 31;
   const uint32_t px0 = tx * P.tile_w, py0 = ty * P.tile_h;
-  const uint32_t px = px0 + (uint32_t)lane % P.tile_w;
-  const uint32_t py = py0 + (uint32_t)lane / P.tile_w;
+  const uint32_t px = px0 + ((uint32_t)lane & (P.tile_w - 1u));
+  const uint32_t py = py0 + ((uint32_t)lane >> P.tile_shift);
   uint32_t st[4] = {0, 0, 0, 0};
   // The tile's hit records (24 B each) are staged in shared memory and
   // written back as runs of consecutive 8-byte words, one run per tile row,
@@ -620,9 +656,9 @@ __global__ void __launch_bounds__(128, 8) raymarch_kernel(const RayParams P, con
   // one), so no line crosses the CPU-GPU link in two pieces.  (Into device
   // memory the barrier costs more than it saves.)
   bool done = false;
-  if (P.cta_rows && warps == 4 && P.tile_w == 8 && P.tile_h == 4 && (bid + 1) * 4 <= P.total_tiles) {
+  if (P.cta_rows && warps == 4 && P.tile_w == 8 && P.tile_h == 4 && (bx + 1) * 4 <= tiles_x) {
     const uint32_t x0 = px0 - 8u * (threadIdx.x >> 5);  // the CTA's first pixel column
-    const bool ok = (tx & 3u) == (threadIdx.x >> 5) && px0 + 8 <= V.width && py0 + 4 <= V.height &&
+    const bool ok = px0 + 8 <= V.width && py0 + 4 <= V.height &&
                     ((reinterpret_cast<uintptr_t>(base) + (((uint64_t)py0 * V.width + x0) * 24)) & 15u) == 0 &&
                     (V.width & 1u) == 0;
     if (__syncthreads_and(ok)) {
@@ -643,12 +679,13 @@ __global__ void __launch_bounds__(128, 8) raymarch_kernel(const RayParams P, con
                      (V.width & 1u) == 0 && (P.tile_w & 1u) == 0 && px0 + P.tile_w <= V.width &&
                      py0 + P.tile_h <= V.height;
     if (vec) {
+      // the usual 8-pixel tile with its 12 chunks per row known at compile time
       const uint32_t row_vecs = row_words / 2;
 #pragma unroll
       for (int r = 0; r < 2; r++) {
         const uint32_t c = (uint32_t)lane + 32u * r;  // 16-byte chunk c of the tile (48 in all)
         if (c < 48u) {
-          const uint32_t row = c / row_vecs, q = c % row_vecs;
+          const uint32_t row = P.tile_w == 8 ? c / 12u : c / row_vecs, q = c - row * row_vecs;
           const uint4 v = reinterpret_cast<const uint4*>(sw)[c];
           reinterpret_cast<uint4*>(base + ((uint64_t)(py0 + row) * V.width + px0) * 3)[q] = v;
         }
@@ -693,19 +730,50 @@ __global__ void __launch_bounds__(128, 8) raymarch_kernel(const RayParams P, con
 
 size_t raymarch_view_table_bytes(uint32_t n_views) { return sizeof(RayView) * (size_t)n_views; }
 
-// CTAs take their blocks in a strided order, b * 7919 mod blocks (a bijection
-// unless blocks is a multiple of the prime 7919), so the cheap sky tiles and
-// the expensive terrain tiles of a frame mix over the whole launch: the hit
-// records leave at an even rate, which the CPU-GPU link needs when they are
-// written to page-locked host memory (1080p end to end 0.48 -> 0.39 ms; the
-// frame into device memory is unchanged).
-static uint32_t block_order_mul(uint32_t blocks) { return blocks > 1 && blocks % 7919u ? 7919u : 0u; }
+// Into page-locked host memory the CTAs take their blocks in a strided order,
+// b * 7919 mod blocks (a bijection unless blocks is a multiple of the prime
+// 7919), so the cheap sky tiles and the expensive terrain tiles of a frame mix
+// over the whole launch and the hit records leave at an even rate, which the
+// CPU-GPU link needs (1080p end to end 0.48 -> 0.39 ms).  Into device memory
+// they go in their own order: neighbouring blocks run at the same time and
+// share what they fetch (1080p with shadow rays 149.5 us strided, 141.7 us in
+// order; 40 served requests 4.53 and 4.45 ms).  Launches of more than
+// 2^32 / 7919 blocks (278 Mpixel) keep their order: the product must fit 32 bits.
+static uint32_t block_order_mul(uint32_t blocks, bool host_out) {
+  return host_out && blocks > 1 && blocks < 542000u && blocks % 7919u ? 7919u : 0u;
+}
 
-// Fills the host descriptors out[0 .. n) of views scenes/cams[0 .. n).  tiles
-// and hits are running totals over all views of the launch (in: those of
-// the views before these; out: including them).
+// A view's margin in the region walk: 2^-20 of the largest coordinate that its
+// rays reach (twice the error bound derived at walk_regions), or 0 (every ray
+// step by step) outside what that bound was derived for: coordinates beyond
+// 2^17 voxels, an origin that is not finite.
+static float region_margin(const meso_scene* s, const meso_camera& c) {
+  const int32_t n[3] = {s->nx, s->ny, s->nz};
+  float R = 0.0f;
+  for (int a = 0; a < 3; a++) {
+    const float r = 32.0f * fabsf((float)c.origin_chunk[a]) + (float)n[a] + fabsf(c.origin_frac[a]) + 64.0f;
+    if (!(r < 131072.0f)) return 0.0f;
+    R = r > R ? r : R;
+  }
+  return R * 4.76837158203125e-7f;
+}
+
+// Tiles of a block side by side, as a power of two: two by two for four warps
+// (the block's rays stay in a squarer patch of the scene and share more of its
+// lines in L1: 1080p 155.6 -> 151.3 us, 40 served requests 4.85 -> 4.59 ms);
+// four in a row where whole rows of the block are written at once (host output).
+static uint32_t block_tiles_shift(uint32_t wpc, bool rows) { return wpc == 4 ? (rows ? 2u : 1u) : (wpc == 2 ? 1u : 0u); }
+
+// Running totals over the views of a launch.
+struct ViewTotals {
+  uint64_t tiles = 0, blocks = 0, hits = 0;
+};
+
+// Fills the host descriptors out[0 .. n) of views scenes/cams[0 .. n) for
+// blocks of wpc warps, after those that the totals count already.
 static void fill_views(const meso_scene* const* scenes, const meso_camera* cams, uint32_t n, uint32_t tw, uint32_t th,
-                       meso_hit* d_hits, meso_hit* const* view_out, RayView* out, uint64_t& tiles, uint64_t& hits) {
+                       uint32_t wpc, uint32_t bsh, meso_hit* d_hits, meso_hit* const* view_out, RayView* out,
+                       ViewTotals& tot) {
   for (uint32_t v = 0; v < n; v++) {
     const meso_scene* s = scenes[v];
     const meso_camera& c = cams[v];
@@ -713,7 +781,6 @@ static void fill_views(const meso_scene* const* scenes, const meso_camera* cams,
     memset(&V, 0, sizeof(V));
     V.ptr = s->d_ptr;
     V.level = s->d_level;
-    V.mask = s->d_mask;
     V.sub = s->d_sub;
     V.occ = s->d_occ;
     V.mat = s->d_mat;
@@ -731,29 +798,15 @@ static void fill_views(const meso_scene* const* scenes, const meso_camera* cams,
     V.aspect = (float)c.width / (float)c.height;  // IEEE conversions and division, as on the device
     V.width = c.width;
     V.height = c.height;
-    V.tiles_x = (c.width + tw - 1) / tw;
-    const uint32_t tiles_y = (c.height + th - 1) / th;
-    V.tile_start = (uint32_t)tiles;
-    V.out = view_out && view_out[v] ? view_out[v] : d_hits + hits;
-    tiles += (uint64_t)V.tiles_x * tiles_y;
-    hits += (uint64_t)c.width * c.height;
+    V.margin = region_margin(s, c);
+    V.block_start = (uint32_t)tot.blocks;
+    V.out = view_out && view_out[v] ? view_out[v] : d_hits + tot.hits;
+    const uint32_t tiles_x = (c.width + tw - 1) / tw, tiles_y = (c.height + th - 1) / th;
+    const uint32_t bw = 1u << bsh, bh = wpc >> bsh;
+    tot.tiles += (uint64_t)tiles_x * tiles_y;
+    tot.blocks += (uint64_t)((tiles_x + bw - 1) / bw) * ((tiles_y + bh - 1) / bh);
+    tot.hits += (uint64_t)c.width * c.height;
   }
-}
-
-// The region walk's margin for a launch: 2^-20 of the largest coordinate a
-// ray of the views reaches (twice the error bound derived at walk_regions),
-// or 0 (every ray step by step) where a view lies outside what that bound was
-// derived for: coordinates beyond 2^17 voxels, an origin that is not finite.
-static float region_margin(const meso_scene* const* scenes, const meso_camera* cams, uint32_t n_views) {
-  float R = 0.0f;
-  for (uint32_t v = 0; v < n_views; v++)
-    for (int a = 0; a < 3; a++) {
-      const int n = a == 0 ? scenes[v]->nx : (a == 1 ? scenes[v]->ny : scenes[v]->nz);
-      const float c = 32.0f * fabsf((float)cams[v].origin_chunk[a]) + (float)n + fabsf(cams[v].origin_frac[a]) + 64.0f;
-      if (!(c < 131072.0f)) return 0.0f;
-      R = c > R ? c : R;
-    }
-  return R * 9.5367431640625e-7f;
 }
 
 }  // namespace meso
@@ -783,21 +836,27 @@ __global__ void view_fill_kernel(const __grid_constant__ ViewBatch b, uint32_t n
 
 // Writes the descriptors of n_views views into the device table d_table,
 // stream-ordered before the launch that reads it: one small kernel per 64
-// views, the descriptors travelling as its parameters.  *tiles receives the
-// total tiles of the views.
+// views, the descriptors travelling as its parameters.
 static meso_status stage_view_table(const meso_scene* const* scenes, const meso_camera* cams, uint32_t n_views,
-                                    uint32_t tw, uint32_t th, meso_hit* d_hits, meso_hit* const* view_out,
-                                    RayView* d_table, cudaStream_t st, uint64_t* tiles) {
+                                    uint32_t tw, uint32_t th, uint32_t wpc, uint32_t bsh,
+                                    meso_hit* d_hits, meso_hit* const* view_out, RayView* d_table, cudaStream_t st, ViewTotals& tot) {
   ViewBatch batch;
-  uint64_t t = 0, hits = 0;
   for (uint32_t v0 = 0; v0 < n_views; v0 += kFillViews) {
     const uint32_t n = n_views - v0 < kFillViews ? n_views - v0 : kFillViews;
-    fill_views(scenes + v0, cams + v0, n, tw, th, d_hits, view_out ? view_out + v0 : nullptr, batch.v, t, hits);
+    fill_views(scenes + v0, cams + v0, n, tw, th, wpc, bsh, d_hits, view_out ? view_out + v0 : nullptr, batch.v, tot);
     view_fill_kernel<<<1, 128, 0, st>>>(batch, n, d_table + v0);
     MESO_CUDA_TRY(cudaGetLastError());
   }
-  *tiles = t;
   return MESO_OK;
+}
+
+// Launches one mode's kernel over the totals' blocks.
+template <int kViews>
+static void launch_mode(const RayParams& P, const Views<kViews ? kViews : 1>& iv, uint32_t blocks, uint32_t wpc,
+                        cudaStream_t st) {
+  if (P.stats) raymarch_kernel<kViews, kStatsMode><<<blocks, wpc * 32, 0, st>>>(P, iv);
+  else if (P.hash) raymarch_kernel<kViews, kHashMode><<<blocks, wpc * 32, 0, st>>>(P, iv);
+  else raymarch_kernel<kViews, kPlain><<<blocks, wpc * 32, 0, st>>>(P, iv);
 }
 
 meso_status launch_raymarch(meso_ctx* ctx, const meso_scene* const* scenes, const meso_camera* cams,
@@ -825,8 +884,9 @@ meso_status launch_raymarch(meso_ctx* ctx, const meso_scene* const* scenes, cons
   P.n_views = n_views;
   P.tile_w = tw;
   P.tile_h = th;
+  P.tile_shift = (uint32_t)__builtin_ctz(tw);
+  P.block_shift = block_tiles_shift(wpc, host_out);
   P.shadow = (flags & MESO_RAY_SHADOW) ? 1u : 0u;
-  P.margin = region_margin(scenes, cams, n_views);
   if (light)
     for (int a = 0; a < 3; a++) {
       P.light[a] = light[a];
@@ -835,33 +895,29 @@ meso_status launch_raymarch(meso_ctx* ctx, const meso_scene* const* scenes, cons
   P.stats = d_stats;
   P.hash = d_hash;
   P.cta_rows = host_out ? 1u : 0u;
-  static InlineViews empty_views;  // zero-initialised
-  uint64_t tiles;
+  ViewTotals tot;
   if (n_views <= (uint32_t)kInlineViews) {
-    InlineViews iv;
-    tiles = 0;
-    uint64_t hits = 0;
-    fill_views(scenes, cams, n_views, tw, th, d_hits, view_out, iv.v, tiles, hits);
-    if (tiles >= (1ull << 31)) return fail(MESO_ERR_INVALID_ARG, "raymarch: too many tiles");
-    P.total_tiles = (uint32_t)tiles;
-    const uint32_t blocks = (uint32_t)((tiles + wpc - 1) / wpc);
-    P.order_mul = block_order_mul(blocks);
-    if (d_stats) raymarch_kernel<true, kStatsMode><<<blocks, wpc * 32, 0, st>>>(P, iv);
-    else if (d_hash) raymarch_kernel<true, kHashMode><<<blocks, wpc * 32, 0, st>>>(P, iv);
-    else raymarch_kernel<true, kPlain><<<blocks, wpc * 32, 0, st>>>(P, iv);
+    Views<kInlineViews> iv;
+    fill_views(scenes, cams, n_views, tw, th, wpc, P.block_shift, d_hits, view_out, iv.v, tot);
+    if (tot.tiles >= (1ull << 31)) return fail(MESO_ERR_INVALID_ARG, "raymarch: too many tiles");
+    P.order_mul = block_order_mul((uint32_t)tot.blocks, P.cta_rows != 0);
+    if (n_views == 1) {
+      Views<1> one;
+      one.v[0] = iv.v[0];
+      launch_mode<1>(P, one, (uint32_t)tot.blocks, wpc, st);
+    } else {
+      launch_mode<kInlineViews>(P, iv, (uint32_t)tot.blocks, wpc, st);
+    }
   } else {
     if (!d_view_table || view_table_bytes < raymarch_view_table_bytes(n_views))
       return fail(MESO_ERR_INVALID_ARG, "raymarch: view table too small");
-    MESO_TRY(stage_view_table(scenes, cams, n_views, tw, th, d_hits, view_out, static_cast<RayView*>(d_view_table),
-                              st, &tiles));
-    if (tiles >= (1ull << 31)) return fail(MESO_ERR_INVALID_ARG, "raymarch: too many tiles");
-    P.total_tiles = (uint32_t)tiles;
+    MESO_TRY(stage_view_table(scenes, cams, n_views, tw, th, wpc, P.block_shift, d_hits, view_out,
+                              static_cast<RayView*>(d_view_table), st, tot));
+    if (tot.tiles >= (1ull << 31)) return fail(MESO_ERR_INVALID_ARG, "raymarch: too many tiles");
     P.table = static_cast<const RayView*>(d_view_table);
-    const uint32_t blocks = (uint32_t)((tiles + wpc - 1) / wpc);
-    P.order_mul = block_order_mul(blocks);
-    if (d_stats) raymarch_kernel<false, kStatsMode><<<blocks, wpc * 32, 0, st>>>(P, empty_views);
-    else if (d_hash) raymarch_kernel<false, kHashMode><<<blocks, wpc * 32, 0, st>>>(P, empty_views);
-    else raymarch_kernel<false, kPlain><<<blocks, wpc * 32, 0, st>>>(P, empty_views);
+    P.order_mul = block_order_mul((uint32_t)tot.blocks, P.cta_rows != 0);
+    static Views<1> unused;  // zero-initialised; the table path does not read it
+    launch_mode<0>(P, unused, (uint32_t)tot.blocks, wpc, st);
   }
   ctx->launches.fetch_add(1);
   MESO_CUDA_TRY(cudaGetLastError());
@@ -885,7 +941,7 @@ meso_status launch_raymarch(meso_ctx* ctx, const meso_scene* const* scenes, cons
 // Limits and behaviour:
 //  - at most kNoAllocViews (512) views per call; more is rejected with
 //    MESO_ERR_INVALID_ARG;
-//  - the array (512 x 152 B = 76 KiB) stays resident on every device that
+//  - the array (512 x 144 B = 72 KiB) stays resident on every device that
 //    loads the library until the process exits;
 //  - the calling thread's current device must be the context's device;
 //  - the first call on a device looks up the array's device address (with
@@ -898,7 +954,7 @@ namespace meso {
 namespace {
 
 constexpr uint32_t kNoAllocViews = 512;
-static_assert(sizeof(RayView) == 152, "the documented size of the fixed view table is 512 x 152 bytes");
+static_assert(sizeof(RayView) == 144, "the documented size of the fixed view table is 512 x 144 bytes");
 static __device__ __align__(256) unsigned char g_noalloc_views[kNoAllocViews * sizeof(RayView)];
 
 std::mutex g_noalloc_mu;
@@ -955,23 +1011,23 @@ extern "C" meso_status meso_raymarch_noalloc(meso_ctx* ctx, const meso_scene* co
   memset(&P, 0, sizeof(P));
   P.table = static_cast<const RayView*>(table);
   P.n_views = n_views;
-  P.total_tiles = (uint32_t)tiles;
   P.tile_w = tw;
   P.tile_h = th;
+  P.tile_shift = (uint32_t)__builtin_ctz(tw);
+  P.block_shift = block_tiles_shift(wpc, false);
   P.shadow = (flags & MESO_RAY_SHADOW) ? 1u : 0u;
-  P.margin = region_margin(scenes, h_cams, n_views);
   if (light)
     for (int a = 0; a < 3; a++) {
       P.light[a] = light[a];
       P.inv_light[a] = light[a] != 0.0f ? 1.0f / light[a] : 0.0f;  // IEEE division, as __fdiv_rn
     }
   const cudaStream_t st = pick_stream(ctx, stream);
-  MESO_TRY(stage_view_table(scenes, h_cams, n_views, tw, th, d_hits, nullptr, static_cast<RayView*>(table), st,
-                            &tiles));
-  static InlineViews unused_inline;  // zero-initialised; the table path does not read it
-  const uint32_t blocks = (uint32_t)((tiles + wpc - 1) / wpc);
-  P.order_mul = block_order_mul(blocks);
-  raymarch_kernel<false, kPlain><<<blocks, wpc * 32, 0, st>>>(P, unused_inline);
+  ViewTotals tot;
+  MESO_TRY(stage_view_table(scenes, h_cams, n_views, tw, th, wpc, P.block_shift, d_hits, nullptr,
+                            static_cast<RayView*>(table), st, tot));
+  P.order_mul = block_order_mul((uint32_t)tot.blocks, P.cta_rows != 0);
+  static Views<1> unused;  // zero-initialised; the table path does not read it
+  launch_mode<0>(P, unused, (uint32_t)tot.blocks, wpc, st);
   ctx->launches.fetch_add(1);
   MESO_CUDA_TRY(cudaGetLastError());
   return MESO_OK;

@@ -309,7 +309,8 @@ __global__ void __launch_bounds__(kDenseThreads) dense_flag_kernel(const T* grid
 // layers per store and a brick's 8 occupancy words leave together.
 template <typename T, bool kWide>
 __global__ void __launch_bounds__(kDenseThreads) dense_fill_kernel(const T* grid, int nx, int ny, uint64_t nb,
-                                                                   const uint32_t* ptr, uint64_t* occ, uint16_t* mat) {
+                                                                   const uint32_t* ptr, uint64_t* occ, uint16_t* mat,
+                                                                   uint64_t* sub) {
   __shared__ uint4 rows[kDenseThreads / 32][8][kDenseBricks + 1];
   __shared__ uint64_t words[kDenseBricks][9];
   __shared__ uint32_t slots[kDenseBricks];
@@ -338,6 +339,15 @@ __global__ void __launch_bounds__(kDenseThreads) dense_fill_kernel(const T* grid
     const uint32_t s = slots[brick];
     if (s != MESO_EMPTY_BRICK)
       reinterpret_cast<uint4*>(mat)[(size_t)s * 64 + z * 8 + (lane & 7)] = rows[z][lane & 7][brick];
+  }
+  if (z == 0 && slot != MESO_EMPTY_BRICK) {
+    uint32_t w[16];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      w[2 * k] = (uint32_t)words[lane][k];
+      w[2 * k + 1] = (uint32_t)(words[lane][k] >> 32);
+    }
+    sub[slot] = sub_mask(w);
   }
   const int brick = threadIdx.x >> 3;
   const uint32_t s = slots[brick];
@@ -619,13 +629,13 @@ __global__ void macro3_kernel(const uint8_t* macro2, int bx, int by, int bz, uin
   if (lane == 0) macro3[i] = set ? 1 : 0;
 }
 
-// Level bytes: per 4x4x4-brick cell log2 of the edge, in voxels, of the
-// largest aligned cube of empty space that the cell is part of and that lies
-// in the grid (9: 64^3 bricks, 8: 32^3, 7: 16^3, 6: 8^3, 5: the cell), 0 if
-// the cell is occupied.  The cells of one 64^3-brick cell depend on nothing
-// outside it, so an edit recomputes those of the 64^3-brick cells it touches
-// (list; 4096 threads each), a build all of them.
-__global__ void level_kernel(const uint8_t* macro, const uint8_t* macro2, const uint8_t* macro3, int bx, int by,
+// Level bytes: per brick log2 of the edge, in voxels, of the largest aligned
+// cube of empty space that it is part of and that lies in the grid (9: 64^3
+// bricks .. 3: the brick), 0 if it is occupied; one thread per 4x4x4-brick
+// cell.  The bricks of one 64^3-brick cell depend on nothing outside it, so an
+// edit recomputes those of the 64^3-brick cells it touches (list; 4096 threads
+// each), a build all of them.
+__global__ void level_kernel(const uint64_t* mask, const uint8_t* macro, const uint8_t* macro2, const uint8_t* macro3, int bx, int by,
                              int bz, uint8_t* level, const uint32_t* list, uint64_t n) {
   const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= n) return;
@@ -656,14 +666,30 @@ __global__ void level_kernel(const uint8_t* macro, const uint8_t* macro2, const 
     return any == 0;
   };
   const uint32_t i = (uint32_t)cx + (uint32_t)mx * ((uint32_t)cy + (uint32_t)my * (uint32_t)cz);
-  int l;
-  if (macro[i]) l = 0;
+  uint32_t l;
+  const uint64_t bricks = mask[i];
+  if (bricks) l = 0;
   else if (!macro3[(uint32_t)(cx >> 4) + (uint32_t)m3x * ((uint32_t)(cy >> 4) + (uint32_t)m3y * (uint32_t)(cz >> 4))]) l = 9;
   else if (block_empty(macro2, cx >> 2, cy >> 2, cz >> 2, m2x, m2y, m2z)) l = 8;
   else if (!macro2[(uint32_t)(cx >> 2) + (uint32_t)m2x * ((uint32_t)(cy >> 2) + (uint32_t)m2y * (uint32_t)(cz >> 2))]) l = 7;
   else if (block_empty(macro, cx, cy, cz, mx, my, mz)) l = 6;
   else l = 5;
-  level[i] = (uint8_t)l;
+  // 16 rows of 4 bricks, a byte each
+  uint32_t* dst = reinterpret_cast<uint32_t*>(level) + (size_t)cx + (size_t)mx * ((size_t)cy * 4 + (size_t)by * ((size_t)cz * 4));
+#pragma unroll
+  for (int k = 0; k < 16; k++) {
+    uint32_t v = l * 0x01010101u;
+    if (bricks) {
+      const int y = k & 3, z = k >> 2;
+#pragma unroll
+      for (int x = 0; x < 4; x++) {
+        const bool set = (bricks >> (x + 4 * y + 16 * z)) & 1ull;
+        const bool block = (bricks >> ((x & 2) + 4 * (y & 2) + 16 * (z & 2))) & 0x330033ull;
+        v |= (set ? 0u : (block ? 3u : 4u)) << (8 * x);
+      }
+    }
+    dst[(size_t)mx * ((size_t)(k & 3) + (size_t)by * (size_t)(k >> 2))] = v;
+  }
 }
 
 // d_sub of `slots` consecutive pool slots, one thread each.
@@ -729,18 +755,14 @@ meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint6
   uint8_t* maps = nullptr;
   uint8_t* small = nullptr;
   cudaError_t e = take(&s->d_ptr, nb * 4);
-  if (e == cudaSuccess) e = take(&maps, nm * 10 + nm2 + nm3);
+  if (e == cudaSuccess) e = take(&maps, nm * (8 + 64 + 1) + nm2 + nm3);
   if (e == cudaSuccess) {
-    s->d_mask = reinterpret_cast<uint64_t*>(maps);
+    s->d_mask = reinterpret_cast<uint64_t*>(maps);  // written whole by rebuild_macro
     s->d_level = maps + nm * 8;
-    s->d_macro = s->d_level + nm;
+    s->d_macro = s->d_level + nm * 64;
     s->d_macro2 = s->d_macro + nm;
     s->d_macro3 = s->d_macro2 + nm2;
-    // until the maps are built nothing is known to be empty
-    e = cudaMemsetAsync(maps, 0xFF, nm * 8, st);
   }
-  if (e == cudaSuccess) e = cudaMemsetAsync(s->d_level, 0, nm * 2, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(s->d_macro2, 1, nm2 + nm3, st);
   if (e == cudaSuccess) e = take(&s->d_occ, nslot * 64);
   if (e == cudaSuccess) e = take(&s->d_mat, nslot * 1024);
   if (e == cudaSuccess) e = take(&small, nslot * 12 + 16);
@@ -790,7 +812,7 @@ meso_status rebuild_macro(meso_ctx* ctx, meso_scene* s, const uint32_t* d_cells,
                                                                           s->d_macro3, d_cells3, n3);
   const uint64_t levels = d_cells3 ? (uint64_t)n3 << 12 : n_macro_of(s);
   if (levels)
-    level_kernel<<<(unsigned)((levels + 255) / 256), 256, 0, st>>>(s->d_macro, s->d_macro2, s->d_macro3, s->bx, s->by,
+    level_kernel<<<(unsigned)((levels + 127) / 128), 128, 0, st>>>(s->d_mask, s->d_macro, s->d_macro2, s->d_macro3, s->bx, s->by,
                                                                     s->bz, s->d_level, d_cells3, levels);
   ctx->launches.fetch_add(4);
   MESO_CUDA_TRY(cudaGetLastError());
@@ -807,7 +829,6 @@ meso_status rebuild_sub(meso_ctx* ctx, meso_scene* s, uint64_t slots, cudaStream
 
 static meso_status finish_pools(meso_ctx* ctx, meso_scene* s, uint64_t count, cudaStream_t st) {
   MESO_TRY(rebuild_macro(ctx, s, nullptr, 0, st));
-  MESO_TRY(rebuild_sub(ctx, s, count, st));
   int32_t init[4] = {(int32_t)count, 0, 0, 0};
   MESO_CUDA_TRY(cudaMemcpyAsync(s->d_alloc, init, 16, cudaMemcpyHostToDevice, st));
   MESO_CUDA_TRY(cudaStreamSynchronize(st));
@@ -864,7 +885,8 @@ meso_status scene_create_terrain(meso_ctx* ctx, const meso_terrain* t, uint64_t 
     cudaMemcpyAsync(s->d_ptr, d_ptr_tmp, nb * 4, cudaMemcpyDeviceToDevice, st);
     terrain_brick_kernel<true><<<grid_for(nb), 256, 0, st>>>(T, d_h, d_hmax, d_flags, s->d_ptr, s->d_occ, s->d_mat);
     ctx->launches.fetch_add(1);
-    rc = finish_pools(ctx, s, count, st);
+    rc = rebuild_sub(ctx, s, count, st);
+    if (rc == MESO_OK) rc = finish_pools(ctx, s, count, st);
   }
   cudaFreeAsync(d_h, st);
   cudaFreeAsync(d_hmax, st);
@@ -908,9 +930,11 @@ static meso_status build_from_device_grid(meso_ctx* ctx, const T* d_grid, int32_
   if (rc == MESO_OK) {
     cudaMemcpyAsync(s->d_ptr, d_ptr_tmp, nb * 4, cudaMemcpyDeviceToDevice, st);
     if (wide)
-      dense_fill_kernel<T, true><<<blocks, kDenseThreads, 0, st>>>(d_grid, nx, ny, nb, s->d_ptr, s->d_occ, s->d_mat);
+      dense_fill_kernel<T, true><<<blocks, kDenseThreads, 0, st>>>(d_grid, nx, ny, nb, s->d_ptr, s->d_occ, s->d_mat,
+                                                                     s->d_sub);
     else
-      dense_fill_kernel<T, false><<<blocks, kDenseThreads, 0, st>>>(d_grid, nx, ny, nb, s->d_ptr, s->d_occ, s->d_mat);
+      dense_fill_kernel<T, false><<<blocks, kDenseThreads, 0, st>>>(d_grid, nx, ny, nb, s->d_ptr, s->d_occ, s->d_mat,
+                                                                      s->d_sub);
     ctx->launches.fetch_add(1);
     rc = finish_pools(ctx, s, count, st);
   }

@@ -122,3 +122,22 @@ def test_maps_follow_edits(ctx, radius, tmp_path):
         both(ctx, again, bm, o, t, 120, 80)
     again.destroy()
     scene.destroy()
+
+
+@pytest.mark.parametrize("tile_w", [4, 8, 16, 32])
+@pytest.mark.parametrize("warps", [1, 2, 3, 4])
+def test_every_block_shape(ctx, warps, tile_w):
+    # images that end inside a tile, a row of tiles and a block, of one tile
+    # and of less; one view, several as parameters, and a table of them
+    g = sparse((96, 160, 64), 5, 60, 12)
+    bm = oracle.HostBrickMap.from_dense(g)
+    c = meso.Context(0, ray_warps_per_cta=warps, ray_tile_w=tile_w, ray_tile_h=32 // tile_w)
+    scene = c.scene_from_dense(g)
+    pose = ((-31.0, -17.0, 90.0), (48.0, 80.0, 32.0))
+    sizes = [(1, 1), (7, 3), (33, 9), (64, 32), (65, 33), (3, 70)]
+    for n in (1, len(sizes), 36):
+        cams = [sizes[k % len(sizes)] for k in range(n)]
+        got = c.raymarch(scene, [meso.camera(*pose, w, h) for w, h in cams])
+        same(got, oracle.raymarch(bm, [oracle.camera(*pose, w, h) for w, h in cams]))
+    scene.destroy()
+    c.close()
