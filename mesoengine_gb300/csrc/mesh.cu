@@ -18,20 +18,18 @@
 //     bricks by the whole CTA, after the chunk has been picked out of a
 //     ticket of chunks tested together against the scene's cell map); the
 //     one-voxel occupancy halo is read with plain loads while it lands;
-//  2. masks: lanes = x; every row (y,z) becomes bit-packed words with warp
-//     ballots: occupancy and material-equality with the -x, -y and -z
-//     neighbour, plus warp-transposed copies (bits over y) for the X faces;
+//  2. masks: a lane takes 8 voxels of a row with one wide load, a warp 8 rows;
+//     packed 16-bit (8-bit) operations give the byte of the row's occupancy
+//     word and of its material-equality words with the -x, -y and -z
+//     neighbour; warp-transposed copies (bits over y) serve the X faces;
 //     face masks occ & ~shift(occ) are recomputed from these where needed;
-//  3. faces whose quad cannot depend on the scan order are peeled off
-//     first: isolated faces (no same-material face neighbour in their plane)
-//     become 1x1 quads through a warp-balanced expansion with one output
-//     reservation per warp and chunk, and two-face components become 2x1 or
-//     1x2 quads at the start of their slice's greedy;
-//  4. greedy: warp = slice with non-isolated faces, lane = row; rows are
-//     scanned with run-length bit tricks (Lysenko's order: first unconsumed
-//     face, widen along u while the material matches, grow along v while the
-//     whole run matches); quads are staged per warp in shared memory and
-//     appended to global memory with one atomic per 64 quads.
+//  3. sweep: one warp per face direction, lane = slice, row after row; all quads
+//     of a row grow and start in about 30 word operations (see carry_on), and
+//     what a row leaves behind is the word of its columns that continue a quad
+//     from the row above;
+//  4. emission: from those words any warp can tell the quads that start in a
+//     row, their widths and heights; a task is 32 of the words that hold any,
+//     lane = word, and the output is reserved once per chunk and direction.
 #include <cudaTypedefs.h>
 
 #include <cstdio>
@@ -46,14 +44,11 @@ using namespace ::meso::dev;
 
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-// Warps w and w + 8 form a pair that shares rows (and slabs) 4(w mod 8) ..
-// 4(w mod 8) + 3: in the mask pass each builds half of the slabs' rows, in
-// the isolated-face passes each takes three of the six face directions.
-constexpr int kGroups = 12;  // word groups (direction, row) per warp: 4 rows x 3 directions
-static_assert(kWarps == 16, "eight warp pairs of 4 rows each");
+// In the mask pass warp w takes rows 8 (w mod 4) .. +7 of slabs 8 (w / 4) .. +7.
+static_assert(kWarps == 16, "four row groups by four slab groups");
 constexpr int kS = 33;               // padded row stride of 32x32 word arrays
 constexpr int kArr = 32 * kS;
-constexpr int kQBuf = 64;            // staged quads per warp
+constexpr int kFewLanes = 4;          // emission: words left when they are finished by the whole warp
 constexpr int kBrickSlot = 1040;     // bytes per staged brick (bank-spread padding)
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
@@ -66,14 +61,21 @@ struct __align__(128) MeshSmem {
   uint32_t ex[kArr], ey[kArr], ez[kArr];  // equality with -x / -y / -z neighbour, bits over x, [z][y]
   uint32_t eyt[kArr], ezt[kArr];          // equality with -y / -z neighbour, bits over y, [z][x]
   uint32_t halo[6][32];                   // -X,+X: bits y by z; -Y,+Y: bits x by z; -Z,+Z: bits x by y
-  uint64_t qbuf[kWarps][kQBuf];           // staged greedy quads per warp
-  uint32_t rest_slices[6];                // per direction: bit s = slice s holds non-isolated faces
+  // columns that continue a quad from the row above, bits and layout as the
+  // words of the direction: the odd directions'; the even directions' replace
+  // the equality with the row above, which the sweep is the last to read
+  uint32_t cont[3][kArr];
+  uint64_t quad_base[6];                  // per direction: first output index of its quads
+  uint32_t quad_next[6];                  // how many of them have their place
+  uint32_t start_rows[6][32];             // per direction and row: slices in whose row quads start
+  uint32_t start_rank[6][32];             // how many such words the rows before hold
+  uint32_t start_words[6];                // how many all rows hold
   uint64_t bar;
   int32_t chunk;
   int32_t valid;
   int32_t coord[3];
   uint32_t chunk_quads;
-  uint32_t task_next;                     // dynamic task counter of the greedy
+  uint32_t task_next;                     // dynamic task counter of the emission
   uint32_t any_solid;
   uint32_t bptr[64];  // brick maps: the chunk's 64 brick pointers
 };
@@ -127,25 +129,14 @@ struct KindTraits<MESO_SRC_GRID_U16> : KindBase<MESO_SRC_GRID_U16> {};
 template <>
 struct KindTraits<MESO_SRC_BRICKMAP> : KindBase<MESO_SRC_BRICKMAP> {};
 
-template <int KIND>
-__device__ __forceinline__ uint32_t load_mat(const uint8_t* buf, int x, int y, int z) {
-  using T = KindTraits<KIND>;
-  if constexpr (T::kBrick) {
-    const int b = (x >> 3) + 4 * (y >> 3) + 16 * (z >> 3);
-    return reinterpret_cast<const uint16_t*>(buf + b * kBrickSlot)[(x & 7) + 8 * (y & 7) + 64 * (z & 7)];
-  } else if constexpr (T::kElem == 2) {
-    return reinterpret_cast<const uint16_t*>(buf)[(z * 32 + y) * 32 + x];
-  } else {
-    return buf[(z * 32 + y) * 32 + x];
-  }
-}
-
 // Material at chunk-local linear index lin = x + 32 y + 1024 z.
 template <int KIND>
 __device__ __forceinline__ uint32_t load_mat_lin(const uint8_t* buf, uint32_t lin) {
   using T = KindTraits<KIND>;
   if constexpr (T::kBrick) {
-    return load_mat<KIND>(buf, (int)(lin & 31u), (int)((lin >> 5) & 31u), (int)(lin >> 10));
+    const uint32_t x = lin & 31u, y = (lin >> 5) & 31u, z = lin >> 10;
+    const uint32_t b = (x >> 3) + 4 * (y >> 3) + 16 * (z >> 3);
+    return reinterpret_cast<const uint16_t*>(buf + b * kBrickSlot)[(x & 7) + 8 * (y & 7) + 64 * (z & 7)];
   } else if constexpr (T::kElem == 2) {
     return reinterpret_cast<const uint16_t*>(buf)[lin];
   } else {
@@ -153,24 +144,54 @@ __device__ __forceinline__ uint32_t load_mat_lin(const uint8_t* buf, uint32_t li
   }
 }
 
-// True iff the 8 rows y0..y0+7 (y0 % 8 == 0) of slab z are all empty: one
-// 16-byte (8-byte for uint8) shared load per lane covers the 256 voxels.
+// The 8 voxels 8 seg .. of row (y, z): 16-bit materials in 4 registers, 8-bit
+// ones in 2.
 template <int KIND>
-__device__ __forceinline__ bool rows8_empty(const uint8_t* buf, int y0, int z, int lane) {
+struct Seg {
+  static constexpr int kRegs = KindTraits<KIND>::kElem == 2 ? 4 : 2;
+  uint32_t w[kRegs];
+};
+template <int KIND>
+__device__ __forceinline__ Seg<KIND> load_seg(const uint8_t* buf, int seg, int y, int z) {
   using T = KindTraits<KIND>;
-  bool nz;
-  if constexpr (T::kBrick) {
-    const int b = (lane >> 3) + 4 * (y0 >> 3) + 16 * (z >> 3);
-    const uint4 w = *reinterpret_cast<const uint4*>(buf + b * kBrickSlot + 128 * (z & 7) + 16 * (lane & 7));
-    nz = (w.x | w.y | w.z | w.w) != 0;
-  } else if constexpr (T::kElem == 2) {
-    const uint4 w = *reinterpret_cast<const uint4*>(buf + (z * 32 + y0) * 64 + 16 * lane);
-    nz = (w.x | w.y | w.z | w.w) != 0;
+  Seg<KIND> r;
+  if constexpr (T::kElem == 2) {
+    const uint8_t* a;
+    if constexpr (T::kBrick)
+      a = buf + (seg + 4 * (y >> 3) + 16 * (z >> 3)) * kBrickSlot + 128 * (z & 7) + 16 * (y & 7);
+    else
+      a = buf + (z * 32 + y) * 64 + 16 * seg;
+    const uint4 v = *reinterpret_cast<const uint4*>(a);
+    r.w[0] = v.x;
+    r.w[1] = v.y;
+    r.w[2] = v.z;
+    r.w[3] = v.w;
   } else {
-    const uint2 w = *reinterpret_cast<const uint2*>(buf + (z * 32 + y0) * 32 + 8 * lane);
-    nz = (w.x | w.y) != 0;
+    const uint2 v = *reinterpret_cast<const uint2*>(buf + (z * 32 + y) * 32 + 8 * seg);
+    r.w[0] = v.x;
+    r.w[1] = v.y;
   }
-  return !__any_sync(kFull, nz);
+  return r;
+}
+
+// Bit x set iff voxel x of a and of b differ.
+template <int KIND>
+__device__ __forceinline__ uint32_t differ(const Seg<KIND>& a, const Seg<KIND>& b) {
+  if constexpr (KindTraits<KIND>::kElem == 2) {
+    uint32_t t = 0;  // even voxels in bits 0, 2, 4, 6, odd ones 16 higher
+#pragma unroll
+    for (int k = 3; k >= 0; k--) t = t * 4u + __vminu2(a.w[k] ^ b.w[k], 0x00010001u);
+    return (t | t >> 15) & 0xFFu;
+  } else {
+    uint32_t m[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const uint32_t d = a.w[k] ^ b.w[k];
+      const uint32_t f = ((((d & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | d) >> 7) & 0x01010101u;  // bit 0 of each byte
+      m[k] = f * 0x01020408u >> 24;                                                    // .. side by side
+    }
+    return m[0] | m[1] << 4;
+  }
 }
 
 // Occupancy (material != 0) of a global voxel for halo reads; 0 outside.
@@ -436,49 +457,14 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
 // Array addressing of direction d: (slice s, row v) -> word offset.
 __device__ __forceinline__ int word_off(int d, int s, int v) { return d < 4 ? v * kS + s : s * kS + v; }
 
-// Origin voxel of a face at (dir d, slice s, column u, row v).
-__device__ __forceinline__ void face_xyz(int d, int s, int u, int v, int& x, int& y, int& z) {
-  if (d < 2) { x = s; y = u; z = v; }
-  else if (d < 4) { x = u; y = s; z = v; }
-  else { x = u; y = v; z = s; }
-}
-
 // In-plane equality arrays of direction d: E along u, V along v.
 __device__ __forceinline__ const uint32_t* e_arr(const MeshSmem& sm, int d) { return d < 2 ? sm.eyt : sm.ex; }
-__device__ __forceinline__ const uint32_t* v_arr(const MeshSmem& sm, int d) {
-  return d < 2 ? sm.ezt : (d < 4 ? sm.ez : sm.ey);
-}
+__device__ __forceinline__ uint32_t* v_arr(MeshSmem& sm, int d) { return d < 2 ? sm.ezt : (d < 4 ? sm.ez : sm.ey); }
+// After the sweep: the words of the columns that continue from the row above.
+__device__ __forceinline__ uint32_t* c_arr(MeshSmem& sm, int d) { return d & 1 ? sm.cont[d >> 1] : v_arr(sm, d); }
 
-// Face word of direction d, row v, for the slice s = lane (all lanes call):
-// the occupancy word of the slice minus that of the next slice along the
-// face normal, taken from the neighbouring lane or the halo.
-__device__ __forceinline__ uint32_t face_row(const MeshSmem& sm, int d, int v, int lane) {
-  uint32_t c, hi, lo;
-  if (d < 2) {
-    c = sm.occt[v * kS + lane];
-    hi = sm.halo[1][v];
-    lo = sm.halo[0][v];
-  } else if (d < 4) {
-    c = sm.occ[v * kS + lane];
-    hi = sm.halo[3][v];
-    lo = sm.halo[2][v];
-  } else {
-    c = sm.occ[lane * kS + v];
-    hi = sm.halo[5][v];
-    lo = sm.halo[4][v];
-  }
-  uint32_t n;
-  if ((d & 1) == 0) {
-    n = __shfl_down_sync(kFull, c, 1);
-    if (lane == 31) n = hi;
-  } else {
-    n = __shfl_up_sync(kFull, c, 1);
-    if (lane == 0) n = lo;
-  }
-  return c & ~n;
-}
-
-// Face word of direction d, slice s, for the row v = r (lanes = rows).
+// Face word of direction d, slice s, row r: the occupancy word of the slice
+// minus that of the next slice along the face normal, or of the halo.
 __device__ __forceinline__ uint32_t face_col(const MeshSmem& sm, int d, int s, int r) {
   const bool pos = (d & 1) == 0;
   const int sn = pos ? s + 1 : s - 1;
@@ -489,13 +475,146 @@ __device__ __forceinline__ uint32_t face_col(const MeshSmem& sm, int d, int s, i
   return sm.occ[s * kS + r] & ~(edge ? sm.halo[d ^ 1][r] : sm.occ[sn * kS + r]);
 }
 
-// Faces of a word with a same-material face neighbour in the plane: f the
-// faces of the row, fu / fd those of rows v-1 / v+1, e equality with the -u
-// neighbour, vv / vd equality of this row / of row v+1 with the row above.
-__device__ __forceinline__ uint32_t isolated(uint32_t f, uint32_t fu, uint32_t fd, uint32_t e, uint32_t vv,
-                                             uint32_t vd) {
-  const uint32_t left = f & e & (f << 1);
-  return f & ~(left | (left >> 1) | (f & vv & fu) | (f & vd & fd));
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Barrier of a pair of warps (ids 1.. ; 0 is __syncthreads).
+__device__ __forceinline__ void pair_sync(int g) {
+  asm volatile("bar.sync %0, 64;" ::"r"(1 + g) : "memory");
+}
+
+// The columns of a row in which the quads of the row above go on.  A: the
+// faces of the row above (each belongs to a quad), B: the first columns of its
+// quads, G: the columns whose face continues the one above in material.  A quad
+// goes on iff all of its columns are in G.
+//
+// A carry runs through consecutive ones, so adding a bit below a run of ones
+// marks the run up to its end: from the first column of each quad up as far as
+// the columns are in G; a quad whose last column is reached goes on.  From
+// those last columns the same, in reversed bits, marks the quads' columns down
+// to their first.
+__device__ __forceinline__ uint32_t carry_on(uint32_t A, uint32_t B, uint32_t G) {
+  const uint32_t joined = A & ~B;  // columns of the same quad as the one before
+  const uint32_t good = A & G, first = B & good, run = joined & good;
+  const uint32_t reach = (((run + ((first << 1) & run)) ^ run) & run) | first;
+  const uint32_t next = joined >> 1;  // columns of the same quad as the one after
+  const uint32_t rnext = __brev(next), rlast = __brev(A & ~next & reach);
+  return __brev((((rnext + ((rlast << 1) & rnext)) ^ rnext) & rnext) | rlast);
+}
+
+// The sweep of direction d (one warp, lane = slice; the warps of directions 2k
+// and 2k + 1 run together): Lysenko's scan takes the first face that no quad
+// has, widens it along u while the material matches and grows it along v while
+// the whole run matches.  Row by row that is: the quads of the row above whose
+// columns all continue go on (they were started earlier and come first), and
+// every maximal run of the faces that are left starts a quad.  Words of the
+// columns that go on are left in c_arr; the slices' quads are counted, the
+// direction's output range reserved.
+//
+// About 30 instructions per row and 32 slices, whatever the faces look like.  It
+// replaces a warp per slice that grew the runs of one row at a time, some 1300
+// instructions for a slice of the 256^3 noise grid, on which its chunks spent
+// 40 us of 58 (now 4 of 16).
+template <bool kHalo>
+__device__ __forceinline__ void sweep(MeshSmem& sm, const MeshParams& p, int d, int lane) {
+  const int st = d < 4 ? kS : 1, base = d < 4 ? lane : lane * kS;  // word_off(d, lane, v) = base + v * st
+  const uint32_t* occ = d < 2 ? sm.occt : sm.occ;
+  const uint32_t* eq = e_arr(sm, d);
+  const uint32_t* up = v_arr(sm, d);
+  uint32_t* out = c_arr(sm, d);
+  const bool plus = (d & 1) == 0;
+  const bool edge = lane == (plus ? 31 : 0);
+  const int src = (lane + (plus ? 1 : 31)) & 31;
+  uint32_t A = 0, B = 0, n = 0, rows = 0;
+#pragma unroll 1
+  for (int v0 = 0; v0 < 32; v0 += 8) {
+    uint32_t F[8], G[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int o = base + (v0 + k) * st;
+      const uint32_t c = occ[o];
+      uint32_t beyond = __shfl_sync(kFull, c, src);
+      if (edge) beyond = kHalo ? sm.halo[d ^ 1][v0 + k] : 0u;
+      F[k] = c & ~beyond;
+      G[k] = F[k] & up[o];
+    }
+    // both directions have read these rows of `up` before one overwrites them
+    pair_sync(d >> 1);
+    uint32_t any = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) any |= F[k];
+    if (!__any_sync(kFull, any != 0)) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) out[base + (v0 + k) * st] = 0;
+      A = B = 0;
+      continue;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int o = base + (v0 + k) * st;
+      const uint32_t C = carry_on(A, B, G[k]);
+      const uint32_t left = F[k] & ~C;
+      const uint32_t starts = left & ~(eq[o] & (left << 1));
+      out[o] = C;
+      n += __popc(starts);
+      const uint32_t any_start = __ballot_sync(kFull, starts != 0);
+      if (lane == v0 + k) rows = any_start;
+      A = F[k];
+      B = (B & C) | starts;
+    }
+  }
+  const uint32_t total = __reduce_add_sync(kFull, n);
+  uint32_t rank = __popc(rows);
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFull, rank, o);
+    if (lane >= o) rank += y;
+  }
+  sm.start_rows[d][lane] = rows;
+  sm.start_rank[d][lane] = rank - __popc(rows);
+  if (lane == 31) sm.start_words[d] = rank;
+  if (lane == 0) {
+    sm.quad_next[d] = 0;
+    if (total) {
+      sm.quad_base[d] = atomicAdd(p.count, (unsigned long long)total);
+      atomicAdd(&sm.chunk_quads, total);
+    }
+  }
+}
+
+// What the emission of a direction needs of it.
+struct EmitDir {
+  const uint32_t* C;       // columns that continue
+  int dir;
+  int sh_s, sh_u, sh_v;    // bit offsets of slice, column and row in the linear voxel index
+  uint32_t hi_bits;        // chunk and direction in a quad's upper word
+};
+
+// Starts of quads in row v of the slice, and the columns that widen them.
+__device__ __forceinline__ void row_words(uint32_t faces, uint32_t C, uint32_t E, uint32_t& starts, uint32_t& link) {
+  const uint32_t left = faces & ~C;
+  link = left & E & (left << 1);
+  starts = left & ~link;
+}
+
+// Rows of the quad that starts in column u, row v of slice sl.
+__device__ __forceinline__ uint32_t quad_height(const EmitDir& D, int sl, uint32_t u, int v) {
+  uint32_t h = 1;
+  while (v + (int)h < 32 && (D.C[word_off(D.dir, sl, v + (int)h)] >> u) & 1u) h++;
+  return h;
+}
+
+template <int KIND>
+__device__ __forceinline__ void put_quad(const MeshParams& p, const uint8_t* mb, const EmitDir& D, int sl, uint32_t u,
+                                         int v, uint32_t w, uint32_t h, unsigned long long at) {
+  const uint32_t lin = (uint32_t)sl << D.sh_s | u << D.sh_u | (uint32_t)v << D.sh_v;
+  const uint32_t mat = load_mat_lin<KIND>(mb, lin);
+  if (at < p.cap)
+    reinterpret_cast<uint2*>(p.quads)[at] =
+        make_uint2(lin << 26 | (w - 1u) << 21 | (h - 1u) << 16 | mat, D.hi_bits | lin >> 6);
 }
 
 // Position of the (r+1)-th set bit of w (r < popc(w)): halving on popcounts.
@@ -512,58 +631,56 @@ __device__ __forceinline__ uint32_t select_bit(uint32_t w, uint32_t r) {
   return pos + (r >= (w & 1u) ? 1u : 0u);
 }
 
-// Appends the warp's staged quads to the output (one atomic per flush).
-__device__ __forceinline__ void flush_warp(MeshSmem& sm, int warp, const MeshParams& p, int lane, uint32_t cnt) {
-  __syncwarp();
-  unsigned long long base = 0;
-  if (lane == 0 && cnt) base = atomicAdd(p.count, (unsigned long long)cnt);
-  base = __shfl_sync(kFull, base, 0);
-  for (uint32_t i = lane; i < cnt; i += 32) {
-    const unsigned long long idx = base + i;
-    if (idx < p.cap) p.quads[idx] = sm.qbuf[warp][i];
+// The quads of words j0 .. j0+31 of a direction, of the words (slice, row) in
+// which any start, lane = word.  Lanes take their words' quads one by one while
+// more than kFewLanes have some left; the rest, words with many, are finished
+// one word at a time, lane = column.
+//
+// On the chunk workload 800 of a chunk's 6144 words hold quads, 3.3 each.
+// 4096 chunks: 256 us; with one lane per slice taking quads one by one 459 us (9
+// lanes in 10 idle), with those quads queued in shared memory 293; kFewLanes 2
+// 276, 7 258, 10 270.
+template <int KIND>
+__device__ __forceinline__ void emit_words(MeshSmem& sm, const MeshParams& p, const uint8_t* mb, const EmitDir& D,
+                                           uint32_t j0, int lane) {
+  const bool mine = j0 + (uint32_t)lane < sm.start_words[D.dir];
+  const uint32_t j = mine ? j0 + (uint32_t)lane : sm.start_words[D.dir] - 1u;
+  const uint32_t rank = sm.start_rank[D.dir][lane];
+  int v = 0;
+#pragma unroll
+  for (int step = 16; step >= 1; step >>= 1) {
+    const uint32_t r = __shfl_sync(kFull, rank, v + step);
+    if (r <= j) v += step;
   }
-  __syncwarp();
-}
-
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// Barrier of the warp pair that shares row group g (ids 1..8; 0 is __syncthreads).
-__device__ __forceinline__ void pair_sync(int g) {
-  asm volatile("bar.sync %0, 64;" ::"r"(1 + g) : "memory");
-}
-
-// Isolated faces of the three directions DB .. DB+2 for the rows v0 .. v0+3
-// (lane = slice); see pass 2 in the kernel.
-template <int DB>
-__device__ __forceinline__ void isolated_rows(MeshSmem& sm, int v0, int lane, uint32_t (&isow)[kGroups],
-                                              uint32_t& lane_iso) {
-#pragma unroll
-  for (int dd = 0; dd < 3; dd++) {
-    const int d = DB + dd;
-    uint32_t fu = v0 > 0 ? face_row(sm, d, v0 - 1, lane) : 0u;
-    uint32_t fv = face_row(sm, d, v0, lane);
-    uint32_t vv = v_arr(sm, d)[word_off(d, lane, v0)];
-    uint32_t rest = 0;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int v = v0 + q;
-      const bool last = q == 3 && v0 == 28;
-      const uint32_t fd = last ? 0u : face_row(sm, d, v + 1, lane);
-      const uint32_t vd = last ? 0u : v_arr(sm, d)[word_off(d, lane, v + 1)];
-      const uint32_t w = isolated(fv, fu, fd, e_arr(sm, d)[word_off(d, lane, v)], vv, vd);
-      isow[4 * dd + q] = w;
-      lane_iso += __popc(w);
-      rest |= fv & ~w;
-      fu = fv;
-      fv = fd;
-      vv = vd;
+  const int sl = (int)select_bit(sm.start_rows[D.dir][v], j - __shfl_sync(kFull, rank, v));
+  const int o = word_off(D.dir, sl, v);
+  uint32_t starts, link;
+  row_words(face_col(sm, D.dir, sl, v), D.C[o], e_arr(sm, D.dir)[o], starts, link);
+  if (!mine) starts = 0;
+  const uint32_t sum = __reduce_add_sync(kFull, (uint32_t)__popc(starts));
+  uint32_t place = 0;
+  if (lane == 0) place = atomicAdd(&sm.quad_next[D.dir], sum);
+  unsigned long long at = sm.quad_base[D.dir] + __shfl_sync(kFull, place, 0);
+  uint32_t todo = __ballot_sync(kFull, starts != 0);
+  while (__popc(todo) > kFewLanes) {
+    if (starts) {
+      const uint32_t u = (uint32_t)__ffs(starts) - 1u;
+      starts &= starts - 1u;
+      put_quad<KIND>(p, mb, D, sl, u, v, __ffs(~__funnelshift_rc(link, 0u, u + 1u)), quad_height(D, sl, u, v),
+                     at + __popc(todo & lanemask_lt()));
     }
-    const uint32_t m = __ballot_sync(kFull, rest != 0u);
-    if (lane == 0 && m) atomicOr(&sm.rest_slices[d], m);
+    at += __popc(todo);
+    todo = __ballot_sync(kFull, starts != 0);
+  }
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1u;
+    const uint32_t word = __shfl_sync(kFull, starts, src), lk = __shfl_sync(kFull, link, src);
+    const int s1 = __shfl_sync(kFull, sl, src), v1 = __shfl_sync(kFull, v, src);
+    if ((word >> lane) & 1u)
+      put_quad<KIND>(p, mb, D, s1, (uint32_t)lane, v1, __ffs(~__funnelshift_rc(lk, 0u, (uint32_t)lane + 1u)),
+                     quad_height(D, s1, (uint32_t)lane, v1), at + __popc(word & lanemask_lt()));
+    at += __popc(word);
   }
 }
 
@@ -589,11 +706,9 @@ __global__ void __launch_bounds__(kThreads, KindTraits<KIND>::kCtasPerSm)
     if (p.use_queue && !T::kBrick) pending = atomicAdd(p.ticket, p.per_ticket);
   }
   for (int i = tid; i < 6 * 32; i += kThreads) (&sm.halo[0][0])[i] = 0;
-  if (tid < 6) sm.rest_slices[tid] = 0;
   __syncthreads();
 
   uint32_t phase = 0;
-  uint32_t qc = 0;  // quads staged in qbuf[warp] (warp-uniform)
   int bc = -1;         // brick maps: warp 0's ticket entries (see issue_chunk)
   uint32_t bmask = 0;
   for (;;) {
@@ -640,64 +755,46 @@ __global__ void __launch_bounds__(kThreads, KindTraits<KIND>::kCtasPerSm)
     }
     if (valid) {
       const uint8_t* mb = mat;
-      // ---- pass 1: the warp pair of row group g builds slabs z0 .. z0+3
-      // (z0 = 4g; lanes = x), warp w < 8 rows 0..15 and warp w + 8 rows
-      // 16..31, 8 rows of the 4 slabs at a time, so the previous slab's
-      // materials are still in registers for the -z equality.  Row words come
-      // from ballots and are stored by lane 0; after a pair barrier each warp
-      // makes the transposed copies (for the X faces) of two of the slabs.
+      // ---- pass 1: rows y0 .. y0+7 of slabs z0 .. z0+7, lane = 8 voxels (seg)
+      // of a row; the slab below stays in registers.  Neighbours outside the
+      // chunk need no care: the equality bits of the first column and row and
+      // of the first slab meet no face that is joined across them.  Bits of
+      // empty voxels are never looked at, so an empty group only clears its
+      // occupancy.
       {
-        const int g = warp & 7, half = warp >> 3;
-        const int z0 = g * 4, ybeg = half * 16;
-        uint32_t prev_m[4];  // row y0-1 of each slab
+        const int y0 = (warp & 3) * 8, z0 = (warp >> 2) * 8;
+        const int seg = lane & 3, y = y0 + (lane >> 2), yu = y > 0 ? y - 1 : 0;
+        Seg<KIND> below = load_seg<KIND>(mb, seg, y, z0 > 0 ? z0 - 1 : 0);
+        Seg<KIND> none;
 #pragma unroll
-        for (int j = 0; j < 4; j++) prev_m[j] = half ? load_mat<KIND>(mb, lane, ybeg - 1, z0 + j) : 0u;
-#pragma unroll 1
-        for (int y0 = ybeg; y0 < ybeg + 16; y0 += 8) {
-          uint32_t mp[8];  // rows y0 .. y0+7 of the slab below
+        for (int k = 0; k < Seg<KIND>::kRegs; k++) none.w[k] = 0;
+#pragma unroll 2
+        for (int z = z0; z < z0 + 8; z++) {
+          const Seg<KIND> m = load_seg<KIND>(mb, seg, y, z);
+          const int o = (z * kS + y0) * 4 + lane;  // byte seg of row y's word
+          uint32_t any = 0;
 #pragma unroll
-          for (int k = 0; k < 8; k++) mp[k] = z0 > 0 ? load_mat<KIND>(mb, lane, y0 + k, z0 - 1) : 0u;
+          for (int k = 0; k < Seg<KIND>::kRegs; k++) any |= m.w[k];
+          if (!__any_sync(kFull, any != 0)) {
+            reinterpret_cast<uint8_t*>(sm.occ)[o] = 0;
+          } else {
+            const Seg<KIND> up = load_seg<KIND>(mb, seg, yu, z);
+            Seg<KIND> left;
+            const uint32_t before = __shfl_up_sync(kFull, m.w[Seg<KIND>::kRegs - 1], 1);
 #pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const int z = z0 + j, o = z * kS + y0;
-            if (rows8_empty<KIND>(mb, y0, z, lane)) {
-              if (lane < 8) {
-                sm.occ[o + lane] = 0;
-                sm.ex[o + lane] = 0;
-                sm.ey[o + lane] = 0;
-                sm.ez[o + lane] = 0;
-              }
-#pragma unroll
-              for (int k = 0; k < 8; k++) mp[k] = 0;
-              prev_m[j] = 0;
-              continue;
-            }
-            uint32_t m[8];
-#pragma unroll
-            for (int k = 0; k < 8; k++) m[k] = load_mat<KIND>(mb, lane, y0 + k, z);
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-              const uint32_t ml = __shfl_up_sync(kFull, m[k], 1);
-              const uint32_t occw = __ballot_sync(kFull, m[k] != 0);
-              const uint32_t exw = __ballot_sync(kFull, m[k] == ml);
-              const uint32_t eyw = __ballot_sync(kFull, m[k] == (k ? m[k - 1] : prev_m[j]));
-              const uint32_t ezw = __ballot_sync(kFull, m[k] == mp[k]);
-              if (lane == 0) {
-                sm.occ[o + k] = occw;
-                sm.ex[o + k] = exw;
-                sm.ey[o + k] = eyw;
-                sm.ez[o + k] = ezw;
-              }
-            }
-            prev_m[j] = m[7];
-#pragma unroll
-            for (int k = 0; k < 8; k++) mp[k] = m[k];
+            for (int k = 0; k < Seg<KIND>::kRegs; k++)
+              left.w[k] = __byte_perm(k ? m.w[k ? k - 1 : 0] : before, m.w[k], KindTraits<KIND>::kElem == 2 ? 0x5432 : 0x6543);
+            reinterpret_cast<uint8_t*>(sm.occ)[o] = (uint8_t)differ<KIND>(m, none);
+            reinterpret_cast<uint8_t*>(sm.ex)[o] = (uint8_t)~differ<KIND>(m, left);
+            reinterpret_cast<uint8_t*>(sm.ey)[o] = (uint8_t)~differ<KIND>(m, up);
+            reinterpret_cast<uint8_t*>(sm.ez)[o] = (uint8_t)~differ<KIND>(m, below);
           }
+          below = m;
         }
-        // the pair's other warp builds the other half of these slabs' rows
-        pair_sync(g);
+        // the four warps of these slabs' rows; then two slabs' transposes each
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + (warp >> 2)) : "memory");
 #pragma unroll 1
-        for (int j = 2 * half; j < 2 * half + 2; j++) {
+        for (int j = 2 * (warp & 3); j < 2 * (warp & 3) + 2; j++) {
           const int o = (z0 + j) * kS + lane;
           const uint32_t r_occ = sm.occ[o];
           uint32_t occT = 0, eyT = 0, ezT = 0;
@@ -716,242 +813,36 @@ __global__ void __launch_bounds__(kThreads, KindTraits<KIND>::kCtasPerSm)
       int32_t pf_a = -1, pf_b = 0, pf_c = 0;
       if (tid == 0) next_chunk<KIND>(p, cur, end, pending, pf_a, pf_b, pf_c);
       if (sm.any_solid) {
-        // ---- pass 2: isolated faces (no same-material face neighbour in
-        // the plane).  Quads never leave a component of same-material,
-        // edge-adjacent faces, so these are 1x1 quads whatever the greedy
-        // does elsewhere: they are peeled off into registers.  Warp w holds
-        // rows v0 .. v0+3 (v0 = 4 (w mod 8)) of three directions (0-2 for
-        // w < 8, 3-5 for the others; lane = slice), walking the rows in order
-        // so the face words of the rows above and below are carried, not
-        // recomputed.
-        const int v0 = (warp & 7) * 4, dbase = (warp >> 3) * 3;
-        uint32_t isow[kGroups];
-        uint32_t lane_iso = 0;
-        if (dbase) isolated_rows<3>(sm, v0, lane, isow, lane_iso);
-        else isolated_rows<0>(sm, v0, lane, isow, lane_iso);
-        const uint32_t total = __reduce_add_sync(kFull, lane_iso);
-        unsigned long long run = 0;
-        if (lane == 0 && total) run = atomicAdd(p.count, (unsigned long long)total);
-        run = __shfl_sync(kFull, run, 0);
-        uint32_t mine = total;
-        const uint64_t chunk_bits = (uint64_t)((p.chunk_id_base + (uint32_t)c) & 0xFFFFFu) << 44;
+        // ---- pass 2: the sweep, one warp per direction
+        if (warp < 6) sweep<T::kHalo>(sm, p, warp, lane);
         if (tid == 0) prefetch_chunk<KIND>(p, &tmap, pf_a, pf_b, pf_c);
-        // the slices' rest flags are complete after this barrier; each warp
-        // then emits its own isolated quads and pulls greedy tasks as soon as
-        // it is done, so uneven emission work does not idle warps at a barrier
         __syncthreads();
-        // ---- pass 3: isolated quads of this warp's words, the 4 rows of one
-        // direction at a time (lane = slice).  A warp-balanced expansion over
-        // all set bits of the 4 x 32 words: lane j of a round takes the
-        // (32k+j)-th bit; its owning lane comes from a binary search over
-        // the lanes' exclusive prefixes, the row from the owner's packed
-        // running counts, the word from the warp's staging buffer (its
-        // greedy staging area, empty at this point), the column from a
-        // popcount-halving select.
-        uint32_t* const stage = reinterpret_cast<uint32_t*>(sm.qbuf[warp]);  // [row q][lane]
+        // ---- pass 3: emission
+        const uint32_t chunk_hi = ((p.chunk_id_base + (uint32_t)c) & 0xFFFFFu) << 12;
+        uint32_t first[7];  // tasks of the directions before
+        first[0] = 0;
+#pragma unroll
+        for (int d = 0; d < 6; d++) first[d + 1] = first[d] + ((sm.start_words[d] + 31u) >> 5);
 #pragma unroll 1
-        for (int dir = dbase; dir < dbase + 3; dir++) {
-          // this direction's words are isow[0..3]; the rest shift down by 4
-          const uint32_t w0 = isow[0], w1 = isow[1], w2 = isow[2], w3 = isow[3];
-#pragma unroll
-          for (int i = 0; i + 4 < kGroups; i++) isow[i] = isow[i + 4];
-          const uint32_t c1 = __popc(w0), c2 = c1 + __popc(w1), c3 = c2 + __popc(w2);
-          const uint32_t n = c3 + __popc(w3);
-          uint32_t incl = n;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += y;
-          }
-          const uint32_t G = __shfl_sync(kFull, incl, 31);
-          if (G == 0) continue;
-          const uint32_t ex = incl - n;
-          // running counts before rows 1, 2, 3 in bytes 1..3 (byte 0: 0)
-          const uint32_t packed = c1 << 8 | c2 << 16 | c3 << 24;
-          stage[lane] = w0;
-          stage[32 + lane] = w1;
-          stage[64 + lane] = w2;
-          stage[96 + lane] = w3;
-          __syncwarp();
-          // run: this direction's first output index (the warp reserved all
-          // three directions' isolated quads at once, after pass 2)
-          const bool all_fit = run + G <= p.cap;
-          uint2* const dst = reinterpret_cast<uint2*>(p.quads) + run;
-          // bit offsets of slice, column and row in the linear voxel index
-          const int sh_s = dir < 2 ? 0 : (dir < 4 ? 5 : 10);
-          const int sh_u = dir < 2 ? 5 : 0;
-          const int sh_v = dir < 4 ? 10 : 5;
-          const uint32_t hi_bits = (uint32_t)(chunk_bits >> 32) | (uint32_t)dir << 9;
-          auto emit = [&](uint32_t j, int l) {
-            const uint32_t r = j - __shfl_sync(kFull, ex, l);
-            const uint32_t pk = __shfl_sync(kFull, packed, l);
-            if (j < G) {
-              const uint32_t q = (uint32_t)(r >= ((pk >> 8) & 0xFFu)) + (uint32_t)(r >= ((pk >> 16) & 0xFFu)) +
-                                 (uint32_t)(r >= (pk >> 24));
-              const uint32_t rb = (pk >> (8 * q)) & 0xFFu;
-              const uint32_t u = select_bit(stage[32 * q + l], r - rb);
-              const uint32_t lin = (uint32_t)l << sh_s | u << sh_u | ((uint32_t)v0 + q) << sh_v;
-              const uint32_t mat = load_mat_lin<KIND>(mb, lin);
-              if (all_fit || run + j < p.cap) dst[j] = make_uint2(lin << 26 | mat, hi_bits | lin >> 6);
-            }
-          };
-          // two rounds (64 bits) per pass, so their shuffle chains interleave
-          for (uint32_t k2 = 0; k2 < G; k2 += 64) {
-            const uint32_t ja = k2 + (uint32_t)lane, jb = ja + 32u;
-            int la = 0, lb = 0;
-#pragma unroll
-            for (int step = 16; step >= 1; step >>= 1) {
-              const uint32_t oa = __shfl_sync(kFull, ex, la + step);
-              const uint32_t ob = __shfl_sync(kFull, ex, lb + step);
-              if (oa <= ja) la += step;
-              if (ob <= jb) lb += step;
-            }
-            emit(ja, la);
-            if (k2 + 32u < G) emit(jb, lb);
-          }
-          run += G;
-          __syncwarp();  // the stage is rewritten by the next direction
-        }
-        // ---- pass 4: greedy on the remaining faces, one warp per slice.
-        // Lane r holds row r of the slice in registers: its faces (isolated
-        // ones removed again), their equality with the -u and -v neighbours,
-        // and the bits consumed so far.  Rows are scanned in order; in a row
-        // every maximal run of unconsumed same-material faces is one quad
-        // (Lysenko's left-to-right scan gives exactly these runs); a quad's
-        // height is one ballot over the rows below, and the quads of one row
-        // never interact because their columns are disjoint.
-        uint32_t rs[6], pre[6];
-        uint32_t n_tasks = 0;
-#pragma unroll
-        for (int d = 0; d < 6; d++) {
-          rs[d] = sm.rest_slices[d];
-          pre[d] = n_tasks;
-          n_tasks += __popc(rs[d]);
-        }
-        uint64_t* qb = sm.qbuf[warp];
         for (;;) {
           uint32_t t = 0;
           if (lane == 0) t = atomicAdd(&sm.task_next, 1u);
           t = __shfl_sync(kFull, t, 0);
-          if (t >= n_tasks) break;
-          int dir = 0;
-          uint32_t before = 0, smask = rs[0];
+          if (t >= first[6]) break;
+          EmitDir D;
+          D.dir = 0;
+          uint32_t before = 0;
 #pragma unroll
           for (int d = 1; d < 6; d++) {
-            if (t >= pre[d]) {
-              dir = d;
-              before = pre[d];
-              smask = rs[d];
-            }
+            D.dir = t >= first[d] ? d : D.dir;
+            before = t >= first[d] ? first[d] : before;
           }
-          const int sl = (int)select_bit(smask, t - before);
-          const int orow = word_off(dir, sl, lane);
-          const uint32_t F0 = face_col(sm, dir, sl, lane);
-          const uint32_t Er = e_arr(sm, dir)[orow];
-          const uint32_t Vr = v_arr(sm, dir)[orow];
-          uint32_t fu = __shfl_up_sync(kFull, F0, 1), fd = __shfl_down_sync(kFull, F0, 1);
-          uint32_t vd = __shfl_down_sync(kFull, Vr, 1);
-          if (lane == 0) fu = 0;
-          if (lane == 31) fd = vd = 0;
-          // the faces pass 2 left: not isolated and not in a domino
-          const uint32_t hl = F0 & Er & (F0 << 1), hh = hl | (hl >> 1);
-          const uint32_t ul = F0 & Vr & fu, dl = F0 & vd & fd, vl = ul | dl;
-          const uint32_t hd = hl & ~(hl << 1) & ~(hl >> 1) & ~vl & ~(vl << 1);
-          uint32_t hn = __shfl_down_sync(kFull, hh, 1), dn = __shfl_down_sync(kFull, dl, 1);
-          if (lane == 31) hn = dn = 0;
-          const uint32_t vdt = dl & ~hh & ~ul & ~hn & ~dn;
-          uint32_t vdb = __shfl_up_sync(kFull, vdt, 1);
-          if (lane == 0) vdb = 0;
-          const uint32_t Fr = F0 & (hh | vl) & ~(hd | (hd >> 1) | vdt | vdb);
-          {
-            // two-face components first: a 2x1 or 1x2 quad whatever the
-            // scan order (origins hd >> 1: 2 wide, vdt: 2 high; lane = row)
-            uint32_t ho = hd >> 1, vo = vdt;
-            while (__any_sync(kFull, (ho | vo) != 0u)) {
-              const bool horiz = ho != 0u;
-              const uint32_t act = __ballot_sync(kFull, (ho | vo) != 0u);
-              const uint32_t n = __popc(act);
-              if (qc + n > (uint32_t)kQBuf) {
-                flush_warp(sm, warp, p, lane, qc);
-                qc = 0;
-              }
-              if (ho | vo) {
-                uint32_t u;
-                if (horiz) {
-                  u = __ffs(ho) - 1;
-                  ho &= ho - 1u;
-                } else {
-                  u = __ffs(vo) - 1;
-                  vo &= vo - 1u;
-                }
-                int x, y, z;
-                face_xyz(dir, sl, (int)u, lane, x, y, z);
-                const uint32_t mat = load_mat<KIND>(mb, x, y, z);
-                qb[qc + __popc(act & lanemask_lt())] =
-                    chunk_bits | (uint64_t)dir << 41 | (uint64_t)z << 36 | (uint64_t)y << 31 | (uint64_t)x << 26 |
-                    (uint64_t)(horiz ? 1u : 0u) << 21 | (uint64_t)(horiz ? 0u : 1u) << 16 | (uint64_t)mat;
-              }
-              qc += n;
-              mine += n;
-            }
-          }
-          uint32_t rows = __ballot_sync(kFull, Fr != 0);
-          const uint64_t dir_bits = chunk_bits | (uint64_t)dir << 41;
-          uint32_t cons = 0;
-          while (rows) {
-            const int v = __ffs(rows) - 1;
-            rows &= rows - 1;
-            const uint32_t cur = Fr & ~cons;
-            const uint32_t word = __shfl_sync(kFull, cur, v);
-            if (!word) continue;
-            const uint32_t e = __shfl_sync(kFull, Er, v);
-            const uint32_t link = word & e & (word << 1);
-            const uint32_t starts = word & ~link;
-            const uint32_t cnt = __popc(starts);
-            if (qc + cnt > (uint32_t)kQBuf) {
-              flush_warp(sm, warp, p, lane, qc);
-              qc = 0;
-            }
-            const uint32_t q0 = qc;
-            // every start lane grows its quad; row r's words come from lane r
-            const bool is_start = (starts >> lane) & 1u;
-            const int w = __ffs(~__funnelshift_rc(link, 0u, (uint32_t)lane + 1u));
-            const uint32_t mask = is_start ? ((2u << (w - 1)) - 1u) << lane : 0u;
-            const uint32_t grow = Fr & Vr;  // faces that continue the row above in material
-            bool active = is_start;
-            int h = 1;
-            // two rows per step: row r+1's word is fetched with row r's (a
-            // row's consumed bits change only when its own turn comes)
-            for (int r = v + 1; r < 32; r += 2) {
-              const uint32_t gr = grow & ~cons;
-              const uint32_t g0 = __shfl_sync(kFull, gr, r);
-              const uint32_t g1 = __shfl_sync(kFull, gr, r + 1 < 32 ? r + 1 : 31);
-              const bool c0 = active && (g0 & mask) == mask;
-              const bool c1 = c0 && r + 1 < 32 && (g1 & mask) == mask;
-              const uint32_t t0 = __reduce_or_sync(kFull, c0 ? mask : 0u);
-              const uint32_t t1 = __reduce_or_sync(kFull, c1 ? mask : 0u);
-              if (lane == r) cons |= t0;
-              if (lane == r + 1) cons |= t1;
-              h += (c0 ? 1 : 0) + (c1 ? 1 : 0);
-              active = c1;
-              if (!__any_sync(kFull, active)) break;
-            }
-            if (is_start) {
-              int x, y, z;
-              face_xyz(dir, sl, lane, v, x, y, z);
-              const uint32_t mat = load_mat<KIND>(mb, x, y, z);
-              qb[q0 + __popc(starts & lanemask_lt())] = dir_bits | (uint64_t)z << 36 | (uint64_t)y << 31 |
-                                                         (uint64_t)x << 26 | (uint64_t)(w - 1) << 21 |
-                                                         (uint64_t)(h - 1) << 16 | (uint64_t)mat;
-            }
-            qc = q0 + cnt;
-            mine += cnt;
-          }
-        }
-        if (p.chunk_counts && lane == 0 && mine) atomicAdd(&sm.chunk_quads, mine);
-        if (qc) {  // the staging area doubles as pass 3's word buffer
-          flush_warp(sm, warp, p, lane, qc);
-          qc = 0;
+          D.C = c_arr(sm, D.dir);
+          D.sh_s = D.dir < 2 ? 0 : (D.dir < 4 ? 5 : 10);
+          D.sh_u = D.dir < 2 ? 5 : 0;
+          D.sh_v = D.dir < 4 ? 10 : 5;
+          D.hi_bits = chunk_hi | (uint32_t)D.dir << 9;
+          emit_words<KIND>(sm, p, mb, D, (t - before) * 32u, lane);
         }
       }
     }
@@ -962,9 +853,7 @@ __global__ void __launch_bounds__(kThreads, KindTraits<KIND>::kCtasPerSm)
       sm.task_next = 0;
       sm.any_solid = 0;
     }
-    if (tid < 6) sm.rest_slices[tid] = 0;
   }
-  flush_warp(sm, warp, p, lane, qc);
 }
 
 // --------------------------------------------------------------- host side
