@@ -311,8 +311,8 @@ meso_status meso_raymarch_stats(meso_ctx* ctx, const meso_scene* const* scenes, 
  * call -- a frame loop on a fixed device-memory budget that must not
  * allocate mid-frame (an allocation can synchronise the device and stall the
  * frame), or a host application whose own memory manager owns all device
- * memory -- the view descriptors go to a fixed device array of 512 x 144
- * bytes (72 KiB) instead of a per-call allocation; they travel there as
+ * memory -- the view descriptors go to a fixed device array of 512 x 152
+ * bytes (76 KiB) instead of a per-call allocation; they travel there as
  * kernel parameters, 64 views at a time (9.5 KiB of the caller's stack).
  * At most 512 views per call (more returns MESO_ERR_INVALID_ARG).  The array
  * stays resident on every device that loads the library until the process

@@ -92,6 +92,8 @@ struct meso_scene {
   // not part of `bytes`, so that a budget admits what it did without them):
   uint8_t* d_level = nullptr;  // per brick: 0 if occupied, else log2 of the edge in voxels of the largest
                                // aligned empty cube it is part of (3 .. 9)
+  int32_t* d_bounds = nullptr; // of the occupied 4x4x4-brick cells, in voxels: [0..2] the largest -lowest, [4..6] the
+                               // largest highest coordinate per axis; edits only widen them
   uint64_t* d_mask = nullptr;  // per 4x4x4-brick cell: its occupied bricks, bit x + 4y + 16z
   uint64_t* d_sub = nullptr;   // per pool slot: the non-empty 2x2x2-voxel blocks, bit x + 4y + 16z
   uint64_t capacity = 0;       // pool slots

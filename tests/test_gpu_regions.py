@@ -141,3 +141,45 @@ def test_every_block_shape(ctx, warps, tile_w):
         same(got, oracle.raymarch(bm, [oracle.camera(*pose, w, h) for w, h in cams]))
     scene.destroy()
     c.close()
+
+
+@pytest.mark.parametrize("lo,hi", [((0, 0, 0), (32, 32, 32)), ((64, 96, 32), (96, 160, 64)), ((130, 70, 40), (131, 71, 41)),
+                                   ((0, 128, 0), (256, 160, 96)), ((200, 0, 90), (256, 192, 96)), (None, None)])
+def test_space_outside_the_bounds(ctx, lo, hi):
+    # content in one part of the grid (a corner cell, an inner box, one voxel,
+    # slabs along faces, none): rays that enter its bounds from each side and
+    # from inside, that miss them, that pass along their faces and corners;
+    # then bounds that edits widen, and that keep their size as edits empty them
+    dims = (256, 192, 96)
+    rng = np.random.default_rng(11)
+    g = np.zeros(dims[::-1], dtype=np.uint16)
+    if lo is not None:
+        part = g[lo[2]:hi[2], lo[1]:hi[1], lo[0]:hi[0]]
+        part[...] = (rng.random(part.shape) < 0.02) * 9
+        part.flat[0] = part.flat[-1] = 3
+    lo, hi = lo or (96, 96, 32), hi or (128, 128, 64)
+    scene, bm = ctx.scene_from_dense(g, spare_bricks=2000), oracle.HostBrickMap.from_dense(g)
+    mid = [(a + b) / 2.0 for a, b in zip(lo, hi)]
+    face = [32.0 * (a // 32) for a in lo]  # of the cell that the lowest voxel is in
+
+    def look():
+        for k in range(8):
+            s = [1 if (k >> a) & 1 else -1 for a in range(3)]
+            both(ctx, scene, bm, [mid[a] - s[a] * (0.7 * dims[a] + 9.3) for a in range(3)], mid, 40, 30)
+            both(ctx, scene, bm, [dims[a] * (0.5 - 0.45 * s[a]) for a in range(3)], mid, 40, 30,
+                 light=np.array([0.3 * s[0], 0.5 * s[1], 0.8 * s[2]], np.float32))
+        both(ctx, scene, bm, mid, [0.0, 0.0, 0.0], 40, 30)
+        for a in range(3):  # in the plane of a face of the bounds, and through its corner
+            d = [40.0 * (b != a) for b in range(3)]
+            both(ctx, scene, bm, [f - v for f, v in zip(face, d)], face, 33, 33)
+        both(ctx, scene, bm, [f - 40.0 for f in face], face, 33, 33)
+
+    look()
+    scene.edit([meso.SphereEdit((ctypes.c_int32 * 3)(20, 30, 80), 5, 7, 0)])
+    bm.edit([oracle.Sphere((ctypes.c_int32 * 3)(20, 30, 80), 5, 7, 0)])
+    look()
+    whole = [((x, y, z), 70, 0) for x in (0, 85, 170, 255) for y in (0, 95, 191) for z in (0, 95)]
+    scene.edit([meso.SphereEdit((ctypes.c_int32 * 3)(*c), r, m, 0) for c, r, m in whole])
+    bm.edit([oracle.Sphere((ctypes.c_int32 * 3)(*c), r, m, 0) for c, r, m in whole])
+    look()
+    scene.destroy()
