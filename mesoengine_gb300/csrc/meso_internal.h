@@ -82,11 +82,6 @@ struct meso_scene {
   // one byte per 4x4x4-brick cell (a 32^3 chunk): nonzero iff a brick of the
   // cell is occupied; lets a ray cross an empty cell in one jump
   uint8_t* d_macro = nullptr;
-  // one byte per 16x16x16-brick cell (128^3 voxels, partial at the far
-  // edges): nonzero iff one of its 32^3 cells is, or it extends past the grid
-  uint8_t* d_macro2 = nullptr;
-  // one byte per 64x64x64-brick cell (512^3 voxels), built like d_macro2 from it
-  uint8_t* d_macro3 = nullptr;
   // Derived maps of the raymarch's region walk (a byte per brick, 8 per
   // 4x4x4-brick cell and 8 per pool slot, a few percent of the scene at most;
   // not part of `bytes`, so that a budget admits what it did without them):
@@ -129,12 +124,11 @@ inline cudaStream_t pick_stream(meso_ctx* ctx, void* s) {
 meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint64_t capacity,
                         meso_scene** out);
 void scene_release(meso_ctx* ctx, meso_scene* s);
-// Recomputes the cell maps (occupancy bytes, brick masks, level bytes): every
-// cell (lists null), or the listed cells of 4^3, 16^3 and 64^3 bricks (each
-// list sorted unique, children before parents).
+// Recomputes the cell maps (occupancy bytes, brick masks, level bytes,
+// bounds): all of them (lists null), or of the listed cells of 4^3 and 64^3
+// bricks (each list unique) after an edit, whose pool counters it also clamps.
 meso_status rebuild_macro(meso_ctx* ctx, meso_scene* s, const uint32_t* d_cells, uint32_t n, cudaStream_t st,
-                          const uint32_t* d_cells2 = nullptr, uint32_t n2 = 0, const uint32_t* d_cells3 = nullptr,
-                          uint32_t n3 = 0);
+                          const uint32_t* d_cells3 = nullptr, uint32_t n3 = 0);
 // Recomputes d_sub of the first `slots` pool slots from their occupancy.
 meso_status rebuild_sub(meso_ctx* ctx, meso_scene* s, uint64_t slots, cudaStream_t st);
 

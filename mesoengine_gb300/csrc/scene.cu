@@ -530,11 +530,6 @@ __global__ void edit_alloc_kernel(EditParams P) {
   }
 }
 
-__global__ void edit_fix_kernel(int32_t* alloc, uint32_t capacity) {
-  if (alloc[1] < 0) alloc[1] = 0;
-  if ((uint32_t)alloc[0] > capacity) alloc[0] = (int32_t)capacity;
-}
-
 // Solid voxels of the live bricks: popcount of each linked brick's 8
 // occupancy words, summed per warp and added to *count.
 __global__ void count_solid_kernel(const uint32_t* ptr, uint64_t nb, const uint64_t* occ,
@@ -565,11 +560,22 @@ unsigned grid_for(uint64_t warps, int threads = 256) {
 }  // namespace
 
 // One warp per macro cell (4x4x4 bricks): the mask of its occupied bricks
-// (bit x + 4y + 16z), and a byte that says whether there are any.
-__global__ void macro_kernel(const uint32_t* ptr, int bx, int by, uint8_t* macro, uint64_t* mask,
-                             const uint32_t* cells, uint64_t n) {
+// (bit x + 4y + 16z), and a byte that says whether there are any.  Its first
+// threads also do what must lie between the kernels before and behind it: of a
+// whole rebuild, reset the bounds; of an edit (cells given), bring the pool's
+// counters back into their range where allocations overran it.
+__global__ void macro_kernel(const uint32_t* ptr, int bx, int by, uint8_t* macro, uint64_t* mask, int32_t* bounds,
+                             int32_t* alloc, uint32_t capacity, const uint32_t* cells, uint64_t n) {
   const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
+  if (blockIdx.x == 0) {
+    if (!cells) {
+      if (threadIdx.x < 8) bounds[threadIdx.x] = INT32_MIN / 2;  // nothing occupied
+    } else if (threadIdx.x == 0) {
+      if (alloc[1] < 0) alloc[1] = 0;
+      if ((uint32_t)alloc[0] > capacity) alloc[0] = (int32_t)capacity;
+    }
+  }
   if (w >= n) return;
   const uint32_t m = cells ? cells[w] : (uint32_t)w;
   const int mx = bx >> 2, my = by >> 2;
@@ -584,112 +590,88 @@ __global__ void macro_kernel(const uint32_t* ptr, int bx, int by, uint8_t* macro
   }
 }
 
-// One warp per 16x16x16-brick cell: any occupied 4x4x4-brick child -> 1 (its
-// 64 children read two per lane, at once); a cell that extends past the grid
-// is marked 1 too, so no jump leaves the grid.  The bounds of the occupied
-// children widen the scene's where they lie outside them: one warp speaks for
-// 64 cells and looks before it sends an atomic (512^3 build: 1 us; a warp per
-// 4x4x4-brick cell, all of them at once, 6 us).
-__global__ void macro2_kernel(const uint8_t* macro, int bx, int by, int bz, uint8_t* macro2, int32_t* bounds,
-                              const uint32_t* list, uint32_t n) {
-  const int m2x = (bx + 15) / 16, m2y = (by + 15) / 16, m2z = (bz + 15) / 16;
-  const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= (list ? n : (uint64_t)m2x * m2y * m2z)) return;
-  const uint32_t i = list ? list[w] : (uint32_t)w;
-  const int cx = (int)(i % (uint32_t)m2x), cy = (int)((i / (uint32_t)m2x) % (uint32_t)m2y), cz = (int)(i / ((uint32_t)m2x * m2y));
-  const int mx = bx / 4, my = by / 4, mz = bz / 4;
-  const bool edge = (cx + 1) * 4 > mx || (cy + 1) * 4 > my || (cz + 1) * 4 > mz;
-  // lane: child (lane & 3, lane >> 2 & 3) of layers lane >> 4 and 2 + (lane >> 4)
-  const int x = cx * 4 + (lane & 3), y = cy * 4 + ((lane >> 2) & 3), z = cz * 4 + (lane >> 4);
-  const uint8_t* m = macro + (uint32_t)x + (uint32_t)mx * ((uint32_t)y + (uint32_t)my * (uint32_t)z);
-  const bool in = x < mx && y < my;
-  const uint32_t low = __ballot_sync(0xFFFFFFFFu, in && z < mz && m[0] != 0);
-  const uint32_t high = __ballot_sync(0xFFFFFFFFu, in && z + 2 < mz && m[2ull * mx * my] != 0);
-  const uint32_t layer = low | high;
-  if (lane == 0) macro2[i] = edge || layer != 0 ? 1 : 0;
-  if (layer != 0 && lane < 6) {
-    // the occupied columns, rows and layers of children, four bits each
-    const uint32_t two = layer | layer >> 16, cols = two | two >> 4 | two >> 8 | two >> 12;
-    const int a = lane % 3;
-    uint32_t set;
-    if (a == 0) set = cols & 0xFu;
-    else if (a == 1) set = ((two & 0xFu) != 0) | ((two & 0xF0u) != 0) << 1 | ((two & 0xF00u) != 0) << 2 | ((two & 0xF000u) != 0) << 3;
-    else set = ((low & 0xFFFFu) != 0) | (low >> 16 != 0) << 1 | ((high & 0xFFFFu) != 0) << 2 | (high >> 16 != 0) << 3;
-    const int c = 4 * (a == 0 ? cx : (a == 1 ? cy : cz));
-    const int v = lane < 3 ? -32 * (c + __ffs((int)set) - 1) : 32 * (c + 31 - __clz((int)set)) + 31;
-    int32_t* b = bounds + (lane < 3 ? a : 4 + a);
-    if (v > *static_cast<volatile int32_t*>(b)) atomicMax(b, v);
-  }
-}
-
-// One warp per 64x64x64-brick cell: any nonzero 16x16x16 child, or a cell
-// extending past the grid -> 1.
-__global__ void macro3_kernel(const uint8_t* macro2, int bx, int by, int bz, uint8_t* macro3, const uint32_t* list,
-                              uint32_t n) {
-  const int m3x = (bx + 63) / 64, m3y = (by + 63) / 64, m3z = (bz + 63) / 64;
-  const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= (list ? n : (uint64_t)m3x * m3y * m3z)) return;
-  const uint32_t i = list ? list[w] : (uint32_t)w;
-  const int cx = (int)(i % (uint32_t)m3x), cy = (int)((i / (uint32_t)m3x) % (uint32_t)m3y), cz = (int)(i / ((uint32_t)m3x * m3y));
-  const int m2x = (bx + 15) / 16, m2y = (by + 15) / 16;
-  const bool edge = (cx + 1) * 64 > bx || (cy + 1) * 64 > by || (cz + 1) * 64 > bz;
-  bool any = false;
-  if (!edge)
-    for (int k = lane; k < 64; k += 32) {
-      const int x = cx * 4 + (k & 3), y = cy * 4 + ((k >> 2) & 3), z = cz * 4 + (k >> 4);
-      any |= macro2[(uint32_t)x + (uint32_t)m2x * ((uint32_t)y + (uint32_t)m2y * (uint32_t)z)] != 0;
-    }
-  const bool set = edge || __any_sync(0xFFFFFFFFu, any);
-  if (lane == 0) macro3[i] = set ? 1 : 0;
-}
-
 // Level bytes: per brick log2 of the edge, in voxels, of the largest aligned
 // cube of empty space that it is part of and that lies in the grid (9: 64^3
-// bricks .. 3: the brick), 0 if it is occupied; one thread per 4x4x4-brick
-// cell.  The bricks of one 64^3-brick cell depend on nothing outside it, so an
-// edit recomputes those of the 64^3-brick cells it touches (list; 4096 threads
-// each), a build all of them.
-__global__ void level_kernel(const uint64_t* mask, const uint8_t* macro, const uint8_t* macro2, const uint8_t* macro3, int bx, int by,
-                             int bz, uint8_t* level, const uint32_t* list, uint64_t n) {
-  const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= n) return;
+// bricks .. 3: the brick), 0 if it is occupied; and the bounds of the occupied
+// cells, widened where a 64^3-brick cell holds some outside them (looked at
+// before, so that few send an atomic).
+//
+// The bricks of one 64^3-brick cell depend on nothing outside it, so an edit
+// recomputes those of the cells it touches (list), a build all of them: 32
+// blocks each, a thread per 4x4x4-brick cell.  Every block reads the cell's
+// 16^3 occupancy bytes (4 KB, of which the 32 share the fetches) and derives the
+// coarser levels itself.  (With the 16^3- and 64^3-brick cells' maps from two
+// launches in between, and two more for what macro_kernel's first threads do, a
+// 512^3 build took 202 us and now 194, 16 sphere edits with remesh and frame 318
+// and now 308.)
+constexpr int kLevelThreads = 128;
+
+__global__ void __launch_bounds__(kLevelThreads)
+    level_kernel(const uint64_t* mask, const uint8_t* macro, int bx, int by, int bz, uint8_t* level, int32_t* bounds,
+                 const uint32_t* list) {
+  // two rows of 16 4x4x4-brick cells a word (y = 2i and 2i + 1), bit x, outside of the grid set
+  __shared__ uint32_t rows[16 * 8];
+  __shared__ uint32_t set2[2];  // 16^3-brick cells that are not empty or reach past the grid, bit x + 4y + 16z
   const int mx = bx / 4, my = by / 4, mz = bz / 4;
-  const int m2x = (bx + 15) / 16, m2y = (by + 15) / 16, m2z = (bz + 15) / 16;
-  const int m3x = (bx + 63) / 64, m3y = (by + 63) / 64;
-  int cx, cy, cz;
-  if (list) {
-    const uint32_t r = list[w >> 12], k = (uint32_t)w & 4095u;
-    cx = (int)(r % (uint32_t)m3x) * 16 + (int)(k & 15u);
-    cy = (int)((r / (uint32_t)m3x) % (uint32_t)m3y) * 16 + (int)((k >> 4) & 15u);
-    cz = (int)(r / ((uint32_t)m3x * m3y)) * 16 + (int)(k >> 8);
-    if (cx >= mx || cy >= my || cz >= mz) return;
-  } else {
-    cx = (int)(w % (uint32_t)mx);
-    cy = (int)((w / (uint32_t)mx) % (uint32_t)my);
-    cz = (int)(w / ((uint32_t)mx * my));
+  const uint32_t m3x = (uint32_t)(bx + 63) / 64, m3y = (uint32_t)(by + 63) / 64;
+  const uint32_t r = list ? list[blockIdx.x >> 5] : blockIdx.x >> 5;
+  const int ox = (int)(r % m3x) * 16, oy = (int)((r / m3x) % m3y) * 16, oz = (int)(r / (m3x * m3y)) * 16;
+  const int t = (int)threadIdx.x, lane = t & 31, warp = t >> 5;
+#pragma unroll 8
+  for (int k = 0; k < 32; k++) {  // warp: layers 4 warp .. 4 warp + 3
+    const int x = ox + (lane & 15), y = oy + 2 * (k & 7) + (lane >> 4), z = oz + 4 * warp + (k >> 3);
+    const bool in = x < mx && y < my && z < mz;
+    const uint32_t w = __ballot_sync(0xFFFFFFFFu, !in || macro[(size_t)x + (size_t)mx * ((size_t)y + (size_t)my * (size_t)z)] != 0);
+    if (lane == 0) rows[32 * warp + k] = w;
   }
-  // all 2x2x2 cells (aligned) around (x, y, z) of a map of nx x ny x nz cells in the grid and zero
-  auto block_empty = [](const uint8_t* m, int x, int y, int z, int nx, int ny, int nz) {
-    x &= ~1;
-    y &= ~1;
-    z &= ~1;
-    if (x + 1 >= nx || y + 1 >= ny || z + 1 >= nz) return false;
-    uint32_t any = 0;
-    for (int k = 0; k < 8; k++)
-      any |= m[(uint32_t)(x + (k & 1)) + (uint32_t)nx * ((uint32_t)(y + ((k >> 1) & 1)) + (uint32_t)ny * (uint32_t)(z + (k >> 2)))];
-    return any == 0;
-  };
-  const uint32_t i = (uint32_t)cx + (uint32_t)mx * ((uint32_t)cy + (uint32_t)my * (uint32_t)cz);
+  __syncthreads();
+  if (t < 64) {
+    uint32_t any = 0;  // child (t & 3, t >> 2 & 3, t >> 4): 4 layers of 2 words
+#pragma unroll
+    for (int k = 0; k < 8; k++) any |= rows[32 * (t >> 4) + 8 * (k >> 1) + 2 * ((t >> 2) & 3) + (k & 1)];
+    any |= any >> 16;
+    const uint32_t b = __ballot_sync(0xFFFFFFFFu, (any >> (4 * (t & 3))) & 15u);
+    if (lane == 0) set2[warp] = b;
+  } else if (warp == 2 && (blockIdx.x & 31u) == 0) {
+    uint32_t xs = 0, ys = 0, zs = 0;
+    const uint32_t inx = mx - ox < 16 ? (1u << (mx - ox)) - 1u : 0xFFFFu;
+    for (int k = lane; k < 128; k += 32) {
+      const int y = 2 * (k & 7), z = k >> 3;
+      const uint32_t a = oz + z < mz && oy + y < my ? rows[k] & inx : 0u;
+      const uint32_t b = oz + z < mz && oy + y + 1 < my ? (rows[k] >> 16) & inx : 0u;
+      xs |= a | b;
+      ys |= (uint32_t)(a != 0) << y | (uint32_t)(b != 0) << (y + 1);
+      zs |= (uint32_t)((a | b) != 0) << z;
+    }
+    xs = __reduce_or_sync(0xFFFFFFFFu, xs);
+    ys = __reduce_or_sync(0xFFFFFFFFu, ys);
+    zs = __reduce_or_sync(0xFFFFFFFFu, zs);
+    if (xs && lane < 6) {
+      const int a = lane % 3;
+      const uint32_t s = a == 0 ? xs : (a == 1 ? ys : zs);
+      const int c = a == 0 ? ox : (a == 1 ? oy : oz);
+      const int v = lane < 3 ? -32 * (c + __ffs((int)s) - 1) : 32 * (c + 31 - __clz((int)s)) + 31;
+      int32_t* b = bounds + (lane < 3 ? a : 4 + a);
+      if (v > *static_cast<volatile int32_t*>(b)) atomicMax(b, v);
+    }
+  }
+  __syncthreads();
+  const int k12 = (int)(blockIdx.x & 31u) * kLevelThreads + t;  // the thread's cell of the 16^3
+  const int lx = k12 & 15, ly = (k12 >> 4) & 15, lz = k12 >> 8;
+  const int cx = ox + lx, cy = oy + ly, cz = oz + lz;
+  if (cx >= mx || cy >= my || cz >= mz) return;
+  const uint64_t bricks = mask[(size_t)cx + (size_t)mx * ((size_t)cy + (size_t)my * (size_t)cz)];
   uint32_t l;
-  const uint64_t bricks = mask[i];
   if (bricks) l = 0;
-  else if (!macro3[(uint32_t)(cx >> 4) + (uint32_t)m3x * ((uint32_t)(cy >> 4) + (uint32_t)m3y * (uint32_t)(cz >> 4))]) l = 9;
-  else if (block_empty(macro2, cx >> 2, cy >> 2, cz >> 2, m2x, m2y, m2z)) l = 8;
-  else if (!macro2[(uint32_t)(cx >> 2) + (uint32_t)m2x * ((uint32_t)(cy >> 2) + (uint32_t)m2y * (uint32_t)(cz >> 2))]) l = 7;
-  else if (block_empty(macro, cx, cy, cz, mx, my, mz)) l = 6;
-  else l = 5;
+  else if ((set2[0] | set2[1]) == 0) l = 9;
+  else {
+    const uint32_t half = set2[lz >> 3] >> ((lx >> 2 & 2) + 4 * (ly >> 2 & 2));  // the aligned 2x2x2 children's
+    const uint32_t* w = rows + 8 * (lz & ~1) + (ly >> 1);                        // the aligned 2x2x2 cells'
+    if ((half & 0x330033u) == 0) l = 8;
+    else if (!((set2[lz >> 3] >> ((lx >> 2) + 4 * (ly >> 2) + 16 * (lz >> 2 & 1))) & 1u)) l = 7;
+    else if ((((w[0] | w[8]) >> (lx & ~1)) & 0x30003u) == 0) l = 6;
+    else l = 5;
+  }
   // 16 rows of 4 bricks, a byte each
   uint32_t* dst = reinterpret_cast<uint32_t*>(level) + (size_t)cx + (size_t)mx * ((size_t)cy * 4 + (size_t)by * ((size_t)cz * 4));
 #pragma unroll
@@ -748,6 +730,8 @@ meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint6
   s->bz = nz / 8;
   s->capacity = capacity;
   const uint64_t nb = n_bricks_of(s);
+  // (a byte for each cell of 4^3, 16^3 and 64^3 bricks is counted, whatever the
+  // maps derived from the pointers take)
   const uint64_t bytes = nb * 4 + nb / 64 + n_macro2_of(s) + n_macro3_of(s) + capacity * (64 + 1024 + 4) + 16;
   if (ctx->budget_bytes && ctx->scene_bytes.load() + bytes > ctx->budget_bytes) {
     delete s;
@@ -766,19 +750,16 @@ meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint6
     if (err == cudaSuccess) s->pool_bytes += n;
     return err;
   };
-  const uint64_t nm = std::max<uint64_t>(n_macro_of(s), 1), nm2 = std::max<uint64_t>(n_macro2_of(s), 1),
-                 nm3 = std::max<uint64_t>(n_macro3_of(s), 1), nslot = std::max<uint64_t>(capacity, 1);
+  const uint64_t nm = std::max<uint64_t>(n_macro_of(s), 1), nslot = std::max<uint64_t>(capacity, 1);
   uint8_t* maps = nullptr;
   uint8_t* small = nullptr;
   cudaError_t e = take(&s->d_ptr, nb * 4);
-  if (e == cudaSuccess) e = take(&maps, 32 + nm * (8 + 64 + 1) + nm2 + nm3);
+  if (e == cudaSuccess) e = take(&maps, 32 + nm * (8 + 64 + 1));
   if (e == cudaSuccess) {
     s->d_bounds = reinterpret_cast<int32_t*>(maps);  // all written whole by rebuild_macro
     s->d_mask = reinterpret_cast<uint64_t*>(maps + 32);
     s->d_level = maps + 32 + nm * 8;
     s->d_macro = s->d_level + nm * 64;
-    s->d_macro2 = s->d_macro + nm;
-    s->d_macro3 = s->d_macro2 + nm2;
   }
   if (e == cudaSuccess) e = take(&s->d_occ, nslot * 64);
   if (e == cudaSuccess) e = take(&s->d_mat, nslot * 1024);
@@ -814,25 +795,15 @@ void scene_release(meso_ctx* ctx, meso_scene* s) {
 }
 
 meso_status rebuild_macro(meso_ctx* ctx, meso_scene* s, const uint32_t* d_cells, uint32_t n, cudaStream_t st,
-                          const uint32_t* d_cells2, uint32_t n2, const uint32_t* d_cells3, uint32_t n3) {
-  const uint64_t cells = d_cells ? n : n_macro_of(s);
+                          const uint32_t* d_cells3, uint32_t n3) {
+  const uint64_t cells = d_cells ? n : n_macro_of(s), cells3 = d_cells3 ? n3 : n_macro3_of(s);
   if (cells == 0) return MESO_OK;
-  if (!d_cells) MESO_CUDA_TRY(cudaMemsetAsync(s->d_bounds, 0x80, 32, st));  // the most negative: nothing occupied
-  macro_kernel<<<(unsigned)((cells * 32 + 255) / 256), 256, 0, st>>>(s->d_ptr, s->bx, s->by, s->d_macro, s->d_mask,
-                                                                     d_cells, cells);
-  const uint64_t cells2 = d_cells2 ? n2 : n_macro2_of(s);
-  if (cells2)
-    macro2_kernel<<<(unsigned)((cells2 * 32 + 255) / 256), 256, 0, st>>>(s->d_macro, s->bx, s->by, s->bz,
-                                                                          s->d_macro2, s->d_bounds, d_cells2, n2);
-  const uint64_t cells3 = d_cells3 ? n3 : n_macro3_of(s);
-  if (cells3)
-    macro3_kernel<<<(unsigned)((cells3 * 32 + 255) / 256), 256, 0, st>>>(s->d_macro2, s->bx, s->by, s->bz,
-                                                                          s->d_macro3, d_cells3, n3);
-  const uint64_t levels = d_cells3 ? (uint64_t)n3 << 12 : n_macro_of(s);
-  if (levels)
-    level_kernel<<<(unsigned)((levels + 127) / 128), 128, 0, st>>>(s->d_mask, s->d_macro, s->d_macro2, s->d_macro3, s->bx, s->by,
-                                                                    s->bz, s->d_level, d_cells3, levels);
-  ctx->launches.fetch_add(4);
+  macro_kernel<<<(unsigned)((cells * 32 + 255) / 256), 256, 0, st>>>(s->d_ptr, s->bx, s->by, s->d_macro, s->d_mask, s->d_bounds,
+                                                                     reinterpret_cast<int32_t*>(s->d_alloc),
+                                                                     (uint32_t)s->capacity, d_cells, cells);
+  level_kernel<<<(unsigned)(cells3 * 32), kLevelThreads, 0, st>>>(s->d_mask, s->d_macro, s->bx, s->by, s->bz, s->d_level,
+                                                                  s->d_bounds, d_cells3);
+  ctx->launches.fetch_add(2);
   MESO_CUDA_TRY(cudaGetLastError());
   return MESO_OK;
 }
@@ -1144,12 +1115,12 @@ static void touched_cells(const int64_t (*lo)[3], const int64_t (*hi)[3], uint32
 // The bricks a set of sphere edits may change (the voxel boxes of the
 // spheres) and the chunks to remesh (the boxes grown by one voxel, whose
 // faces may change), both sorted by linear index.
-// The bricks and chunks the spheres' boxes touch, and the cells of 4^3, 16^3
-// and 64^3 bricks holding those bricks (all unique; all but the bricks sorted).  A cell holds a
+// The bricks and chunks the spheres' boxes touch, and the cells of 4^3 and
+// 64^3 bricks holding those bricks (all unique; all but the bricks sorted).  A cell holds a
 // touched brick iff the box overlaps it, so the cells come from the boxes
 // directly, at the cells' own granularity.
 static void edit_sets(const meso_scene* s, const meso_sphere_edit* sp, uint32_t n, std::vector<uint32_t>& bricks,
-                      std::vector<uint32_t>& chunks, std::vector<uint32_t> (&cells)[3]) {
+                      std::vector<uint32_t>& chunks, std::vector<uint32_t> (&cells)[2]) {
   const int64_t N[3] = {s->nx, s->ny, s->nz};
   std::vector<int64_t> box((size_t)n * 12);
   auto lo = reinterpret_cast<int64_t (*)[3]>(box.data());
@@ -1166,13 +1137,9 @@ static void edit_sets(const meso_scene* s, const meso_sphere_edit* sp, uint32_t 
   const int64_t B[3] = {s->bx, s->by, s->bz}, C[3] = {s->nx / 32, s->ny / 32, s->nz / 32};
   touched_cells(lo, hi, n, 3, B, bricks, /*any_order=*/true);  // the edit kernels take them in any order
   touched_cells(clo, chi, n, 5, C, chunks);
-  for (int l = 0; l < 3; l++) {
-    // cells of (4^(l+1))^3 bricks: 2^(5+2l) voxels on a side, grids as the cell maps index them
-    const int64_t cell = 4ll << (2 * l);
-    const int64_t G[3] = {l == 0 ? s->bx / 4 : (s->bx + cell - 1) / cell, l == 0 ? s->by / 4 : (s->by + cell - 1) / cell,
-                          l == 0 ? s->bz / 4 : (s->bz + cell - 1) / cell};
-    touched_cells(lo, hi, n, 5 + 2 * l, G, cells[l]);
-  }
+  const int64_t M[3] = {s->bx / 4, s->by / 4, s->bz / 4}, M3[3] = {(s->bx + 63) / 64, (s->by + 63) / 64, (s->bz + 63) / 64};
+  touched_cells(lo, hi, n, 5, M, cells[0]);
+  touched_cells(lo, hi, n, 9, M3, cells[1]);
 }
 
 meso_status edit_spheres(meso_ctx* ctx, meso_scene* s, const meso_sphere_edit* h_sp, uint32_t n, uint32_t* h_dirty,
@@ -1180,24 +1147,24 @@ meso_status edit_spheres(meso_ctx* ctx, meso_scene* s, const meso_sphere_edit* h
   if (!s || (n && !h_sp)) return fail(MESO_ERR_INVALID_ARG, "edit: null argument");
   for (uint32_t i = 0; i < n; i++)
     if (h_sp[i].radius < 0 || h_sp[i].radius > 4096) return fail(MESO_ERR_INVALID_ARG, "edit: radius out of range");
-  std::vector<uint32_t> bricks, chunks, cells[3];
+  std::vector<uint32_t> bricks, chunks, cells[2];
   edit_sets(s, h_sp, n, bricks, chunks, cells);
   if (n_dirty) *n_dirty = (uint32_t)chunks.size();
   if (h_dirty) std::copy(chunks.begin(), chunks.begin() + std::min<size_t>(chunks.size(), dirty_cap), h_dirty);
   if (bricks.empty()) return chunks.size() > dirty_cap && h_dirty ? fail(MESO_ERR_OVERFLOW, "edit: dirty list overflow") : MESO_OK;
   const size_t nb = bricks.size();
-  // only the emptiness bytes of the cells holding touched bricks are recomputed
-  // device scratch: [spheres | bricks | cells | cells2 | cells3] uploaded in
-  // one copy, then the per-brick temporaries
-  const size_t nc = cells[0].size(), nc2 = cells[1].size(), nc3 = cells[2].size();
-  const size_t up = n * sizeof(meso_sphere_edit) + 4 * (nb + nc + nc2 + nc3);
+  // only the maps of the cells holding touched bricks are recomputed
+  // device scratch: [spheres | bricks | cells | cells3] uploaded in one copy,
+  // then the per-brick temporaries
+  const size_t nc = cells[0].size(), nc3 = cells[1].size();
+  const size_t up = n * sizeof(meso_sphere_edit) + 4 * (nb + nc + nc3);
   const size_t up16 = (up + 15) & ~size_t(15);
   std::vector<uint8_t> h(up);
   std::memcpy(h.data(), h_sp, n * sizeof(meso_sphere_edit));
   size_t o = n * sizeof(meso_sphere_edit);
   std::memcpy(h.data() + o, bricks.data(), nb * 4);
   o += nb * 4;
-  for (int l = 0; l < 3; l++) {
+  for (int l = 0; l < 2; l++) {
     std::memcpy(h.data() + o, cells[l].data(), cells[l].size() * 4);
     o += cells[l].size() * 4;
   }
@@ -1207,8 +1174,7 @@ meso_status edit_spheres(meso_ctx* ctx, meso_scene* s, const meso_sphere_edit* h
   meso_sphere_edit* d_sp = reinterpret_cast<meso_sphere_edit*>(d);
   uint32_t* d_b = reinterpret_cast<uint32_t*>(d + n * sizeof(meso_sphere_edit));
   uint32_t* d_cells = d_b + nb;
-  uint32_t* d_cells2 = d_cells + nc;
-  uint32_t* d_cells3 = d_cells2 + nc2;
+  uint32_t* d_cells3 = d_cells + nc;
   uint16_t* d_temp = reinterpret_cast<uint16_t*>(d + up16);
   uint8_t* d_state = reinterpret_cast<uint8_t*>(d_temp) + nb * 1024;
   const cudaError_t ce = cudaMemcpyAsync(d, h.data(), up, cudaMemcpyHostToDevice, st);
@@ -1236,10 +1202,9 @@ meso_status edit_spheres(meso_ctx* ctx, meso_scene* s, const meso_sphere_edit* h
   const unsigned blocks = (unsigned)((nb + 7) / 8);
   edit_compute_kernel<<<blocks, 256, 0, st>>>(P);
   edit_alloc_kernel<<<blocks, 256, 0, st>>>(P);
-  edit_fix_kernel<<<1, 1, 0, st>>>(P.alloc, P.capacity);
-  ctx->launches.fetch_add(3);
+  ctx->launches.fetch_add(2);
   const meso_status mrc =
-      rebuild_macro(ctx, s, d_cells, (uint32_t)nc, st, d_cells2, (uint32_t)nc2, d_cells3, (uint32_t)nc3);
+      rebuild_macro(ctx, s, d_cells, (uint32_t)nc, st, d_cells3, (uint32_t)nc3);
   MESO_CUDA_TRY(cudaFreeAsync(d, st));
   if (mrc != MESO_OK) return mrc;
   MESO_CUDA_TRY(cudaGetLastError());
