@@ -86,7 +86,6 @@ __global__ void __launch_bounds__(kQvThreads) quads_to_vertices_kernel(const uin
 
 // ------------------------------------------------------------ erosion
 struct ErodeParams {
-  int32_t kind;
   const uint8_t* data;
   int32_t nx, ny, nz;
   const uint32_t* bptr;
@@ -99,138 +98,142 @@ struct ErodeParams {
   uint32_t* err;
 };
 
-// Occupancy of chunk-local voxel (x, y, z) of chunk c (x from the lane).
-__device__ __forceinline__ bool chunk_voxel(const ErodeParams& p, uint32_t c, int cx, int cy, int cz, int x, int y,
-                                            int z) {
-  switch (p.kind) {
-    case MESO_SRC_CHUNKS_U16: {
-      const uint32_t idx = p.coords ? (uint32_t)p.coords[c] : c;
-      return reinterpret_cast<const uint16_t*>(p.data)[(size_t)idx * 32768u + (z * 32 + y) * 32 + x] != 0;
-    }
-    case MESO_SRC_CHUNKS_U8: {
-      const uint32_t idx = p.coords ? (uint32_t)p.coords[c] : c;
-      return p.data[(size_t)idx * 32768u + (z * 32 + y) * 32 + x] != 0;
-    }
-    case MESO_SRC_GRID_U8:
-    case MESO_SRC_GRID_U16: {
-      const size_t g = (size_t)(cx * 32 + x) + (size_t)p.nx * ((size_t)(cy * 32 + y) + (size_t)p.ny * (cz * 32 + z));
-      return p.kind == MESO_SRC_GRID_U8 ? p.data[g] != 0 : reinterpret_cast<const uint16_t*>(p.data)[g] != 0;
-    }
-    default: {
-      const int gx = cx * 32 + x, gy = cy * 32 + y, gz = cz * 32 + z;
-      const uint32_t b = p.bptr[(size_t)(gx >> 3) + (size_t)p.bx * ((size_t)(gy >> 3) + (size_t)p.by * (gz >> 3))];
-      if (b == MESO_EMPTY_BRICK) return false;
-      return (p.bocc[(size_t)b * 8 + (gz & 7)] >> ((gx & 7) + 8 * (gy & 7))) & 1ull;
+// Bits of the nonzero voxels of 16 bytes: 8 (16-bit) or 16 (8-bit).
+template <bool k16>
+__device__ __forceinline__ uint32_t solid_bits(const uint4& v) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  uint32_t b = 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    if constexpr (k16) {
+      const uint32_t t = (((w[k] & 0x7FFF7FFFu) + 0x7FFF7FFFu) | w[k]) & 0x80008000u;  // a bit per half, no carry leaves it
+      b |= (t >> 15 | t >> 30) << (2 * k) & 3u << (2 * k);
+    } else {
+      const uint32_t t = (((w[k] & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | w[k]) >> 7 & 0x01010101u;
+      b |= (t * 0x01020408u >> 24) << (4 * k);  // bits 0, 8, 16, 24 to 24 .. 27; nothing else lands there
     }
   }
+  return b;
 }
 
-// One CTA (256 threads) per chunk.  Mip d from mip d-1 on bit rows (z, y):
-// (R << 1) & (R >> 1) covers the two x neighbours of the own row, and
-// Q & (Q << 1) & (Q >> 1) the three x positions of each of the 8 other rows.
+// One CTA of 8 warps per chunk.  The occupancy bits of its rows (z, y) come from
+// 16-byte loads (chunk arrays, and grids that start on 16 bytes; nx is a multiple
+// of 32, so their rows then do too), from the bricks' occupancy words, each byte
+// of which is a quarter of a row, or voxel by voxel (grids that do not).  Then
+// lane = y and a warp has four layers z in registers: mip d from mip d-1, with
+// the y neighbours by shuffles and the layers of the neighbouring warps by shared
+// memory.  P = R & (R << 1) & (R >> 1) covers the three x positions of each of the
+// 8 other rows, (R << 1) & (R >> 1) the two x neighbours of the own row.
+//
+// Bound by DRAM: 4096 uint16 chunks, depth 4, 268 MB read and 67 written in 55 us
+// (63 with the rows in shared memory and nine reads of them per row and step; 62
+// at 32 registers, which leave too few loads in flight), uint8 chunks 34 (55),
+// and chunks of a grid or a scene, which went voxel by voxel through ballots:
+// uint8 grid 45 (202), uint16 grid 62 (205), 1024^3 terrain 29 (190).
 constexpr int kErodeThreads = 256;
 constexpr int kErodeBatch = 8;  // 16-byte loads a thread has in flight at once
-static_assert(4096 % (kErodeBatch * kErodeThreads) == 0, "a uint16 chunk is whole batches of loads");
+static_assert(2048 % (kErodeBatch * kErodeThreads) == 0, "a chunk is whole batches of loads");
 
-__global__ void __launch_bounds__(kErodeThreads) erode_kernel(const ErodeParams p) {
-  __shared__ uint32_t mip0[1024], cur[1024], nxt[1024];
+template <int KIND, bool kWide>
+__global__ void __launch_bounds__(kErodeThreads, 4) erode_kernel(const ErodeParams p) {
+  constexpr bool kBrick = KIND == MESO_SRC_BRICKMAP;
+  constexpr bool kGrid = KIND == MESO_SRC_GRID_U8 || KIND == MESO_SRC_GRID_U16;
+  constexpr bool k16 = KIND == MESO_SRC_GRID_U16 || KIND == MESO_SRC_CHUNKS_U16;
+  __shared__ uint32_t rows[1024];
+  __shared__ uint32_t edge[2][16][32];  // first and last layer of each warp, of the last step and this one
   const uint32_t c = blockIdx.x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = (int)threadIdx.x, warp = t >> 5, lane = t & 31;
   int cx = 0, cy = 0, cz = 0;
-  const bool grid = p.kind == MESO_SRC_GRID_U8 || p.kind == MESO_SRC_GRID_U16 || p.kind == MESO_SRC_BRICKMAP;
+  uint32_t idx = c;
   bool ok = true;
-  if (grid) {
+  if constexpr (kGrid || kBrick) {
     cx = p.coords[3 * c];
     cy = p.coords[3 * c + 1];
     cz = p.coords[3 * c + 2];
-    const int lx = p.kind == MESO_SRC_BRICKMAP ? p.bx / 4 : p.nx / 32;
-    const int ly = p.kind == MESO_SRC_BRICKMAP ? p.by / 4 : p.ny / 32;
-    const int lz = p.kind == MESO_SRC_BRICKMAP ? p.bz / 4 : p.nz / 32;
+    const int lx = kBrick ? p.bx / 4 : p.nx / 32, ly = kBrick ? p.by / 4 : p.ny / 32, lz = kBrick ? p.bz / 4 : p.nz / 32;
     ok = cx >= 0 && cy >= 0 && cz >= 0 && cx < lx && cy < ly && cz < lz;
   } else if (p.coords) {
-    ok = (uint32_t)p.coords[c] < (uint32_t)p.nx;
+    idx = (uint32_t)p.coords[c];
+    ok = idx < (uint32_t)p.nx;
   }
   uint32_t* out = p.out + (size_t)c * p.depth * 1024;
   if (!ok) {
-    if (threadIdx.x == 0) atomicOr(p.err, ERR_BAD_INPUT);
-    for (uint32_t i = threadIdx.x; i < p.depth * 1024; i += blockDim.x) out[i] = 0;
+    if (t == 0) atomicOr(p.err, ERR_BAD_INPUT);
+    for (uint32_t i = t; i < p.depth * 1024; i += kErodeThreads) out[i] = 0;
     return;
   }
-  if (p.kind == MESO_SRC_CHUNKS_U16 || p.kind == MESO_SRC_CHUNKS_U8) {
-    // contiguous chunk: 16-byte streaming loads, kErodeBatch per thread in
-    // flight at once, each giving the occupancy bits of 8 (uint16) or 16
-    // (uint8) consecutive voxels of a row, written to the row word in shared
-    // memory as a byte or a half word (bit x = voxel x)
-    const uint32_t idx = p.coords ? (uint32_t)p.coords[c] : c;
-    if (p.kind == MESO_SRC_CHUNKS_U16) {
-      const uint4* src = reinterpret_cast<const uint4*>(p.data + (size_t)idx * 65536u);
-      uint8_t* dst = reinterpret_cast<uint8_t*>(mip0);
+  if constexpr (kBrick) {
+    // word (brick, z) holds rows y of 8 voxels, a byte each
 #pragma unroll
-      for (int i0 = 0; i0 < 4096; i0 += kErodeBatch * kErodeThreads) {
-        uint4 v[kErodeBatch];
+    for (int i = t; i < 512; i += kErodeThreads) {
+      const int b = i >> 3, z = i & 7;  // brick b of the chunk: bit x + 4y + 16z
+      const uint32_t slot = __ldg(p.bptr + (size_t)(4 * cx + (b & 3)) +
+                                  (size_t)p.bx * ((size_t)(4 * cy + ((b >> 2) & 3)) + (size_t)p.by * (size_t)(4 * cz + (b >> 4))));
+      const uint64_t w = slot != MESO_EMPTY_BRICK ? __ldg(p.bocc + (size_t)slot * 8 + z) : 0ull;
+      uint8_t* dst = reinterpret_cast<uint8_t*>(rows) + (32 * (8 * (b >> 4) + z) + 8 * ((b >> 2) & 3)) * 4 + (b & 3);
 #pragma unroll
-        for (int j = 0; j < kErodeBatch; j++) v[j] = __ldcs(src + i0 + j * kErodeThreads + threadIdx.x);
+      for (int y = 0; y < 8; y++) dst[4 * y] = (uint8_t)(w >> (8 * y));
+    }
+  } else if constexpr (kWide) {
+    constexpr int kPer = k16 ? 4 : 2;  // loads per row
+    const size_t pitch_y = kGrid ? (size_t)p.nx * (k16 ? 2 : 1) : 16 * kPer,
+                 pitch_z = kGrid ? pitch_y * (size_t)p.ny : 32 * 16 * kPer;
+    const uint8_t* src = kGrid ? p.data + (size_t)cx * (16 * kPer) + (size_t)cy * 32 * pitch_y + (size_t)cz * 32 * pitch_z
+                               : p.data + (size_t)idx * (32 * 32 * 16 * kPer);
+#pragma unroll 1
+    for (int i0 = t; i0 < 1024 * kPer; i0 += kErodeBatch * kErodeThreads) {
+      uint4 v[kErodeBatch];
 #pragma unroll
-        for (int j = 0; j < kErodeBatch; j++) {
-          const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-          uint32_t b = 0;
-#pragma unroll
-          for (int k = 0; k < 4; k++)
-            b |= ((w[k] & 0xFFFFu) != 0 ? 1u : 0u) << (2 * k) | ((w[k] >> 16) != 0 ? 2u : 0u) << (2 * k);
-          dst[i0 + j * kErodeThreads + threadIdx.x] = (uint8_t)b;
-        }
+      for (int j = 0; j < kErodeBatch; j++) {
+        const int i = i0 + j * kErodeThreads, row = i / kPer;
+        v[j] = __ldcs(reinterpret_cast<const uint4*>(src + (size_t)(row & 31) * pitch_y + (size_t)(row >> 5) * pitch_z) + i % kPer);
       }
-    } else {
-      const uint4* src = reinterpret_cast<const uint4*>(p.data + (size_t)idx * 32768u);
-      uint16_t* dst = reinterpret_cast<uint16_t*>(mip0);
 #pragma unroll
-      for (int i = threadIdx.x; i < 2048; i += kErodeThreads) {
-        const uint4 v = __ldcs(src + i);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-        uint32_t b = 0;
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-#pragma unroll
-          for (int j = 0; j < 4; j++) b |= (((w[k] >> (8 * j)) & 0xFFu) != 0 ? 1u : 0u) << (4 * k + j);
-        dst[i] = (uint16_t)b;
+      for (int j = 0; j < kErodeBatch; j++) {
+        const uint32_t b = solid_bits<k16>(v[j]);
+        if constexpr (k16) reinterpret_cast<uint8_t*>(rows)[i0 + j * kErodeThreads] = (uint8_t)b;
+        else reinterpret_cast<uint16_t*>(rows)[i0 + j * kErodeThreads] = (uint16_t)b;
       }
     }
   } else {
+#pragma unroll 4
     for (int row = warp; row < 1024; row += kErodeThreads / 32) {
       const int z = row >> 5, y = row & 31;
-      const uint32_t w = __ballot_sync(kFull, chunk_voxel(p, c, cx, cy, cz, lane, y, z));
-      if (lane == 0) mip0[row] = w;
+      const size_t g = (size_t)(cx * 32 + lane) + (size_t)p.nx * ((size_t)(cy * 32 + y) + (size_t)p.ny * (size_t)(cz * 32 + z));
+      const uint32_t w = __ballot_sync(kFull, (k16 ? reinterpret_cast<const uint16_t*>(p.data)[g] : p.data[g]) != 0);
+      if (lane == 0) rows[row] = w;
     }
   }
   __syncthreads();
-  for (int row = threadIdx.x; row < 1024; row += blockDim.x) {
-    cur[row] = mip0[row];
-    out[row] = mip0[row];
+  uint32_t mip0[4], R[6];  // this warp's layers 4 warp .. + 3, and R also the ones around them
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    mip0[j] = R[j + 1] = rows[32 * (4 * warp + j) + lane];
+    out[32 * (4 * warp + j) + lane] = mip0[j];
+    // the chunk's first and last voxels have neighbours outside it
+    const bool border = lane == 0 || lane == 31 || (warp == 0 && j == 0) || (warp == 7 && j == 3);
+    mip0[j] = border ? 0u : mip0[j] & 0x7FFFFFFEu;
   }
-  __syncthreads();
   for (uint32_t d = 1; d < p.depth; d++) {
-    for (int row = threadIdx.x; row < 1024; row += blockDim.x) {
-      const int z = row >> 5, y = row & 31;
-      uint32_t acc = 0;
-      if (y >= 1 && y <= 30 && z >= 1 && z <= 30) {
-        const uint32_t R = cur[row];
-        acc = (R << 1) & (R >> 1);
+    uint32_t(*const e)[32] = edge[d & 1];
+    e[2 * warp][lane] = R[1];
+    e[2 * warp + 1][lane] = R[4];
+    __syncthreads();
+    R[0] = e[warp > 0 ? 2 * warp - 1 : 0][lane];
+    R[5] = e[warp < 7 ? 2 * warp + 2 : 15][lane];
+    uint32_t sides[6], all[6];  // rows y - 1 and y + 1, and the three of them
 #pragma unroll
-        for (int dz = -1; dz <= 1; dz++)
-#pragma unroll
-          for (int dy = -1; dy <= 1; dy++) {
-            if (dz == 0 && dy == 0) continue;
-            const uint32_t Q = cur[row + dz * 32 + dy];
-            acc &= Q & (Q << 1) & (Q >> 1);
-          }
-        acc &= mip0[row] & 0x7FFFFFFEu;
-      }
-      nxt[row] = acc;
-      out[(size_t)d * 1024 + row] = acc;
+    for (int j = 0; j < 6; j++) {
+      const uint32_t P = R[j] & (R[j] << 1) & (R[j] >> 1);
+      sides[j] = __shfl_up_sync(kFull, P, 1) & __shfl_down_sync(kFull, P, 1);
+      all[j] = sides[j] & P;
     }
-    __syncthreads();
-    for (int row = threadIdx.x; row < 1024; row += blockDim.x) cur[row] = nxt[row];
-    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t r = R[j + 1];
+      R[j + 1] = all[j] & all[j + 2] & sides[j + 1] & (r << 1) & (r >> 1) & mip0[j];
+      out[(size_t)d * 1024 + 32 * (4 * warp + j) + lane] = R[j + 1];
+    }
   }
 }
 
@@ -267,7 +270,6 @@ meso_status meso_erode_mips(meso_ctx* ctx, const meso_mesh_source* src, const in
   if (n > 0x7FFFFFFFu) return fail(MESO_ERR_INVALID_ARG, "erode_mips: too many chunks");
   ErodeParams p;
   memset(&p, 0, sizeof(p));
-  p.kind = src->kind;
   p.coords = d_coords;
   p.n = n;
   p.depth = depth;
@@ -296,7 +298,21 @@ meso_status meso_erode_mips(meso_ctx* ctx, const meso_mesh_source* src, const in
   } else {
     return fail(MESO_ERR_INVALID_ARG, "erode_mips: unknown source kind");
   }
-  erode_kernel<<<n, kErodeThreads, 0, pick_stream(ctx, stream)>>>(p);
+  const cudaStream_t st = pick_stream(ctx, stream);
+  const bool wide = (reinterpret_cast<uintptr_t>(p.data) & 15u) == 0;
+  switch (src->kind) {
+    case MESO_SRC_CHUNKS_U16: erode_kernel<MESO_SRC_CHUNKS_U16, true><<<n, kErodeThreads, 0, st>>>(p); break;
+    case MESO_SRC_CHUNKS_U8: erode_kernel<MESO_SRC_CHUNKS_U8, true><<<n, kErodeThreads, 0, st>>>(p); break;
+    case MESO_SRC_GRID_U8:
+      if (wide) erode_kernel<MESO_SRC_GRID_U8, true><<<n, kErodeThreads, 0, st>>>(p);
+      else erode_kernel<MESO_SRC_GRID_U8, false><<<n, kErodeThreads, 0, st>>>(p);
+      break;
+    case MESO_SRC_GRID_U16:
+      if (wide) erode_kernel<MESO_SRC_GRID_U16, true><<<n, kErodeThreads, 0, st>>>(p);
+      else erode_kernel<MESO_SRC_GRID_U16, false><<<n, kErodeThreads, 0, st>>>(p);
+      break;
+    default: erode_kernel<MESO_SRC_BRICKMAP, false><<<n, kErodeThreads, 0, st>>>(p);
+  }
   ctx->launches.fetch_add(1);
   MESO_CUDA_TRY(cudaGetLastError());
   return MESO_OK;
