@@ -17,7 +17,8 @@
 //     chunk of a dense grid; for a brick map 16-byte copies of the occupied
 //     bricks by the whole CTA, after the chunk has been picked out of a
 //     ticket of chunks tested together against the scene's cell map); the
-//     one-voxel occupancy halo is read with plain loads while it lands;
+//     one-voxel occupancy halo is read with plain loads while it lands (the
+//     columns beside a grid chunk's X faces arrive by TMA too);
 //  2. masks: a lane takes 8 voxels of a row with one wide load, a warp 8 rows;
 //     packed 16-bit (8-bit) operations give the byte of the row's occupancy
 //     word and of its material-equality words with the -x, -y and -z
@@ -33,6 +34,7 @@
 #include <cudaTypedefs.h>
 
 #include <cstdio>
+#include <cstddef>
 #include <cstring>
 
 #include "meso_internal.h"
@@ -53,20 +55,21 @@ constexpr int kArr = 32 * kS;
 constexpr int kFew = 2, kSome = 8;
 constexpr int kBrickSlot = 1040;     // bytes per staged brick (bank-spread padding)
 constexpr uint32_t kFull = 0xFFFFFFFFu;
+constexpr uint32_t kSideBytes = 32 * 32 * 16;  // the column of 16 bytes beside a grid chunk, for its X halo
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
 
-// Shared memory of one CTA: these arrays, then the staged materials of the
-// chunk (KindTraits::kMatBytes, 128-byte aligned).
+// Shared memory of one CTA: these arrays (the words first: see kSideBytes), then
+// the staged materials of the chunk (KindTraits::kMatBytes, 128-byte aligned).
 struct __align__(128) MeshSmem {
   uint32_t occ[kArr];                     // occupancy, bits over x, [z][y]
   uint32_t occt[kArr];                    // occupancy, bits over y, [z][x]
   uint32_t ex[kArr], ey[kArr], ez[kArr];  // equality with -x / -y / -z neighbour, bits over x, [z][y]
   uint32_t eyt[kArr], ezt[kArr];          // equality with -y / -z neighbour, bits over y, [z][x]
-  uint32_t halo[6][32];                   // -X,+X: bits y by z; -Y,+Y: bits x by z; -Z,+Z: bits x by y
   // columns that continue a quad from the row above, bits and layout as the
   // words of the direction: the odd directions'; the even directions' replace
   // the equality with the row above, which the sweep is the last to read
   uint32_t cont[3][kArr];
+  uint32_t halo[6][32];                   // -X,+X: bits y by z; -Y,+Y: bits x by z; -Z,+Z: bits x by y
   uint64_t quad_base[6];                  // per direction: first output index of its quads
   uint32_t quad_next[6];                  // how many of them have their place
   uint32_t start_rows[18][32];            // per class and direction, per row: slices with such a word
@@ -83,6 +86,8 @@ struct __align__(128) MeshSmem {
   uint32_t task_next;                     // dynamic task counter of the emission
   uint32_t any_solid;
 };
+
+static_assert(offsetof(MeshSmem, halo) >= 2 * kSideBytes, "a grid chunk's two side columns land in the word arrays");
 
 struct MeshParams {
   const uint8_t* data;
@@ -317,12 +322,13 @@ __device__ __forceinline__ void take_chunk(Job& job, const MeshParams& p, const 
   }
 }
 
-// Starts the copy of the job's materials into the staging buffer (one thread;
+// Starts the copy of the job's materials into the staging buffer and, for a
+// grid, of the columns beside its X faces into the word arrays (one thread;
 // brick maps are copied by the whole CTA, their phase of the barrier completes
 // with no bytes).
 template <int KIND, typename Job>
 __device__ __forceinline__ void stage_chunk(MeshSmem& sm, uint8_t* dst, const Job& job, const MeshParams& p,
-                                            const CUtensorMap* tmap) {
+                                            const CUtensorMap* tmap, const CUtensorMap* hmap) {
   using T = KindTraits<KIND>;
   uint64_t* bar = &sm.bar;
   if (T::kBrick || job.valid != 1) {
@@ -331,9 +337,13 @@ __device__ __forceinline__ void stage_chunk(MeshSmem& sm, uint8_t* dst, const Jo
   }
   fence_proxy_async_smem();
   const uint32_t bytes = 32768u * T::kElem;
-  mbar_arrive_expect_tx(bar, bytes);
+  mbar_arrive_expect_tx(bar, bytes + (T::kGrid ? 2u * kSideBytes : 0u));
   if constexpr (T::kGrid) {
-    tma_load_3d(dst, tmap, job.coord[0] * 32, job.coord[1] * 32, job.coord[2] * 32, bar);
+    const int x = job.coord[0] * 32, y = job.coord[1] * 32, z = job.coord[2] * 32;
+    uint8_t* const sides = reinterpret_cast<uint8_t*>(&sm);
+    tma_load_3d(sides, hmap, x - 16 / T::kElem, y, z, bar);
+    tma_load_3d(sides + kSideBytes, hmap, x + 32, y, z, bar);
+    tma_load_3d(dst, tmap, x, y, z, bar);
   } else {
     const uint8_t* src = p.data + (size_t)(uint32_t)job.coord[0] * bytes;
     for (uint32_t off = 0; off < bytes; off += 16384u) bulk_g2s(dst + off, src + off, 16384u, bar);
@@ -366,23 +376,22 @@ __device__ __forceinline__ void brick_halos(MeshSmem& sm, const int32_t (&coord)
   }
 }
 
-// The same for a dense grid: 6 faces x 32 rows, a row per ballot; each warp
-// reads its 12 rows' voxels first so all of them are in flight together.
+// The same for the Y and Z faces of a dense grid: 4 faces x 32 rows, a row per
+// ballot; each warp reads its 8 rows' voxels first so all of them are in flight
+// together.
 template <int KIND>
 __device__ __forceinline__ void compute_halos(MeshSmem& sm, const int32_t (&coord)[3], const MeshParams& p, int warp,
                                               int lane) {
-  constexpr int kPer = 6 * 32 / kWarps;
-  static_assert(kPer * kWarps == 6 * 32, "halo rows split evenly over the warps");
+  constexpr int kPer = 4 * 32 / kWarps;
+  static_assert(kPer * kWarps == 4 * 32, "halo rows split evenly over the warps");
   const int X = coord[0] * 32, Y = coord[1] * 32, Z = coord[2] * 32;
   uint32_t solid[kPer];
 #pragma unroll
   for (int i = 0; i < kPer; i++) {
-    const int wi = warp + kWarps * i;
+    const int wi = 64 + warp + kWarps * i;
     const int f = wi >> 5, k = wi & 31;
     int gx, gy, gz;
     switch (f) {
-      case 0: gx = X - 1; gy = Y + lane; gz = Z + k; break;
-      case 1: gx = X + 32; gy = Y + lane; gz = Z + k; break;
       case 2: gx = X + lane; gy = Y - 1; gz = Z + k; break;
       case 3: gx = X + lane; gy = Y + 32; gz = Z + k; break;
       case 4: gx = X + lane; gy = Y + k; gz = Z - 1; break;
@@ -392,7 +401,7 @@ __device__ __forceinline__ void compute_halos(MeshSmem& sm, const int32_t (&coor
   }
 #pragma unroll
   for (int i = 0; i < kPer; i++) {
-    const int wi = warp + kWarps * i;
+    const int wi = 64 + warp + kWarps * i;
     const uint32_t w = __ballot_sync(kFull, solid[i] != 0);
     if (lane == 0) sm.halo[wi >> 5][wi & 31] = w;
   }
@@ -673,7 +682,7 @@ __device__ __forceinline__ void emit_words(MeshSmem& sm, const MeshParams& p, co
 
 template <int KIND>
 __global__ void __launch_bounds__(kThreads, KindTraits<KIND>::kCtasPerSm)
-    mesh_kernel(const MeshParams p, const __grid_constant__ CUtensorMap tmap) {
+    mesh_kernel(const MeshParams p, const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap hmap) {
   using T = KindTraits<KIND>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base_addr = smem_u32(smem_raw);
@@ -704,7 +713,7 @@ __global__ void __launch_bounds__(kThreads, KindTraits<KIND>::kCtasPerSm)
     const int c = job.chunk;
     if (c < 0) break;
     const bool valid = job.valid == 1;
-    if (tid == 0) stage_chunk<KIND>(sm, mat, job, p, &tmap);
+    if (tid == 0) stage_chunk<KIND>(sm, mat, job, p, &tmap, &hmap);
     if constexpr (T::kBrick) {
       if (valid) {
         // 64 bricks x 64 pieces of 16 bytes; a warp covers 512 contiguous
@@ -741,6 +750,27 @@ __global__ void __launch_bounds__(kThreads, KindTraits<KIND>::kCtasPerSm)
       }
       __syncthreads();
       return;
+    }
+    if constexpr (T::kGrid) {
+      // The X faces' halo from the columns of 16 bytes beside the chunk, one row
+      // per ballot.  A voxel there is alone in its line, and as plain loads these
+      // 2048 were 12 % of a chunk's time in the load pipe and most of the wait for
+      // its data; TMA takes them past it, into the word arrays, which are idle
+      // between two chunks, and fills what lies outside of the grid with zeros.
+      // 4096 chunks of a grid: uint8 235 -> 196 us, uint16 241 -> 192; with the
+      // columns prefetched into L2 like the chunk 204 and 200.
+      if (valid) {
+        const uint8_t* sides = reinterpret_cast<const uint8_t*>(&sm);
+#pragma unroll
+        for (int i = 0; i < 64 / kWarps; i++) {
+          const int wi = warp + kWarps * i, f = wi >> 5, k = wi & 31;
+          const uint8_t* a = sides + f * kSideBytes + (k * 32 + lane) * 16 + (f ? 0 : 16 - T::kElem);
+          const uint32_t v = T::kElem == 2 ? *reinterpret_cast<const uint16_t*>(a) : *a;
+          const uint32_t w = __ballot_sync(kFull, v != 0);
+          if (lane == 0) sm.halo[f][k] = w;
+        }
+      }
+      __syncthreads();
     }
     if (valid) {
       const uint8_t* mb = mat;
@@ -869,12 +899,12 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encode_fn() {
   return fn;
 }
 
-meso_status make_grid_map(const meso_mesh_source* src, int elem, CUtensorMap* map) {
+meso_status make_grid_map(const meso_mesh_source* src, int elem, uint32_t width, CUtensorMap* map) {
   auto enc = get_encode_fn();
   if (!enc) return fail(MESO_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
   cuuint64_t dims[3] = {(cuuint64_t)src->nx, (cuuint64_t)src->ny, (cuuint64_t)src->nz};
   cuuint64_t strides[2] = {(cuuint64_t)src->nx * elem, (cuuint64_t)src->nx * src->ny * elem};
-  cuuint32_t box[3] = {32, 32, 32};
+  cuuint32_t box[3] = {width, 32, 32};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = enc(map, elem == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 3,
                    const_cast<void*>(src->d_data), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -885,7 +915,7 @@ meso_status make_grid_map(const meso_mesh_source* src, int elem, CUtensorMap* ma
 }
 
 template <int KIND>
-meso_status launch_kind(meso_ctx* ctx, const MeshParams& base, const CUtensorMap& tmap, uint32_t n_chunks,
+meso_status launch_kind(meso_ctx* ctx, const MeshParams& base, const CUtensorMap& tmap, const CUtensorMap& hmap, uint32_t n_chunks,
                         cudaStream_t st, bool per_launch) {
   const size_t smem = sizeof(MeshSmem) + KindTraits<KIND>::kMatBytes + 128;
   static bool attr_set[64] = {false};
@@ -906,7 +936,7 @@ meso_status launch_kind(meso_ctx* ctx, const MeshParams& base, const CUtensorMap
       else if (base.coords) p.coords = base.coords + i;
       else p.data = base.data + (size_t)i * 32768u * KindTraits<KIND>::kElem;
       if (p.chunk_counts) p.chunk_counts = base.chunk_counts + i;
-      mesh_kernel<KIND><<<1, kThreads, smem, st>>>(p, tmap);
+      mesh_kernel<KIND><<<1, kThreads, smem, st>>>(p, tmap, hmap);
       ctx->launches.fetch_add(1);
     }
     MESO_CUDA_TRY(cudaGetLastError());
@@ -934,7 +964,7 @@ meso_status launch_kind(meso_ctx* ctx, const MeshParams& base, const CUtensorMap
   if (grid > need) grid = need;
   if (grid == 0) grid = 1;
   MESO_CUDA_TRY(cudaMemsetAsync(p.ticket, 0, sizeof(uint32_t), st));
-  mesh_kernel<KIND><<<grid, kThreads, smem, st>>>(p, tmap);
+  mesh_kernel<KIND><<<grid, kThreads, smem, st>>>(p, tmap, hmap);
   ctx->launches.fetch_add(1);
   MESO_CUDA_TRY(cudaGetLastError());
   return MESO_OK;
@@ -961,8 +991,9 @@ meso_status launch_mesh(meso_ctx* ctx, const meso_mesh_source* src, const int32_
   p.err = ctx->d_scratch + 1;
   p.per_ticket = ctx->tuning.mesh_chunks_per_ticket ? ctx->tuning.mesh_chunks_per_ticket : 1;
   p.chunk_id_base = chunk_id_base;
-  CUtensorMap tmap;
+  CUtensorMap tmap, hmap;
   memset(&tmap, 0, sizeof(tmap));
+  memset(&hmap, 0, sizeof(hmap));
   const int kind = src->kind;
   if (kind == MESO_SRC_BRICKMAP) {
     const meso_scene* s = src->scene;
@@ -988,7 +1019,9 @@ meso_status launch_mesh(meso_ctx* ctx, const meso_mesh_source* src, const int32_
       if (!d_coords && n_chunks) return fail(MESO_ERR_INVALID_ARG, "mesh: grid source needs chunk coordinates");
       if ((reinterpret_cast<uintptr_t>(src->d_data) & 15u) != 0)
         return fail(MESO_ERR_INVALID_ARG, "mesh: grid base must be 16-byte aligned");
-      MESO_TRY(make_grid_map(src, kind == MESO_SRC_GRID_U16 ? 2 : 1, &tmap));
+      const int elem = kind == MESO_SRC_GRID_U16 ? 2 : 1;
+      MESO_TRY(make_grid_map(src, elem, 32, &tmap));
+      MESO_TRY(make_grid_map(src, elem, 16 / elem, &hmap));
     } else if (kind == MESO_SRC_CHUNKS_U16 || kind == MESO_SRC_CHUNKS_U8) {
       if ((reinterpret_cast<uintptr_t>(src->d_data) & 15u) != 0)
         return fail(MESO_ERR_INVALID_ARG, "mesh: chunk array must be 16-byte aligned");
@@ -1001,11 +1034,11 @@ meso_status launch_mesh(meso_ctx* ctx, const meso_mesh_source* src, const int32_
   if (!accumulate) MESO_CUDA_TRY(cudaMemsetAsync(out->d_quad_count, 0, sizeof(uint64_t), st));
   if (n_chunks == 0) return MESO_OK;
   switch (kind) {
-    case MESO_SRC_CHUNKS_U16: return launch_kind<MESO_SRC_CHUNKS_U16>(ctx, p, tmap, n_chunks, st, per_launch);
-    case MESO_SRC_CHUNKS_U8: return launch_kind<MESO_SRC_CHUNKS_U8>(ctx, p, tmap, n_chunks, st, per_launch);
-    case MESO_SRC_GRID_U8: return launch_kind<MESO_SRC_GRID_U8>(ctx, p, tmap, n_chunks, st, per_launch);
-    case MESO_SRC_GRID_U16: return launch_kind<MESO_SRC_GRID_U16>(ctx, p, tmap, n_chunks, st, per_launch);
-    default: return launch_kind<MESO_SRC_BRICKMAP>(ctx, p, tmap, n_chunks, st, per_launch);
+    case MESO_SRC_CHUNKS_U16: return launch_kind<MESO_SRC_CHUNKS_U16>(ctx, p, tmap, hmap, n_chunks, st, per_launch);
+    case MESO_SRC_CHUNKS_U8: return launch_kind<MESO_SRC_CHUNKS_U8>(ctx, p, tmap, hmap, n_chunks, st, per_launch);
+    case MESO_SRC_GRID_U8: return launch_kind<MESO_SRC_GRID_U8>(ctx, p, tmap, hmap, n_chunks, st, per_launch);
+    case MESO_SRC_GRID_U16: return launch_kind<MESO_SRC_GRID_U16>(ctx, p, tmap, hmap, n_chunks, st, per_launch);
+    default: return launch_kind<MESO_SRC_BRICKMAP>(ctx, p, tmap, hmap, n_chunks, st, per_launch);
   }
 }
 
