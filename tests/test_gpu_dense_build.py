@@ -52,3 +52,20 @@ def test_empty_grid(ctx):
     assert int(scene.info().n_bricks) == 0
     assert (scene.download()[0] == meso.EMPTY_BRICK).all()
     scene.destroy()
+
+
+@pytest.mark.parametrize("dims", [(32, 32, 32), (96, 64, 32), (512, 512, 64), (512, 512, 544)])
+def test_bricks_are_numbered_in_order(ctx, dims):
+    # words of 32 bricks: fewer than a thread of the scan takes, fewer than one
+    # tile (8192), and more than one with a rest
+    nx, ny, nz = dims
+    rng = np.random.default_rng(nz)
+    keep = rng.random((nz // 8, ny // 8, nx // 8)) < 0.4
+    g = np.zeros(dims[::-1], dtype=np.uint8)
+    z, y, x = np.nonzero(keep)
+    g[8 * z + rng.integers(0, 8, z.size), 8 * y + rng.integers(0, 8, z.size), 8 * x + rng.integers(0, 8, z.size)] = 1
+    scene = build(ctx, meso.SRC_GRID_U8, g, 0)
+    k = keep.reshape(-1)
+    assert np.array_equal(scene.download()[0], np.where(k, np.cumsum(k) - 1, meso.EMPTY_BRICK).astype(np.uint32))
+    assert int(scene.info().n_bricks) == k.sum()
+    scene.destroy()
