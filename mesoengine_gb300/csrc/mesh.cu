@@ -952,13 +952,16 @@ meso_status launch_kind(meso_ctx* ctx, const MeshParams& base, const CUtensorMap
   const uint32_t tuned = ctx->tuning.mesh_ctas_per_sm;
   uint32_t grid = ctx->sm_count * (tuned && tuned < kMaxCtas ? tuned : kMaxCtas);
   if constexpr (KindTraits<KIND>::kBrick) {
-    // tickets of up to 8 list entries (tested together against the cell
-    // map) once every CTA gets several: on all 32,768 chunks of a 1024^3
-    // terrain (80 % air) tickets of 4 or 8 measured 0.84 ms, 16 0.87, 32 0.92
-    // (the last tickets leave CTAs with several heavy chunks each).  7919 and
-    // 104729 are primes, and no list of at most 2^20 entries is a multiple of
-    // both, so t -> (t * perm_mul) mod n is a bijection
-    const uint32_t b = n_chunks / grid;
+    // tickets of up to 8 list entries (tested together against the cell map) as
+    // long as a CTA gets 8 of them, fewer to a ticket on shorter lists: what a CTA
+    // still holds when the queue runs out, the others wait for.  (us, with up to 8
+    // as soon as there are as many entries per CTA, and so: 4096 chunks at a
+    // terrain's ground 209 and 170, 2500 of them 150 and 109, 1200 76 and 61, all
+    // 8000 of a 640^3 terrain 130 and 104, all 32,768 of a 1024^3 one, 80 % of
+    // them air, 290 both; there tickets of 2, 4 and 16 take 311, 291 and 300.)
+    // 7919 and 104729 are primes, and no list of at most 2^20 entries is a
+    // multiple of both, so t -> (t * perm_mul) mod n is a bijection
+    const uint32_t b = n_chunks / (grid * 8u);
     p.per_ticket = b < 1 ? 1 : (b > 8 ? 8 : b);
     p.perm_mul = n_chunks % 7919u ? 7919u : 104729u;
   }

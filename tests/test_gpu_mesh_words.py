@@ -90,3 +90,20 @@ def test_neighbouring_chunks(ctx, dtype):
     q, _ = ctx.mesh(meso.SRC_BRICKMAP, coords=coords, scene=scene)
     assert np.array_equal(np.sort(q), ref)
     scene.destroy()
+
+
+@pytest.mark.parametrize("n", [1, 303, 305, 2431, 2432, 4864, 4871])
+def test_lists_around_the_ticket_sizes(ctx, n):
+    # entries per ticket change with the list's length; every entry is meshed
+    # once, air chunks and chunks that the list names again among them
+    g = np.zeros((64, 96, 96), dtype=np.uint16)
+    g[:32, 32:64, 64:96] = CH[9 % len(CH)]
+    g[32:40, 5, :50] = 3
+    scene = ctx.scene_from_dense(g)
+    every = np.array([(x, y, z) for z in range(2) for y in range(3) for x in range(3)], dtype=np.int32)
+    ref = [oracle.mesh_chunks(oracle.SRC_GRID_U16, g, coords=every[k:k + 1]) for k in range(len(every))]
+    coords = np.resize(every, (n, 3))
+    q, _ = ctx.mesh(meso.SRC_BRICKMAP, coords=coords, scene=scene)
+    want = np.concatenate([ref[k % len(every)] | np.uint64(k << 44) for k in range(n)])
+    assert np.array_equal(np.sort(q), np.sort(want))
+    scene.destroy()
