@@ -20,8 +20,8 @@
 // What bounds it: the instructions of the loop (141 per warp and turn, 45 % of
 // them on the half-rate ALU pipe) and, for small images and at the end of a
 // launch, the longest ray's chain of up to about 100 turns of some 0.3 us.
-// 1920x1080, primary and shadow rays, 1024^3 terrain: 112 M warp instructions
-// with 24.4 of 32 lanes active in 132 us, where separate loops for cell jumps,
+// 1920x1080, primary and shadow rays, 1024^3 terrain: 102 M warp instructions
+// with 23.8 of 32 lanes active in 132 us, where separate loops for cell jumps,
 // brick steps and voxel steps took 290 M with 16.6 lanes in 384 us; DRAM is
 // idle (1 %).
 #include <cmath>
@@ -116,7 +116,7 @@ __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? l
 // takes this path to count its fetches, and so does any ray whose values lie
 // outside what the region walk below was proven for.
 template <bool kStats>
-__device__ __noinline__ void walk_steps(const RayView& V, int bx0, int by0, int bz0, float ox, float oy, float oz,
+__device__ __forceinline__ void walk_steps(const RayView& V, int bx0, int by0, int bz0, float ox, float oy, float oz,
                                         float dx, float dy, float dz, float ix, float iy, float iz, int vx, int vy,
                                         int vz, float t, int ea, Trav& r) {
   uint32_t n_fetch = 0, n_brick = 0;
@@ -129,6 +129,7 @@ __device__ __noinline__ void walk_steps(const RayView& V, int bx0, int by0, int 
   uint32_t cs = 0, fs = 0;
   const uint32_t cap = (uint32_t)(4 * (V.nx + V.ny + V.nz) + 64);
   uint32_t p = MESO_EMPTY_BRICK;
+  bool entered = false;  // into this brick from an empty one
   r.hit = 0;
   for (;;) {
     if (cs + fs > cap) break;
@@ -155,15 +156,19 @@ __device__ __noinline__ void walk_steps(const RayView& V, int bx0, int by0, int 
       By += a == 1 ? sy : 0;
       Bz += a == 2 ? sz : 0;
       if (((unsigned)Bx >= (unsigned)NBx) | ((unsigned)By >= (unsigned)NBy) | ((unsigned)Bz >= (unsigned)NBz)) break;
+      entered = true;
+      continue;
+    }
+    if (entered) {
       // the voxel entered: exact along the stepped axis, floor of the entry
       // point (clamped into the brick) along the others
       const int fx = clampi((int)floorf(__fadd_rn(ox, __fmul_rn(dx, t))) + bx0, Bx * 8, Bx * 8 + 7);
       const int fy = clampi((int)floorf(__fadd_rn(oy, __fmul_rn(dy, t))) + by0, By * 8, By * 8 + 7);
       const int fz = clampi((int)floorf(__fadd_rn(oz, __fmul_rn(dz, t))) + bz0, Bz * 8, Bz * 8 + 7);
-      vx = a == 0 ? (sx > 0 ? Bx * 8 : Bx * 8 + 7) : fx;
-      vy = a == 1 ? (sy > 0 ? By * 8 : By * 8 + 7) : fy;
-      vz = a == 2 ? (sz > 0 ? Bz * 8 : Bz * 8 + 7) : fz;
-      continue;
+      vx = ea == 0 ? (sx > 0 ? Bx * 8 : Bx * 8 + 7) : fx;
+      vy = ea == 1 ? (sy > 0 ? By * 8 : By * 8 + 7) : fy;
+      vz = ea == 2 ? (sz > 0 ? Bz * 8 : Bz * 8 + 7) : fz;
+      entered = false;
     }
     // voxel steps inside occupied brick p
     const uint64_t* occ = V.occ + (size_t)p * 8;
@@ -213,6 +218,13 @@ __device__ __noinline__ void walk_steps(const RayView& V, int bx0, int by0, int 
   r.fine = fs;
   r.fetches = n_fetch;
   r.bricks = n_brick;
+}
+
+// Out of line where few rays take it: it shares no registers with the region walk.
+__device__ __noinline__ void walk_steps_apart(const RayView& V, int bx0, int by0, int bz0, float ox, float oy, float oz,
+                                              float dx, float dy, float dz, float ix, float iy, float iz, int vx, int vy,
+                                              int vz, float t, int ea, Trav& r) {
+  walk_steps<false>(V, bx0, by0, bz0, ox, oy, oz, dx, dy, dz, ix, iy, iz, vx, vy, vz, t, ea, r);
 }
 
 // ---------------------------------------------------------- region walk
@@ -483,16 +495,17 @@ template <bool kStats>
 __device__ __forceinline__ void trace(const RayView& V, float margin, int bx0, int by0, int bz0, float ox, float oy,
                                       float oz, float dx, float dy, float dz, float ix, float iy, float iz, int vx,
                                       int vy, int vz, float t, int ea, Trav& r) {
-  const bool regions = !kStats && margin > 0.0f && regular_axis(dx) && regular_axis(dy) && regular_axis(dz) &&
-                       (dx != 0.0f || dy != 0.0f || dz != 0.0f);
-  if (regions) {
+  if constexpr (kStats) {
+    walk_steps<true>(V, bx0, by0, bz0, ox, oy, oz, dx, dy, dz, ix, iy, iz, vx, vy, vz, t, ea, r);
+  } else if (margin > 0.0f && regular_axis(dx) && regular_axis(dy) && regular_axis(dz) &&
+             (dx != 0.0f || dy != 0.0f || dz != 0.0f)) {
     const int4 nlo = __ldg(V.bounds), hi = __ldg(V.bounds + 1);
     const RayAxis X = ray_axis(bx0, ox, dx, ix, nlo.x, hi.x), Y = ray_axis(by0, oy, dy, iy, nlo.y, hi.y),
                   Z = ray_axis(bz0, oz, dz, iz, nlo.z, hi.z);
     walk_regions(V, X, Y, Z, margin, vx, vy, vz, t, ea, r);
   } else {
     Trav q;
-    walk_steps<kStats>(V, bx0, by0, bz0, ox, oy, oz, dx, dy, dz, ix, iy, iz, vx, vy, vz, t, ea, q);
+    walk_steps_apart(V, bx0, by0, bz0, ox, oy, oz, dx, dy, dz, ix, iy, iz, vx, vy, vz, t, ea, q);
     r = q;
   }
 }
