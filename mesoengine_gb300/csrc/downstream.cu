@@ -398,24 +398,20 @@ meso_status meso_scene_load(meso_ctx* ctx, const char* path, uint64_t spare, mes
     if (ptr[b] != MESO_EMPTY_BRICK && ptr[b] >= n) return fail(MESO_ERR_INVALID_ARG, "scene_load: bad brick pointer");
   meso_scene* s = nullptr;
   MESO_TRY(scene_alloc(ctx, nx, ny, nz, n + spare, &s));
-  // the arrays are ordered after ctx->stream's allocation, the copies below
-  // are on the default stream
-  cudaError_t e = cudaStreamSynchronize(ctx->stream);
-  if (e == cudaSuccess) e = cudaMemcpy(s->d_ptr, ptr.data(), nb * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && n) e = cudaMemcpy(s->d_occ, occ.data(), n * 64, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && n) e = cudaMemcpy(s->d_mat, mat.data(), n * 1024, cudaMemcpyHostToDevice);
+  // All on ctx->stream, as the arrays' allocation and the maps' kernels are: a
+  // pageable copy on the default stream may return before its data has reached
+  // the device, and ctx->stream does not wait for that one.
+  const cudaStream_t st = ctx->stream;
   const int32_t alloc[4] = {(int32_t)n, 0, 0, 0};
-  if (e == cudaSuccess) e = cudaMemcpy(s->d_alloc, alloc, 16, cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) {
-    scene_release(ctx, s);
-    return cuda_fail(e, "scene_load: upload");
-  }
-  meso_status rc = rebuild_macro(ctx, s, nullptr, 0, ctx->stream);
-  if (rc == MESO_OK) rc = rebuild_sub(ctx, s, n, ctx->stream);
-  if (rc == MESO_OK) {
-    e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) rc = cuda_fail(e, "scene_load: macro map");
-  }
+  cudaError_t e = cudaMemcpyAsync(s->d_ptr, ptr.data(), nb * 4, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && n) e = cudaMemcpyAsync(s->d_occ, occ.data(), n * 64, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && n) e = cudaMemcpyAsync(s->d_mat, mat.data(), n * 1024, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(s->d_alloc, alloc, 16, cudaMemcpyHostToDevice, st);
+  meso_status rc = e == cudaSuccess ? MESO_OK : cuda_fail(e, "scene_load: upload");
+  if (rc == MESO_OK) rc = rebuild_macro(ctx, s, nullptr, 0, st);
+  if (rc == MESO_OK) rc = rebuild_sub(ctx, s, n, st);
+  e = cudaStreamSynchronize(st);  // also after a failure: the copies read this call's memory
+  if (rc == MESO_OK && e != cudaSuccess) rc = cuda_fail(e, "scene_load: macro map");
   if (rc != MESO_OK) {
     scene_release(ctx, s);
     return rc;
