@@ -90,7 +90,8 @@ struct meso_scene {
   int32_t* d_bounds = nullptr; // of the occupied 4x4x4-brick cells, in voxels: [0..2] the largest -lowest, [4..6] the
                                // largest highest coordinate per axis; edits only widen them
   uint64_t* d_mask = nullptr;  // per 4x4x4-brick cell: its occupied bricks, bit x + 4y + 16z
-  uint64_t* d_sub = nullptr;   // per pool slot: the non-empty 2x2x2-voxel blocks, bit x + 4y + 16z
+  uint64_t* d_sub = nullptr;   // per pool slot: the non-empty 2x2x2-voxel blocks, bit x + 4y + 16z; one more word
+                               // before them, zero, for rays that read an unlinked brick's pointer as a slot
   uint64_t capacity = 0;       // pool slots
   // allocator state (device): [0] bump (slots ever used), [1] free-stack top
   int64_t* d_alloc = nullptr;

@@ -604,15 +604,17 @@ unsigned grid_for(uint64_t warps, int threads = 256) {
 // One warp per macro cell (4x4x4 bricks): the mask of its occupied bricks
 // (bit x + 4y + 16z), and a byte that says whether there are any.  Its first
 // threads also do what must lie between the kernels before and behind it: of a
-// whole rebuild, reset the bounds; of an edit (cells given), bring the pool's
-// counters back into their range where allocations overran it.
+// whole rebuild, reset the bounds and clear the word before the block masks; of an
+// edit (cells given), bring the pool's counters back into their range where
+// allocations overran it.
 __global__ void macro_kernel(const uint32_t* ptr, int bx, int by, uint8_t* macro, uint64_t* mask, int32_t* bounds,
-                             int32_t* alloc, uint32_t capacity, const uint32_t* cells, uint64_t n) {
+                             uint64_t* sub, int32_t* alloc, uint32_t capacity, const uint32_t* cells, uint64_t n) {
   const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (blockIdx.x == 0) {
     if (!cells) {
       if (threadIdx.x < 8) bounds[threadIdx.x] = INT32_MIN / 2;  // nothing occupied
+      if (threadIdx.x == 8) sub[-1] = 0;
     } else if (threadIdx.x == 0) {
       if (alloc[1] < 0) alloc[1] = 0;
       if ((uint32_t)alloc[0] > capacity) alloc[0] = (int32_t)capacity;
@@ -805,11 +807,11 @@ meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint6
   }
   if (e == cudaSuccess) e = take(&s->d_occ, nslot * 64);
   if (e == cudaSuccess) e = take(&s->d_mat, nslot * 1024);
-  if (e == cudaSuccess) e = take(&small, nslot * 12 + 16);
+  if (e == cudaSuccess) e = take(&small, 8 + nslot * 12 + 16);
   if (e == cudaSuccess) {
-    s->d_sub = reinterpret_cast<uint64_t*>(small);
-    s->d_alloc = reinterpret_cast<int64_t*>(small + nslot * 8);
-    s->d_free = reinterpret_cast<uint32_t*>(small + nslot * 8 + 16);
+    s->d_sub = reinterpret_cast<uint64_t*>(small) + 1;
+    s->d_alloc = reinterpret_cast<int64_t*>(s->d_sub + nslot);
+    s->d_free = reinterpret_cast<uint32_t*>(s->d_alloc + 2);
   }
   scene_pool_account(ctx, (int64_t)s->pool_bytes);
   if (e != cudaSuccess) {
@@ -830,7 +832,7 @@ void scene_release(meso_ctx* ctx, meso_scene* s) {
   cudaFreeAsync(s->d_bounds, ctx->stream);  // the base of the cell maps
   cudaFreeAsync(s->d_occ, ctx->stream);
   cudaFreeAsync(s->d_mat, ctx->stream);
-  cudaFreeAsync(s->d_sub, ctx->stream);  // the base of the pool's small arrays
+  if (s->d_sub) cudaFreeAsync(s->d_sub - 1, ctx->stream);  // the base of the pool's small arrays
   scene_pool_account(ctx, -(int64_t)s->pool_bytes);
   if (s->bytes) ctx->scene_bytes.fetch_sub(s->bytes);
   delete s;
@@ -841,7 +843,7 @@ meso_status rebuild_macro(meso_ctx* ctx, meso_scene* s, const uint32_t* d_cells,
   const uint64_t cells = d_cells ? n : n_macro_of(s), cells3 = d_cells3 ? n3 : n_macro3_of(s);
   if (cells == 0) return MESO_OK;
   macro_kernel<<<(unsigned)((cells * 32 + 255) / 256), 256, 0, st>>>(s->d_ptr, s->bx, s->by, s->d_macro, s->d_mask, s->d_bounds,
-                                                                     reinterpret_cast<int32_t*>(s->d_alloc),
+                                                                     s->d_sub, reinterpret_cast<int32_t*>(s->d_alloc),
                                                                      (uint32_t)s->capacity, d_cells, cells);
   level_kernel<<<(unsigned)(cells3 * 32), kLevelThreads, 0, st>>>(s->d_mask, s->d_macro, s->bx, s->by, s->bz, s->d_level,
                                                                   s->d_bounds, d_cells3);
