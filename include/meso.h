@@ -73,7 +73,10 @@ typedef struct meso_scene meso_scene;
  * binds a device instead of spawning a host ThreadPool (Runtimes/Thread/ThreadPool.h:25-43).
  * Per-call temporaries come from the device's default stream-ordered memory
  * pool; this raises that pool's release threshold (a per-process attribute)
- * to at least 1 GiB so freed blocks are reused rather than remapped. */
+ * to at least 1 GiB so freed blocks are reused rather than remapped.  Scenes
+ * come from a pool of the context's own, which keeps up to 1 GiB of destroyed
+ * scenes' memory for the next ones until the context goes; no budget counts
+ * it. */
 meso_status meso_ctx_create(const meso_config* cfg, meso_ctx** out);
 void meso_ctx_destroy(meso_ctx* ctx);
 const char* meso_last_error_string(void);
@@ -165,6 +168,8 @@ meso_status meso_scene_create_grid(meso_ctx* ctx, int32_t kind, const void* d_gr
  * reporting occupancy (no counterpart in the reference).  Waits for the
  * context's stream. */
 meso_status meso_scene_count_solid(meso_ctx* ctx, const meso_scene* scene, uint64_t* n_solid);
+/* Waits for the device.  Of the memory that destroyed scenes held, all but
+ * 1 GiB is the device's again when the call returns. */
 meso_status meso_scene_destroy(meso_ctx* ctx, meso_scene* scene);
 meso_status meso_scene_get_info(meso_ctx* ctx, const meso_scene* scene, meso_scene_info* info);
 /* Copies the scene to the host: ptr has (nx/8)(ny/8)(nz/8) entries; occ and

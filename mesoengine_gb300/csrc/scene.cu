@@ -755,13 +755,14 @@ __global__ void sub_kernel(const uint64_t* occ, uint64_t slots, uint64_t* sub) {
 
 // Keeps the scene pool's release threshold at the live scenes' bytes plus
 // kScenePoolKeep: what is free beyond that goes back to the device at the next
-// synchronisation.
-static void scene_pool_account(meso_ctx* ctx, int64_t delta) {
+// synchronisation.  Returns the threshold.
+static uint64_t scene_pool_account(meso_ctx* ctx, int64_t delta) {
   constexpr uint64_t kScenePoolKeep = 1ull << 30;
   std::lock_guard<std::mutex> lk(ctx->scene_pool_mu);
   ctx->scene_pool_live += (uint64_t)delta;
   uint64_t keep = ctx->scene_pool_live + kScenePoolKeep;
   cudaMemPoolSetAttribute(ctx->scene_pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  return keep;
 }
 
 meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint64_t capacity, meso_scene** out) {
@@ -833,7 +834,14 @@ void scene_release(meso_ctx* ctx, meso_scene* s) {
   cudaFreeAsync(s->d_occ, ctx->stream);
   cudaFreeAsync(s->d_mat, ctx->stream);
   if (s->d_sub) cudaFreeAsync(s->d_sub - 1, ctx->stream);  // the base of the pool's small arrays
-  scene_pool_account(ctx, -(int64_t)s->pool_bytes);
+  const uint64_t keep = scene_pool_account(ctx, -(int64_t)s->pool_bytes);
+  // what the pool then holds beyond the threshold goes back now, not at some
+  // later synchronisation: the caller's next allocation may need it
+  uint64_t held = 0;
+  if (cudaMemPoolGetAttribute(ctx->scene_pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess && held > keep) {
+    cudaStreamSynchronize(ctx->stream);
+    cudaMemPoolTrimTo(ctx->scene_pool, keep);
+  }
   if (s->bytes) ctx->scene_bytes.fetch_sub(s->bytes);
   delete s;
 }

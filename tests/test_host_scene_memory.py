@@ -1,0 +1,66 @@
+"""What scenes take of the device's memory and when they give it back, on a CUDA runtime of host memory."""
+import ctypes
+
+import pytest
+
+import host_runtime
+
+KEPT = 1 << 30  # of freed scenes' memory, by a context
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    return host_runtime.load(tmp_path_factory.mktemp("host"))
+
+
+@pytest.fixture
+def path(tmp_path):
+    return host_runtime.scene_file(tmp_path / "s", (64, 32, 96), 90)
+
+
+def load(lib, ctx, path, spare):
+    scene = ctypes.c_void_p()
+    rc = lib.meso_scene_load(ctx, path, spare, ctypes.byref(scene))
+    return rc, scene
+
+
+@pytest.mark.parametrize("spare", [0, 900_000, 1_100_000, 3_000_000])  # up to and beyond what is kept
+def test_a_destroyed_scene_is_given_back(lib, path, spare):
+    ctx = host_runtime.context(lib)
+    before = lib.fake_taken()
+    rc, first = load(lib, ctx, path, spare)
+    rc2, second = load(lib, ctx, path, spare // 2)
+    assert rc == rc2 == 0 and lib.fake_taken() - before > 1500 * spare
+    lib.meso_scene_destroy(ctx, first)
+    assert lib.fake_taken() - before <= 1200 * (spare // 2) + (1 << 20) + KEPT
+    lib.meso_scene_destroy(ctx, second)
+    assert lib.fake_taken() - before <= KEPT
+    lib.meso_ctx_destroy(ctx)
+
+
+def test_small_scenes_follow_one_another_without_a_wait(lib, path):
+    # a scene made in place of another finds the memory of the last one
+    ctx = host_runtime.context(lib)
+    rc, scene = load(lib, ctx, path, 100_000)
+    held = lib.fake_taken()
+    lib.fake_clear_log()
+    lib.meso_scene_destroy(ctx, scene)
+    calls = host_runtime.log(lib)
+    last = max(i for i, c in enumerate(calls) if c[0] == "free")
+    assert lib.fake_taken() == held and not [c for c in calls[last:] if c[0].startswith("wait")]
+    rc, scene = load(lib, ctx, path, 100_000)
+    assert rc == 0 and lib.fake_taken() == held
+    lib.meso_scene_destroy(ctx, scene)
+    lib.meso_ctx_destroy(ctx)
+
+
+def test_a_scene_that_does_not_fit_is_given_back(lib, path):
+    # the occupancy of 30 M slots (1.9 GB) fits, the materials do not
+    ctx = host_runtime.context(lib)
+    before = lib.fake_taken()
+    lib.fake_limit(before + (8 << 30))
+    rc, scene = load(lib, ctx, path, 30_000_000)
+    lib.fake_limit(0)
+    assert rc == 2 and not scene.value
+    assert lib.fake_taken() - before <= KEPT
+    lib.meso_ctx_destroy(ctx)
