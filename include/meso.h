@@ -140,7 +140,7 @@ typedef struct meso_scene_info {
   int32_t nx, ny, nz;
   uint64_t n_bricks;        /* live bricks */
   uint64_t brick_capacity;  /* pool slots */
-  uint64_t device_bytes;    /* pointer grid + pools */
+  uint64_t device_bytes;    /* all the scene takes (pointer grid, pools, maps derived from them), as budgets count it */
   const uint32_t* d_ptr;    /* (nx/8)(ny/8)(nz/8) brick pointers */
   const uint64_t* d_occ;    /* 8 words per brick slot, word z, bit x+8y */
   const uint16_t* d_mat;    /* 512 materials per brick slot, x+8y+64z */

@@ -83,8 +83,8 @@ struct meso_scene {
   // cell is occupied; lets a ray cross an empty cell in one jump
   uint8_t* d_macro = nullptr;
   // Derived maps of the raymarch's region walk (a byte per brick, 8 per
-  // 4x4x4-brick cell and 8 per pool slot, a few percent of the scene at most;
-  // not part of `bytes`, so that a budget admits what it did without them):
+  // 4x4x4-brick cell and 8 per pool slot: 1 % of a scene that is mostly bricks,
+  // 28 % of an empty one, which is little but its pointer grid):
   uint8_t* d_level = nullptr;  // per brick: 0 if occupied, else log2 of the edge in voxels of the largest
                                // aligned empty cube it is part of (3 .. 9)
   int32_t* d_bounds = nullptr; // of the occupied 4x4x4-brick cells, in voxels: [0..2] the largest -lowest, [4..6] the
@@ -96,7 +96,7 @@ struct meso_scene {
   // allocator state (device): [0] bump (slots ever used), [1] free-stack top
   int64_t* d_alloc = nullptr;
   uint32_t* d_free = nullptr;  // free stack, capacity entries
-  uint64_t bytes = 0;
+  uint64_t bytes = 0;       // all of the above, once admitted to the budget
   uint64_t pool_bytes = 0;  // taken from the context's scene pool
   uint64_t live_bricks_host = 0;  // as of the last build/edit sync
 };
@@ -107,9 +107,6 @@ inline uint64_t n_bricks_of(const meso_scene* s) {
   return (uint64_t)s->bx * (uint64_t)s->by * (uint64_t)s->bz;
 }
 inline uint64_t n_macro_of(const meso_scene* s) { return n_bricks_of(s) / 64; }
-inline uint64_t n_macro2_of(const meso_scene* s) {
-  return (uint64_t)((s->bx + 15) / 16) * (uint64_t)((s->by + 15) / 16) * (uint64_t)((s->bz + 15) / 16);
-}
 inline uint64_t n_macro3_of(const meso_scene* s) {
   return (uint64_t)((s->bx + 63) / 64) * (uint64_t)((s->by + 63) / 64) * (uint64_t)((s->bz + 63) / 64);
 }

@@ -774,10 +774,10 @@ meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint6
   s->by = ny / 8;
   s->bz = nz / 8;
   s->capacity = capacity;
-  const uint64_t nb = n_bricks_of(s);
-  // (a byte for each cell of 4^3, 16^3 and 64^3 bricks is counted, whatever the
-  // maps derived from the pointers take)
-  const uint64_t bytes = nb * 4 + nb / 64 + n_macro2_of(s) + n_macro3_of(s) + capacity * (64 + 1024 + 4) + 16;
+  const uint64_t nb = n_bricks_of(s), nm = std::max<uint64_t>(n_macro_of(s), 1), nslot = std::max<uint64_t>(capacity, 1);
+  const uint64_t ptr_bytes = nb * 4, map_bytes = 32 + nm * (8 + 64 + 1), occ_bytes = nslot * 64, mat_bytes = nslot * 1024,
+                 small_bytes = 8 + nslot * 12 + 16;
+  const uint64_t bytes = ptr_bytes + map_bytes + occ_bytes + mat_bytes + small_bytes;
   if (ctx->budget_bytes && ctx->scene_bytes.load() + bytes > ctx->budget_bytes) {
     delete s;
     return fail(MESO_ERR_OVER_BUDGET, "scene exceeds the HBM budget");
@@ -795,20 +795,19 @@ meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint6
     if (err == cudaSuccess) s->pool_bytes += n;
     return err;
   };
-  const uint64_t nm = std::max<uint64_t>(n_macro_of(s), 1), nslot = std::max<uint64_t>(capacity, 1);
   uint8_t* maps = nullptr;
   uint8_t* small = nullptr;
-  cudaError_t e = take(&s->d_ptr, nb * 4);
-  if (e == cudaSuccess) e = take(&maps, 32 + nm * (8 + 64 + 1));
+  cudaError_t e = take(&s->d_ptr, ptr_bytes);
+  if (e == cudaSuccess) e = take(&maps, map_bytes);
   if (e == cudaSuccess) {
     s->d_bounds = reinterpret_cast<int32_t*>(maps);  // all written whole by rebuild_macro
     s->d_mask = reinterpret_cast<uint64_t*>(maps + 32);
     s->d_level = maps + 32 + nm * 8;
     s->d_macro = s->d_level + nm * 64;
   }
-  if (e == cudaSuccess) e = take(&s->d_occ, nslot * 64);
-  if (e == cudaSuccess) e = take(&s->d_mat, nslot * 1024);
-  if (e == cudaSuccess) e = take(&small, 8 + nslot * 12 + 16);
+  if (e == cudaSuccess) e = take(&s->d_occ, occ_bytes);
+  if (e == cudaSuccess) e = take(&s->d_mat, mat_bytes);
+  if (e == cudaSuccess) e = take(&small, small_bytes);
   if (e == cudaSuccess) {
     s->d_sub = reinterpret_cast<uint64_t*>(small) + 1;
     s->d_alloc = reinterpret_cast<int64_t*>(s->d_sub + nslot);

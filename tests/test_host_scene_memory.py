@@ -3,6 +3,7 @@ import ctypes
 
 import pytest
 
+import mesoengine_gb300 as meso
 import host_runtime
 
 KEPT = 1 << 30  # of freed scenes' memory, by a context
@@ -36,6 +37,35 @@ def test_a_destroyed_scene_is_given_back(lib, path, spare):
     lib.meso_scene_destroy(ctx, second)
     assert lib.fake_taken() - before <= KEPT
     lib.meso_ctx_destroy(ctx)
+
+
+@pytest.mark.parametrize("dims,n,spare", [((32, 32, 32), 0, 0), ((64, 32, 96), 90, 0), ((64, 32, 96), 90, 5000),
+                                          ((512, 256, 1024), 0, 0)])  # nothing but a pointer grid and its maps
+def test_budgets_count_what_a_scene_takes(lib, tmp_path, dims, n, spare):
+    path = host_runtime.scene_file(tmp_path / "s", dims, n)
+    ctx = host_runtime.context(lib)
+    before = lib.fake_live_bytes()
+    rc, scene = load(lib, ctx, path, spare)
+    info = meso.SceneInfo()
+    assert rc == 0 and lib.meso_scene_get_info(ctx, scene, ctypes.byref(info)) == 0
+    takes = lib.fake_live_bytes() - before
+    assert info.device_bytes == takes
+    lib.meso_scene_destroy(ctx, scene)
+    lib.meso_ctx_destroy(ctx)
+    for budget, status in ((takes - 1, 3), (takes, 0), (2 * takes - 1, 0), (2 * takes, 0)):
+        ctx = host_runtime.context(lib, budget)
+        rc, first = load(lib, ctx, path, spare)
+        assert rc == status
+        if rc == 0:
+            rc, second = load(lib, ctx, path, spare)
+            assert rc == (0 if budget == 2 * takes else 3)
+            lib.meso_scene_destroy(ctx, first)
+            if rc == 0:
+                lib.meso_scene_destroy(ctx, second)
+            rc, first = load(lib, ctx, path, spare)  # what was charged is given back
+            assert rc == 0
+            lib.meso_scene_destroy(ctx, first)
+        lib.meso_ctx_destroy(ctx)
 
 
 def test_small_scenes_follow_one_another_without_a_wait(lib, path):
