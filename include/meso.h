@@ -75,8 +75,8 @@ typedef struct meso_scene meso_scene;
  * pool; this raises that pool's release threshold (a per-process attribute)
  * to at least 1 GiB so freed blocks are reused rather than remapped.  Scenes
  * come from a pool of the context's own, which keeps up to 1 GiB of destroyed
- * scenes' memory for the next ones until the context goes; no budget counts
- * it. */
+ * scenes' memory for the next ones until the context goes or one of its own
+ * allocations would fail without it; no budget counts it. */
 meso_status meso_ctx_create(const meso_config* cfg, meso_ctx** out);
 void meso_ctx_destroy(meso_ctx* ctx);
 const char* meso_last_error_string(void);

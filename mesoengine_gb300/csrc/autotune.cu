@@ -99,7 +99,7 @@ meso_status autotune_search(meso_ctx* ctx, Tuning& best, float& best_ray, float&
   const float o[3] = {-150.0f, -100.0f, 400.0f}, tg[3] = {256.0f, 256.0f, 256.0f};
   const meso_camera cam = look_at(o, tg, 1280, 720);
   const float light[3] = {0.30304575f, 0.50507629f, 0.80812204f};  // normalize(0.3, 0.5, 0.8)
-  MESO_CUDA_TRY(cudaMalloc(&S.d_hits, sizeof(meso_hit) * 1280 * 720));
+  MESO_CUDA_TRY(dev_malloc(ctx, &S.d_hits, sizeof(meso_hit) * 1280 * 720));
   const meso_scene* sc = S.scene;
   best_ray = 1e30f;
   const uint32_t tws[4] = {4, 8, 16, 32}, wpcs[3] = {1, 2, 4};  // the kernel allows at most 128 threads per CTA
@@ -123,9 +123,9 @@ meso_status autotune_search(meso_ctx* ctx, Tuning& best, float& best_ray, float&
   // CTAs per SM x 64 is the bricks in flight per SM
   const uint32_t n = 1024;
   const uint64_t cap = (uint64_t)n * 16384;
-  MESO_CUDA_TRY(cudaMalloc(&S.d_chunks, (size_t)n * 65536));
-  MESO_CUDA_TRY(cudaMalloc(&S.d_quads, cap * 8));
-  MESO_CUDA_TRY(cudaMalloc(&S.d_count, 8));
+  MESO_CUDA_TRY(dev_malloc(ctx, &S.d_chunks, (size_t)n * 65536));
+  MESO_CUDA_TRY(dev_malloc(ctx, &S.d_quads, cap * 8));
+  MESO_CUDA_TRY(dev_malloc(ctx, &S.d_count, 8));
   MESO_TRY(generate_chunks_u16(ctx, n, 1, S.d_chunks, nullptr, st));
   meso_mesh_source src;
   memset(&src, 0, sizeof(src));

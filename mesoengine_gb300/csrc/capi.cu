@@ -223,7 +223,7 @@ meso_status meso_measure_l2_read(meso_ctx* ctx, uint64_t bytes, uint32_t passes,
   *gb_s = 0.0;
   const cudaStream_t st = ctx->stream;
   uint4* buf = nullptr;
-  MESO_CUDA_TRY(cudaMallocAsync(&buf, bytes, st));
+  MESO_CUDA_TRY(dev_malloc_async(ctx, &buf, bytes, st));
   cudaEvent_t a = nullptr, b = nullptr;
   cudaError_t e = cudaMemsetAsync(buf, 0x5A, bytes, st);
   if (e == cudaSuccess) e = cudaEventCreate(&a);
@@ -269,7 +269,7 @@ int meso_sm_count(const meso_ctx* ctx) { return ctx ? ctx->sm_count : 0; }
 
 meso_status meso_dev_alloc(meso_ctx* ctx, size_t bytes, void** d_ptr) {
   if (!ctx || !d_ptr) return fail(MESO_ERR_INVALID_ARG, "dev_alloc: null argument");
-  MESO_CUDA_TRY(cudaMalloc(d_ptr, bytes ? bytes : 16));
+  MESO_CUDA_TRY(dev_malloc(ctx, d_ptr, bytes ? bytes : 16));
   return MESO_OK;
 }
 meso_status meso_dev_free(meso_ctx* ctx, void* d_ptr) {
@@ -481,7 +481,7 @@ meso_status mesh_host_pipelined(meso_ctx* ctx, int32_t kind, const uint8_t* h_da
   // [0, 2 slices) inputs, then the count, then the quads unless written to host memory
   const size_t off_count = 2 * slice_bytes, off_quads = off_count + 256;
   const size_t total = off_quads + (d_direct ? 0 : capacity * 8);
-  if (e == cudaSuccess) e = cudaMallocAsync(&d, total, st);
+  if (e == cudaSuccess) e = dev_malloc_async(ctx, &d, total, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(d + off_count, 0, 8, st);
   if (e == cudaSuccess) e = cudaEventRecord(ready, st);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(cs, ready, 0);  // the buffers exist before the first copy
@@ -575,7 +575,7 @@ meso_status meso_mesh_host(meso_ctx* ctx, int32_t kind, const void* h_data, int3
   const size_t off_count = (off_coords + coord_bytes + 255) & ~size_t(255);
   const size_t off_quads = off_count + 256;
   const size_t total = off_quads + capacity * 8;
-  MESO_CUDA_TRY(cudaMallocAsync(&d, total, st));
+  MESO_CUDA_TRY(dev_malloc_async(ctx, &d, total, st));
   meso_status rc = MESO_OK;
   cudaError_t e = cudaMemcpyAsync(d, h_data, data_bytes, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && coord_bytes) e = cudaMemcpyAsync(d + off_coords, h_coords, coord_bytes, cudaMemcpyHostToDevice, st);
@@ -623,7 +623,7 @@ meso_status meso_raymarch(meso_ctx* ctx, const meso_scene* const* scenes, const 
   if (n_views <= 32) return launch_raymarch(ctx, scenes, cams, n_views, light, flags, d_hits, st, nullptr, 0);
   const size_t tb = raymarch_view_table_bytes(n_views);
   void* d_table = nullptr;
-  MESO_CUDA_TRY(cudaMallocAsync(&d_table, tb, st));
+  MESO_CUDA_TRY(dev_malloc_async(ctx, &d_table, tb, st));
   meso_status rc = launch_raymarch(ctx, scenes, cams, n_views, light, flags, d_hits, st, d_table, tb);
   cudaFreeAsync(d_table, st);
   return rc;
@@ -662,7 +662,7 @@ meso_status meso_raymarch_host(meso_ctx* ctx, const meso_scene* scene, const mes
     return rc;
   }
   meso_hit* d = nullptr;
-  MESO_CUDA_TRY(cudaMallocAsync(&d, n * sizeof(meso_hit), st));
+  MESO_CUDA_TRY(dev_malloc_async(ctx, &d, n * sizeof(meso_hit), st));
   meso_status rc = launch_raymarch(ctx, &scene, cam, 1, light, flags, d, st, nullptr, 0);
   if (rc == MESO_OK) {
     cudaError_t e = cudaMemcpyAsync(h_hits, d, n * sizeof(meso_hit), cudaMemcpyDeviceToHost, st);
@@ -680,7 +680,7 @@ meso_status meso_raymarch_stats(meso_ctx* ctx, const meso_scene* const* scenes, 
   if (n_views > 32) return fail(MESO_ERR_INVALID_ARG, "raymarch_stats: at most 32 views");
   cudaStream_t st = ctx->stream;
   uint64_t* d = nullptr;
-  MESO_CUDA_TRY(cudaMallocAsync(&d, 32, st));
+  MESO_CUDA_TRY(dev_malloc_async(ctx, &d, 32, st));
   MESO_CUDA_TRY(cudaMemsetAsync(d, 0, 32, st));
   meso_status rc = launch_raymarch(ctx, scenes, cams, n_views, light, flags, d_hits, st, nullptr, 0, d);
   if (rc == MESO_OK) {

@@ -122,6 +122,26 @@ inline cudaStream_t pick_stream(meso_ctx* ctx, void* s) {
 meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint64_t capacity,
                         meso_scene** out);
 void scene_release(meso_ctx* ctx, meso_scene* s);
+
+// Gives back to the device what the context's scene pool keeps of destroyed
+// scenes.  False if that is nothing.
+bool scene_pool_give_back(meso_ctx* ctx);
+
+// cudaMalloc and cudaMallocAsync that give back what the scene pool keeps before
+// they fail: neither call does so by itself.
+template <typename T>
+inline cudaError_t dev_malloc(meso_ctx* ctx, T** p, uint64_t bytes) {
+  const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), bytes);
+  if (e != cudaErrorMemoryAllocation || !scene_pool_give_back(ctx)) return e;
+  return cudaMalloc(reinterpret_cast<void**>(p), bytes);
+}
+template <typename T>
+inline cudaError_t dev_malloc_async(meso_ctx* ctx, T** p, uint64_t bytes, cudaStream_t st) {
+  const cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(p), bytes, st);
+  if (e != cudaErrorMemoryAllocation || !scene_pool_give_back(ctx)) return e;
+  return cudaMallocAsync(reinterpret_cast<void**>(p), bytes, st);
+}
+
 // Recomputes the cell maps (occupancy bytes, brick masks, level bytes,
 // bounds): all of them (lists null), or of the listed cells of 4^3 and 64^3
 // bricks (each list unique) after an edit, whose pool counters it also clamps.

@@ -215,7 +215,7 @@ meso_status number_bricks(meso_ctx* ctx, const uint8_t* d_flags, uint64_t nb, ui
   const uint64_t tiles = (nb + kScanTile - 1) / kScanTile;
   if (tiles > 0xFFFFFFFFull) return fail(MESO_ERR_INVALID_ARG, "scene too large");
   uint32_t* d_sums = nullptr;
-  MESO_CUDA_TRY(cudaMallocAsync(&d_sums, sizeof(uint32_t) * (tiles + 1), st));
+  MESO_CUDA_TRY(dev_malloc_async(ctx, &d_sums, sizeof(uint32_t) * (tiles + 1), st));
   scan_tiles_kernel<<<(unsigned)tiles, kScanThreads, 0, st>>>(d_flags, nb, d_ptr, d_sums);
   scan_sums_kernel<<<1, kScanThreads, 0, st>>>(d_sums, (uint32_t)tiles, d_sums + tiles);
   scan_finish_kernel<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(d_flags, nb, d_sums, d_ptr);
@@ -765,6 +765,16 @@ static uint64_t scene_pool_account(meso_ctx* ctx, int64_t delta) {
   return keep;
 }
 
+bool scene_pool_give_back(meso_ctx* ctx) {
+  uint64_t used = 0, held = 0;
+  if (cudaMemPoolGetAttribute(ctx->scene_pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess ||
+      cudaMemPoolGetAttribute(ctx->scene_pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess || held <= used)
+    return false;
+  cudaGetLastError();  // of the allocation that is tried again
+  cudaStreamSynchronize(ctx->stream);
+  return cudaMemPoolTrimTo(ctx->scene_pool, 0) == cudaSuccess;
+}
+
 meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint64_t capacity, meso_scene** out) {
   meso_scene* s = new meso_scene();
   s->nx = nx;
@@ -791,7 +801,9 @@ meso_status scene_alloc(meso_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, uint6
   // against what that keeps of the per-call temporaries.
   const cudaStream_t st = ctx->stream;
   auto take = [&](auto** p, uint64_t n) {
-    const cudaError_t err = cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), n, ctx->scene_pool, st);
+    cudaError_t err = cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), n, ctx->scene_pool, st);
+    if (err == cudaErrorMemoryAllocation && scene_pool_give_back(ctx))
+      err = cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), n, ctx->scene_pool, st);
     if (err == cudaSuccess) s->pool_bytes += n;
     return err;
   };
@@ -902,10 +914,10 @@ meso_status scene_create_terrain(meso_ctx* ctx, const meso_terrain* t, uint64_t 
   float* d_hmax = nullptr;
   uint8_t* d_flags = nullptr;
   uint32_t* d_ptr_tmp = nullptr;
-  cudaError_t ae = cudaMallocAsync(&d_h, ncol * 4, st);
-  if (ae == cudaSuccess) ae = cudaMallocAsync(&d_hmax, (uint64_t)bx * by * 4, st);
-  if (ae == cudaSuccess) ae = cudaMallocAsync(&d_flags, nb, st);
-  if (ae == cudaSuccess) ae = cudaMallocAsync(&d_ptr_tmp, nb * 4, st);
+  cudaError_t ae = dev_malloc_async(ctx, &d_h, ncol * 4, st);
+  if (ae == cudaSuccess) ae = dev_malloc_async(ctx, &d_hmax, (uint64_t)bx * by * 4, st);
+  if (ae == cudaSuccess) ae = dev_malloc_async(ctx, &d_flags, nb, st);
+  if (ae == cudaSuccess) ae = dev_malloc_async(ctx, &d_ptr_tmp, nb * 4, st);
   if (ae != cudaSuccess) {
     cudaFreeAsync(d_h, st);  // cudaFreeAsync(nullptr) is a no-op
     cudaFreeAsync(d_hmax, st);
@@ -950,7 +962,7 @@ static meso_status build_from_device_grid(meso_ctx* ctx, const T* d_grid, int32_
   const uint64_t nb = (uint64_t)nx * ny * nz / 512;
   const unsigned blocks = (unsigned)((nb + kDenseBricks - 1) / kDenseBricks);
   uint32_t* d_occupied = nullptr;  // a word per block: which of its bricks hold anything; then their first slots, and the count
-  const cudaError_t ae = cudaMallocAsync(&d_occupied, 8 * (size_t)blocks + 4, st);
+  const cudaError_t ae = dev_malloc_async(ctx, &d_occupied, 8 * (size_t)blocks + 4, st);
   if (ae != cudaSuccess) {
     cudaStreamSynchronize(st);
     return cuda_fail(ae, "dense scene: scratch allocation");
@@ -1001,7 +1013,7 @@ meso_status scene_create_dense(meso_ctx* ctx, const uint16_t* h_grid, int32_t nx
   cudaStream_t st = ctx->stream;
   const uint64_t nvox = (uint64_t)nx * ny * nz;
   uint16_t* d_grid = nullptr;
-  cudaError_t ae = cudaMallocAsync(&d_grid, nvox * 2, st);
+  cudaError_t ae = dev_malloc_async(ctx, &d_grid, nvox * 2, st);
   if (ae == cudaSuccess) ae = cudaMemcpyAsync(d_grid, h_grid, nvox * 2, cudaMemcpyHostToDevice, st);
   if (ae != cudaSuccess) {
     cudaFreeAsync(d_grid, st);
@@ -1031,7 +1043,7 @@ meso_status scene_count_solid(meso_ctx* ctx, const meso_scene* s, uint64_t* n_so
   if (!s || !n_solid) return fail(MESO_ERR_INVALID_ARG, "scene_count_solid: null argument");
   cudaStream_t st = ctx->stream;
   unsigned long long* d = nullptr;
-  MESO_CUDA_TRY(cudaMallocAsync(&d, 8, st));
+  MESO_CUDA_TRY(dev_malloc_async(ctx, &d, 8, st));
   cudaError_t e = cudaMemsetAsync(d, 0, 8, st);
   const uint64_t nb = n_bricks_of(s);
   if (e == cudaSuccess) {
@@ -1089,7 +1101,7 @@ meso_status generate_chunks_u16(meso_ctx* ctx, uint32_t n, uint32_t seed0, uint1
   std::vector<uint32_t> targets(n);
   for (uint32_t i = 0; i < n; i++) targets[i] = chunk_solid_target(seed0 + i);
   uint32_t* d_t = nullptr;
-  MESO_CUDA_TRY(cudaMallocAsync(&d_t, 4ull * n, st));
+  MESO_CUDA_TRY(dev_malloc_async(ctx, &d_t, 4ull * n, st));
   MESO_CUDA_TRY(cudaMemcpyAsync(d_t, targets.data(), 4ull * n, cudaMemcpyHostToDevice, st));
   static bool attr = false;
   if (!attr) {
@@ -1219,7 +1231,7 @@ meso_status edit_spheres(meso_ctx* ctx, meso_scene* s, const meso_sphere_edit* h
   }
   const size_t bytes = up16 + nb * 1024 + nb + 16;
   uint8_t* d = nullptr;
-  MESO_CUDA_TRY(cudaMallocAsync(&d, bytes, st));
+  MESO_CUDA_TRY(dev_malloc_async(ctx, &d, bytes, st));
   meso_sphere_edit* d_sp = reinterpret_cast<meso_sphere_edit*>(d);
   uint32_t* d_b = reinterpret_cast<uint32_t*>(d + n * sizeof(meso_sphere_edit));
   uint32_t* d_cells = d_b + nb;

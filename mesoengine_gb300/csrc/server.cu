@@ -516,21 +516,21 @@ meso_status meso_server_create(meso_ctx* ctx, const meso_server_config* cfg, mes
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.forked, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.joined, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaMalloc(&s.d_hits, srv->cfg.max_batch_rays * sizeof(meso_hit));
+    if (e == cudaSuccess) e = dev_malloc(ctx, &s.d_hits, srv->cfg.max_batch_rays * sizeof(meso_hit));
     s.hit_cap = srv->cfg.max_batch_rays;
     s.table_bytes = raymarch_view_table_bytes(kMaxBatch);
-    if (e == cudaSuccess) e = cudaMalloc(&s.d_table, s.table_bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&s.d_sums, sizeof(unsigned long long) * kSums);
+    if (e == cudaSuccess) e = dev_malloc(ctx, &s.d_table, s.table_bytes);
+    if (e == cudaSuccess) e = dev_malloc(ctx, &s.d_sums, sizeof(unsigned long long) * kSums);
     if (e == cudaSuccess) e = cudaMallocHost(&s.h_sums, sizeof(unsigned long long) * kSums);
     s.quad_cap = srv->cfg.max_edit_quads;
-    if (e == cudaSuccess) e = cudaMalloc(&s.d_quads, s.quad_cap * 8);
+    if (e == cudaSuccess) e = dev_malloc(ctx, &s.d_quads, s.quad_cap * 8);
     s.coord_cap = coord_cap;
-    if (e == cudaSuccess) e = cudaMalloc(&s.d_coords, 12ull * std::max<uint32_t>(coord_cap, 1));
+    if (e == cudaSuccess) e = dev_malloc(ctx, &s.d_coords, 12ull * std::max<uint32_t>(coord_cap, 1));
     if (e == cudaSuccess) e = cudaMallocHost(&s.h_coords, 12ull * std::max<uint32_t>(coord_cap, 1));
     if (e == cudaSuccess && srv->cfg.keep_hits) e = cudaMallocHost(&s.h_hits, srv->cfg.max_batch_rays * sizeof(meso_hit));
     if (e == cudaSuccess && srv->cfg.keep_meshes) {
-      e = cudaMalloc(&s.d_counts, 4ull * std::max<uint32_t>(coord_cap, 1));
-      if (e == cudaSuccess) e = cudaMalloc(&s.d_place, 12ull * std::max<uint32_t>(coord_cap, 1));
+      e = dev_malloc(ctx, &s.d_counts, 4ull * std::max<uint32_t>(coord_cap, 1));
+      if (e == cudaSuccess) e = dev_malloc(ctx, &s.d_place, 12ull * std::max<uint32_t>(coord_cap, 1));
       if (e == cudaSuccess) e = cudaMallocHost(&s.h_flags, sizeof(unsigned long long));
       if (e == cudaSuccess) *s.h_flags = 0;
     }

@@ -232,8 +232,8 @@ static meso_status compact(meso_ctx* ctx, meso_mesh_store* S, uint64_t min_cap, 
   const uint64_t cap = std::max<uint64_t>({min_cap, top + top / 2 + 4096, S->arena_cap});
   uint64_t* na = nullptr;
   uint64_t* d_noff = nullptr;
-  MESO_CUDA_TRY(cudaMallocAsync(&na, cap * 8, st));
-  cudaError_t e = cudaMallocAsync(&d_noff, N * 8, st);
+  MESO_CUDA_TRY(dev_malloc_async(ctx, &na, cap * 8, st));
+  cudaError_t e = dev_malloc_async(ctx, &d_noff, N * 8, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_noff, noff.data(), N * 8, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) {
     compact_kernel<<<ctx->sm_count * 8, 256, 0, st>>>(S->d_arena, S->d_off, d_noff, S->d_cnt, N, na);
@@ -297,7 +297,7 @@ meso_status store_update_sync(meso_ctx* ctx, meso_mesh_store* S, const uint32_t*
       const size_t off_work = off_counts + (((size_t)4 * m + 255) & ~size_t(255));
       const size_t off_tc = off_work + (((size_t)16 * m + 8 + 255) & ~size_t(255));
       const size_t off_temp = off_tc + 256;
-      MESO_CUDA_TRY(cudaMallocAsync(&d, off_temp + temp_cap * 8, st));
+      MESO_CUDA_TRY(dev_malloc_async(ctx, &d, off_temp + temp_cap * 8, st));
       cudaError_t e = cudaMemcpyAsync(d, coords.data(), 12ull * m, cudaMemcpyHostToDevice, st);
       meso_status rc = e == cudaSuccess ? MESO_OK : cuda_fail(e, "mesh store upload");
       if (rc == MESO_OK)
@@ -361,11 +361,11 @@ meso_status meso_mesh_store_create(meso_ctx* ctx, const meso_scene* scene, meso_
   for (uint64_t c = 0; c < N; c++)
     if (macro[c]) chunks.push_back((uint32_t)c);
   S->arena_cap = std::max<uint64_t>(65536, (uint64_t)chunks.size() * 1024);
-  if (e == cudaSuccess) e = cudaMalloc(&S->d_arena, S->arena_cap * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&S->d_off, N * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&S->d_cnt, N * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&S->d_cap, N * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&S->d_state, 3 * sizeof(unsigned long long));
+  if (e == cudaSuccess) e = dev_malloc(ctx, &S->d_arena, S->arena_cap * 8);
+  if (e == cudaSuccess) e = dev_malloc(ctx, &S->d_off, N * 8);
+  if (e == cudaSuccess) e = dev_malloc(ctx, &S->d_cnt, N * 4);
+  if (e == cudaSuccess) e = dev_malloc(ctx, &S->d_cap, N * 4);
+  if (e == cudaSuccess) e = dev_malloc(ctx, &S->d_state, 3 * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMemsetAsync(S->d_off, 0xFF, N * 8, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(S->d_cnt, 0, N * 4, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(S->d_cap, 0, N * 4, st);
@@ -425,7 +425,7 @@ meso_status meso_mesh_store_gather(meso_ctx* ctx, const meso_mesh_store* store, 
   *h_total = total;
   uint8_t* d = nullptr;
   const size_t off_offs = ((size_t)4 * n + 255) & ~size_t(255);
-  MESO_CUDA_TRY(cudaMallocAsync(&d, off_offs + 8ull * n, st));
+  MESO_CUDA_TRY(dev_malloc_async(ctx, &d, off_offs + 8ull * n, st));
   cudaError_t e = cudaMemcpyAsync(d, h_chunks, 4ull * n, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d + off_offs, offs.data(), 8ull * n, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && capacity) {

@@ -94,3 +94,45 @@ def test_a_scene_that_does_not_fit_is_given_back(lib, path):
     assert rc == 2 and not scene.value
     assert lib.fake_taken() - before <= KEPT
     lib.meso_ctx_destroy(ctx)
+
+
+def full_device(lib, path):
+    """A context that keeps 0.5 GB of a destroyed scene on a device with 64 MB to spare, and a small live scene."""
+    ctx = host_runtime.context(lib)
+    _, kept = load(lib, ctx, path, 500_000)
+    _, scene = load(lib, ctx, path, 0)
+    lib.meso_scene_destroy(ctx, kept)
+    lib.fake_limit(lib.fake_taken() + (64 << 20))
+    return ctx, scene
+
+
+def dev_alloc(lib, ctx, scene, n):
+    p = ctypes.c_void_p()
+    rc = lib.meso_dev_alloc(ctx, n, ctypes.byref(p))
+    return rc, lambda: lib.meso_dev_free(ctx, p)
+
+
+def server(lib, ctx, scene, n):
+    cfg, h = meso.ServerConfig(), ctypes.c_void_p()
+    cfg.max_inflight_batches, cfg.max_batch_rays, cfg.max_edit_quads = 1, n // 24, 1024
+    rc = lib.meso_server_create(ctx, ctypes.byref(cfg), (ctypes.c_void_p * 1)(scene), 1, ctypes.byref(h))
+    return rc, lambda: lib.meso_server_destroy(h)
+
+
+def mesh(lib, ctx, scene, n):
+    # a temporary of the call: the quads of one chunk of host memory
+    chunk, total = (ctypes.c_uint16 * 32768)(), ctypes.c_uint64()
+    return lib.meso_mesh_host(ctx, 1, chunk, 1, 0, 0, None, 1, None, n // 8, ctypes.byref(total)), lambda: None
+
+
+@pytest.mark.parametrize("take", [dev_alloc, server, mesh])
+def test_kept_memory_goes_back_before_an_allocation_fails(lib, path, take):
+    ctx, scene = full_device(lib, path)
+    rc, give = take(lib, ctx, scene, 400 << 20)
+    assert rc == 0
+    give()
+    rc, _ = take(lib, ctx, scene, 900 << 20)  # more than there is
+    lib.fake_limit(0)
+    assert rc == 2
+    lib.meso_scene_destroy(ctx, scene)
+    lib.meso_ctx_destroy(ctx)
