@@ -78,6 +78,8 @@ typedef struct meso_scene meso_scene;
  * scenes' memory for the next ones until the context goes or one of its own
  * allocations would fail without it; no budget counts it. */
 meso_status meso_ctx_create(const meso_config* cfg, meso_ctx** out);
+/* Scenes, mesh stores and servers of the context are destroyed before it: what
+ * still lives keeps its device memory until the process ends. */
 void meso_ctx_destroy(meso_ctx* ctx);
 const char* meso_last_error_string(void);
 const char* meso_status_string(meso_status s);

@@ -188,7 +188,7 @@ void meso_ctx_destroy(meso_ctx* ctx) {
   cudaStreamSynchronize(ctx->stream);
   cudaFree(ctx->d_scratch);
   cudaFree(ctx->d_tickets);
-  cudaMemPoolDestroy(ctx->scene_pool);  // memory of scenes that still live goes with them
+  cudaMemPoolDestroy(ctx->scene_pool);  // (scenes that still live keep their memory)
   cudaStreamDestroy(ctx->stream);
   delete ctx;
 }
