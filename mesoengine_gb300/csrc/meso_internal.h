@@ -92,6 +92,8 @@ struct meso_scene {
   uint64_t* d_mask = nullptr;  // per 4x4x4-brick cell: its occupied bricks, bit x + 4y + 16z
   uint64_t* d_sub = nullptr;   // per pool slot: the non-empty 2x2x2-voxel blocks, bit x + 4y + 16z; one more word
                                // before them, zero, for rays that read an unlinked brick's pointer as a slot
+  bool rough = false;          // of the space that is not solid, much is between scattered voxels (as built; edits
+                               // leave it): rays walk step by step
   uint64_t capacity = 0;       // pool slots
   // allocator state (device): [0] bump (slots ever used), [1] free-stack top
   int64_t* d_alloc = nullptr;
@@ -147,7 +149,8 @@ inline cudaError_t dev_malloc_async(meso_ctx* ctx, T** p, uint64_t bytes, cudaSt
 // bricks (each list unique) after an edit, whose pool counters it also clamps.
 meso_status rebuild_macro(meso_ctx* ctx, meso_scene* s, const uint32_t* d_cells, uint32_t n, cudaStream_t st,
                           const uint32_t* d_cells3 = nullptr, uint32_t n3 = 0);
-// Recomputes d_sub of the first `slots` pool slots from their occupancy.
+// Recomputes d_sub of the first `slots` pool slots from their occupancy, and
+// `rough` (waits for st).
 meso_status rebuild_sub(meso_ctx* ctx, meso_scene* s, uint64_t slots, cudaStream_t st);
 
 // Kernel launchers (defined in the .cu files).

@@ -56,6 +56,7 @@ using namespace ::meso::dev;
 
 constexpr int kInlineViews = 32;
 constexpr int kPlain = 0, kStatsMode = 1, kHashMode = 2;
+constexpr int kByRegion = 0, kEither = 1, kBySteps = 2;  // which walk a launch's rays take (see raymarch_kernel)
 constexpr uint32_t kFullMask = 0xFFFFFFFFu;
 constexpr float kInf = __builtin_huge_valf();
 
@@ -137,8 +138,11 @@ __device__ __forceinline__ int inner_steps(int s, int B, int mask, int nb, float
 // progress (a direction of zeros or NaNs).  The statistics instantiation
 // takes this path to count its fetches, and so does any ray whose values lie
 // outside what the region walk below was proven for.  kCubes: an empty cube of
-// bricks is crossed in one step.
-template <bool kStats, bool kCubes>
+// bricks is crossed in one step.  kKeep: the boundary times and the occupancy word
+// are kept from voxel to voxel, as only a stepped axis has another time and only a
+// step along z another word (256^3 random voxels, 10 % solid, 1280x720: 79.6 us
+// without, 69.3 so); where the walk is out of line it has no registers for them.
+template <bool kStats, bool kCubes, bool kKeep>
 __device__ __forceinline__ void walk_steps(const RayView& V, int bx0, int by0, int bz0, float ox, float oy, float oz,
                                         float dx, float dy, float dz, float ix, float iy, float iz, int vx, int vy,
                                         int vz, float t, int ea, Trav& r) {
@@ -167,8 +171,8 @@ __device__ __forceinline__ void walk_steps(const RayView& V, int bx0, int by0, i
       const int sh = kCubes ? (int)__ldg(V.level + brick) - 3 : 0;
       if (sh > 2) {
         // an empty cube of 2^sh bricks on a side, unless that would pass the cap;
-        // smaller cubes are faster by the brick (the far view below 175 us, with
-        // cubes of 4 188, of 2 as well 197)
+        // smaller cubes are faster by the brick (the far view below, out of line: 175
+        // us, with cubes of 4 188, of 2 as well 197)
         const int mask = (1 << sh) - 1;
         const float tx = sx ? bound_time((((Bx >> sh) + px) << (sh + 3)) - bx0, ox, ix) : kInf;
         const float ty = sy ? bound_time((((By >> sh) + py) << (sh + 3)) - by0, oy, iy) : kInf;
@@ -228,28 +232,40 @@ __device__ __forceinline__ void walk_steps(const RayView& V, int bx0, int by0, i
     }
     // voxel steps inside occupied brick p
     const uint64_t* occ = V.occ + (size_t)p * 8;
+    uint64_t w = 0;
+    int nvx = 0, nvy = 0, nvz = 0;  // next voxel boundary (relative) along each axis, and its time
+    float tx = kInf, ty = kInf, tz = kInf;
+    auto look = [&] {
+      w = __ldg(occ + (vz & 7));
+      nvx = vx + px - bx0;
+      nvy = vy + py - by0;
+      nvz = vz + pz - bz0;
+      tx = sx ? bound_time(nvx, ox, ix) : kInf;
+      ty = sy ? bound_time(nvy, oy, iy) : kInf;
+      tz = sz ? bound_time(nvz, oz, iz) : kInf;
+    };
     bool left = false;
+    if (kKeep) look();
     for (;;) {
-      if ((__ldg(occ + (vz & 7)) >> ((vx & 7) + 8 * (vy & 7))) & 1ull) {
+      if (!kKeep) look();
+      if ((w >> ((vx & 7) + 8 * (vy & 7))) & 1ull) {
         r.hit = 1;
         break;
       }
-      const float tx = sx ? bound_time(vx + px - bx0, ox, ix) : kInf;
-      const float ty = sy ? bound_time(vy + py - by0, oy, iy) : kInf;
-      const float tz = sz ? bound_time(vz + pz - bz0, oz, iz) : kInf;
       const bool cy = ty < tx;
       float tm = cy ? ty : tx;
       const bool cz = tz < tm;
       tm = cz ? tz : tm;
-      const int a = cz ? 2 : (cy ? 1 : 0);
+      const bool a2 = cz, a1 = cy && !cz, a0 = !cy && !cz;
       fs++;
       t = tm;
-      ea = a;
-      vx += a == 0 ? sx : 0;
-      vy += a == 1 ? sy : 0;
-      vz += a == 2 ? sz : 0;
-      const int c = a == 0 ? vx : (a == 1 ? vy : vz);
-      const int cb = a == 0 ? Bx : (a == 1 ? By : Bz);
+      ea = a2 ? 2 : (a1 ? 1 : 0);
+      vx += a0 ? sx : 0;
+      vy += a1 ? sy : 0;
+      vz += a2 ? sz : 0;
+      if (kKeep && a2) w = __ldg(occ + (vz & 7));  // (a word of this brick, unused, where the step leaves it)
+      const int c = a0 ? vx : (a1 ? vy : vz);
+      const int cb = a0 ? Bx : (a1 ? By : Bz);
       if ((c >> 3) != cb) {
         Bx = vx >> 3;
         By = vy >> 3;
@@ -260,6 +276,15 @@ __device__ __forceinline__ void walk_steps(const RayView& V, int bx0, int by0, i
       if (cs + fs > cap) {
         left = true;
         break;
+      }
+      if (kKeep) {
+        nvx += a0 ? sx : 0;
+        nvy += a1 ? sy : 0;
+        nvz += a2 ? sz : 0;
+        const float tn = bound_time(a0 ? nvx : (a1 ? nvy : nvz), a0 ? ox : (a1 ? oy : oz), a0 ? ix : (a1 ? iy : iz));
+        tx = a0 ? tn : tx;
+        ty = a1 ? tn : ty;
+        tz = a2 ? tn : tz;
       }
     }
     if (r.hit || left) break;
@@ -281,7 +306,7 @@ template <bool kCubes>
 __device__ __noinline__ void walk_steps_apart(const RayView& V, int bx0, int by0, int bz0, float ox, float oy, float oz,
                                               float dx, float dy, float dz, float ix, float iy, float iz, int vx, int vy,
                                               int vz, float t, int ea, Trav& r) {
-  walk_steps<false, kCubes>(V, bx0, by0, bz0, ox, oy, oz, dx, dy, dz, ix, iy, iz, vx, vy, vz, t, ea, r);
+  walk_steps<false, kCubes, false>(V, bx0, by0, bz0, ox, oy, oz, dx, dy, dz, ix, iy, iz, vx, vy, vz, t, ea, r);
 }
 
 // ---------------------------------------------------------- region walk
@@ -553,12 +578,14 @@ __device__ __forceinline__ void walk_regions(const RayView& V, const RayAxis& X,
 }
 
 // Traces a ray by regions where its values allow, else step by step.
-template <bool kStats, bool kCubes>
+template <bool kStats, int kWalk>
 __device__ __forceinline__ void trace(const RayView& V, float margin, int bx0, int by0, int bz0, float ox, float oy,
                                       float oz, float dx, float dy, float dz, float ix, float iy, float iz, int vx,
                                       int vy, int vz, float t, int ea, Trav& r) {
   if constexpr (kStats) {
-    walk_steps<true, false>(V, bx0, by0, bz0, ox, oy, oz, dx, dy, dz, ix, iy, iz, vx, vy, vz, t, ea, r);
+    walk_steps<true, false, false>(V, bx0, by0, bz0, ox, oy, oz, dx, dy, dz, ix, iy, iz, vx, vy, vz, t, ea, r);
+  } else if constexpr (kWalk == kBySteps) {
+    walk_steps<false, true, true>(V, bx0, by0, bz0, ox, oy, oz, dx, dy, dz, ix, iy, iz, vx, vy, vz, t, ea, r);
   } else if (margin > 0.0f && regular_axis(dx) && regular_axis(dy) && regular_axis(dz) &&
              (dx != 0.0f || dy != 0.0f || dz != 0.0f)) {
     const int4 nlo = __ldg(V.bounds), hi = __ldg(V.bounds + 1);
@@ -567,7 +594,7 @@ __device__ __forceinline__ void trace(const RayView& V, float margin, int bx0, i
     walk_regions(V, X, Y, Z, margin, vx, vy, vz, t, ea, r);
   } else {
     Trav q;
-    walk_steps_apart<kCubes>(V, bx0, by0, bz0, ox, oy, oz, dx, dy, dz, ix, iy, iz, vx, vy, vz, t, ea, q);
+    walk_steps_apart<kWalk == kEither>(V, bx0, by0, bz0, ox, oy, oz, dx, dy, dz, ix, iy, iz, vx, vy, vz, t, ea, q);
     r = q;
   }
 }
@@ -593,7 +620,7 @@ __device__ __forceinline__ void camera_ray(const RayView& V, uint32_t px, uint32
   dz = __fdiv_rn(d2, len);
 }
 
-template <bool kStats, bool kCubes>
+template <bool kStats, int kWalk>
 __device__ __forceinline__ void trace_pixel(const RayView& V, uint32_t px, uint32_t py, const RayParams& P,
                                             meso_hit& h, uint32_t* st) {
   h.voxel = ~0ull;
@@ -677,7 +704,7 @@ __device__ __forceinline__ void trace_pixel(const RayView& V, uint32_t px, uint3
 #pragma unroll 1
   for (int pass = 0;; pass++) {
     Trav r;
-    trace<kStats, kCubes>(V, V.margin, base_x, base_y, base_z, rox, roy, roz, rdx, rdy, rdz, rix, riy, riz, vx, vy, vz,
+    trace<kStats, kWalk>(V, V.margin, base_x, base_y, base_z, rox, roy, roz, rdx, rdy, rdz, rix, riy, riz, vx, vy, vz,
                           t0, ea, r);
     if (kStats) {
       st[0] += r.fetches;
@@ -735,12 +762,16 @@ __device__ __forceinline__ void trace_pixel(const RayView& V, uint32_t px, uint3
 // idle warps), so the descriptor's index depends on the block alone and its
 // fields are read through the uniform path; one view's are operands in the
 // parameter bank, with no load at all.
-// kCubes: for launches with whole views, or a light, that the region walk does not
-// take; their rays cross empty cubes too.  1080p view of the 1024^3 terrain from
-// 140,000 voxels away: 342 us without, 175 so.  An instantiation of its own, as the
-// longer walk costs the other launches registers (256^2 view 30.7 us with one
-// instantiation for both 31.4, 40 served requests 4.16 and 4.20 ms).
-template <int kViews, int kMode, bool kCubes>
+// kWalk: kByRegion where the region walk takes all views (single rays that it does
+// not take step by the brick).  kBySteps where it takes none: views from beyond its
+// coordinates (1080p view of the 1024^3 terrain from 140,000 voxels away: 342 us by
+// the brick, 148 so) and of rough scenes (see set_rough), whose rays have no empty
+// space to skip (256^3 random voxels, 25 % solid, 1280x720 with shadow rays: 75 us
+// by region, 51 so).  kEither where the views or the shadow rays' light differ in
+// this; an instantiation of its own, as a step over cubes out of line costs the
+// region walk registers (256^2 view 30.7 us, and 31.4; 40 served requests 4.16 and
+// 4.20 ms).
+template <int kViews, int kMode, int kWalk>
 __global__ void __launch_bounds__(128, 8)
     raymarch_kernel(const RayParams P, const __grid_constant__ Views<kViews ? kViews : 1> iv) {
   constexpr bool kStats = kMode == kStatsMode;
@@ -780,7 +811,7 @@ __global__ void __launch_bounds__(128, 8)
   uint64_t* sw = stage[threadIdx.x >> 5];
   if (px < V.width && py < V.height) {
     meso_hit h;
-    trace_pixel<kStats, kCubes>(V, px, py, P, h, st);
+    trace_pixel<kStats, kWalk>(V, px, py, P, h, st);
     sw[3 * lane] = h.voxel;
     sw[3 * lane + 1] = (uint64_t)__float_as_uint(h.t) | (uint64_t)h.material << 32 | (uint64_t)h.face << 48 |
                        (uint64_t)h.shadow << 56;
@@ -906,7 +937,7 @@ static uint32_t block_tiles_shift(uint32_t wpc, bool rows) { return wpc == 4 ? (
 // Running totals over the views of a launch.
 struct ViewTotals {
   uint64_t tiles = 0, blocks = 0, hits = 0;
-  bool stepped = false;  // a view that the region walk does not take
+  uint32_t stepped = 0;  // views that the region walk does not take
 };
 
 // Fills the host descriptors out[0 .. n) of views scenes/cams[0 .. n) for
@@ -939,8 +970,9 @@ static void fill_views(const meso_scene* const* scenes, const meso_camera* cams,
     V.aspect = (float)c.width / (float)c.height;  // IEEE conversions and division, as on the device
     V.width = c.width;
     V.height = c.height;
-    V.margin = region_margin(s, c);
-    tot.stepped |= V.margin == 0.0f || !regular_axis(c.forward[0]) || !regular_axis(c.forward[1]) || !regular_axis(c.forward[2]);
+    V.margin = s->rough ? 0.0f : region_margin(s, c);
+    if (!regular_axis(c.forward[0]) || !regular_axis(c.forward[1]) || !regular_axis(c.forward[2])) V.margin = 0.0f;
+    tot.stepped += V.margin == 0.0f;
     V.block_start = (uint32_t)tot.blocks;
     V.out = view_out && view_out[v] ? view_out[v] : d_hits + tot.hits;
     const uint32_t tiles_x = (c.width + tw - 1) / tw, tiles_y = (c.height + th - 1) / th;
@@ -993,11 +1025,11 @@ static meso_status stage_view_table(const meso_scene* const* scenes, const meso_
 }
 
 // Launches one mode's kernel over the totals' blocks.
-template <int kViews, bool kCubes>
-static void launch_rays(const RayParams& P, const Views<kViews ? kViews : 1>& iv, uint32_t blocks, uint32_t wpc,
+template <int kViews, int kWalk>
+static void launch_walk(const RayParams& P, const Views<kViews ? kViews : 1>& iv, uint32_t blocks, uint32_t wpc,
                         cudaStream_t st) {
-  if (P.hash) raymarch_kernel<kViews, kHashMode, kCubes><<<blocks, wpc * 32, 0, st>>>(P, iv);
-  else raymarch_kernel<kViews, kPlain, kCubes><<<blocks, wpc * 32, 0, st>>>(P, iv);
+  if (P.hash) raymarch_kernel<kViews, kHashMode, kWalk><<<blocks, wpc * 32, 0, st>>>(P, iv);
+  else raymarch_kernel<kViews, kPlain, kWalk><<<blocks, wpc * 32, 0, st>>>(P, iv);
 }
 template <int kViews>
 static void launch_mode(const RayParams& P, const Views<kViews ? kViews : 1>& iv, const ViewTotals& tot, uint32_t wpc,
@@ -1005,9 +1037,10 @@ static void launch_mode(const RayParams& P, const Views<kViews ? kViews : 1>& iv
   const uint32_t blocks = (uint32_t)tot.blocks;
   const float* L = P.light;
   const bool light = regular_axis(L[0]) && regular_axis(L[1]) && regular_axis(L[2]) && (L[0] != 0.0f || L[1] != 0.0f || L[2] != 0.0f);
-  if (P.stats) raymarch_kernel<kViews, kStatsMode, false><<<blocks, wpc * 32, 0, st>>>(P, iv);
-  else if (tot.stepped || (P.shadow && !light)) launch_rays<kViews, true>(P, iv, blocks, wpc, st);
-  else launch_rays<kViews, false>(P, iv, blocks, wpc, st);
+  if (P.stats) raymarch_kernel<kViews, kStatsMode, kByRegion><<<blocks, wpc * 32, 0, st>>>(P, iv);
+  else if (tot.stepped == P.n_views) launch_walk<kViews, kBySteps>(P, iv, blocks, wpc, st);
+  else if (tot.stepped || (P.shadow && !light)) launch_walk<kViews, kEither>(P, iv, blocks, wpc, st);
+  else launch_walk<kViews, kByRegion>(P, iv, blocks, wpc, st);
 }
 
 meso_status launch_raymarch(meso_ctx* ctx, const meso_scene* const* scenes, const meso_camera* cams,

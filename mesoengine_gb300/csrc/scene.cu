@@ -98,6 +98,15 @@ __device__ __forceinline__ uint64_t sub_mask(const uint32_t (&w)[16]) {
   return m;
 }
 
+// Of the 8 squares of 2x2 voxels in 4 rows of 8 bits each: how many hold voxels and
+// are not solid, and 16 bits higher how many are not solid.
+__device__ __forceinline__ uint32_t square_counts(uint32_t rows) {
+  uint32_t some = rows | rows >> 8, solid = rows & rows >> 8;
+  some = (some | some >> 1) & 0x00550055u;
+  solid = solid & solid >> 1 & 0x00550055u;
+  return (uint32_t)__popc(some & ~solid) | (8u - (uint32_t)__popc(solid)) << 16;
+}
+
 // One warp per brick; lane covers voxels lane + 32k (x = i&7, y = (i>>3)&7, z = i>>6).
 template <bool kFill>
 __global__ void terrain_brick_kernel(TerrainDev T, const float* heights, const float* hmax, uint8_t* flags,
@@ -234,9 +243,19 @@ meso_status number_bricks(meso_ctx* ctx, const uint8_t* d_flags, uint64_t nb, ui
 // tile's words are on their way while this one is scanned.  (Three launches over
 // a byte per brick and a copy of the pointers took a build 14 us longer: 512^3
 // uint16 195 us and now 181, 256^3 89 and 72.)
+// It also adds up the sampled square_counts: total[1] and [2].
 __global__ void __launch_bounds__(kScanThreads) scan_words_kernel(const uint32_t* words, uint64_t n, uint32_t* base,
-                                                                  uint32_t* total) {
+                                                                  uint32_t* total, const uint32_t* squares,
+                                                                  uint32_t n_squares) {
   __shared__ uint32_t ws[32];
+  __shared__ uint32_t sums[2];
+  if (threadIdx.x < 2) sums[threadIdx.x] = 0;
+  uint32_t mixed = 0, open = 0;
+  for (uint32_t i = threadIdx.x; i < n_squares; i += kScanThreads) {
+    const uint32_t q = squares[i];
+    mixed += q & 0xFFFFu;
+    open += q >> 16;
+  }
   constexpr int kPer = 8;
   uint32_t carry = 0, v[kPer];
   auto load = [&](uint64_t i0) {
@@ -259,7 +278,15 @@ __global__ void __launch_bounds__(kScanThreads) scan_words_kernel(const uint32_t
       if (i0 + k < n) base[i0 + k] = ex + c[k];
     carry += all;
   }
-  if (threadIdx.x == 0) *total = carry;
+  __syncthreads();  // (sums are clear, with no tile too)
+  mixed = __reduce_add_sync(kFull, mixed);
+  open = __reduce_add_sync(kFull, open);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&sums[0], mixed);
+    atomicAdd(&sums[1], open);
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) total[threadIdx.x] = threadIdx.x ? sums[threadIdx.x - 1] : carry;
 }
 
 // ---------------------------------------------------------- dense -> bricks
@@ -317,11 +344,12 @@ __device__ __forceinline__ const T* brick_layer(const T* grid, int nx, int ny, u
 
 template <typename T, bool kWide>
 __global__ void __launch_bounds__(kDenseThreads) dense_flag_kernel(const T* grid, int nx, int ny, uint64_t nb,
-                                                                   uint32_t* occupied) {
-  __shared__ uint32_t any[kDenseThreads / 32];
+                                                                   uint32_t* occupied, uint32_t* squares, uint32_t step) {
+  __shared__ uint32_t any[kDenseThreads / 32], counts[kDenseThreads / 32];
   const int lane = threadIdx.x & 31, z = threadIdx.x >> 5;
   const uint64_t b = (uint64_t)blockIdx.x * kDenseBricks + lane;
-  uint32_t acc = 0;
+  const bool sample = blockIdx.x % step == 0;  // of the squares, every step-th block's
+  uint32_t acc = 0, q = 0;
   if (b < nb) {
     const T* src = brick_layer(grid, nx, ny, b, z);
     uint4 v[8];
@@ -329,15 +357,32 @@ __global__ void __launch_bounds__(kDenseThreads) dense_flag_kernel(const T* grid
     for (int y = 0; y < 8; y++) v[y] = load_row8<T, kWide, true>(src + (size_t)nx * y);
 #pragma unroll
     for (int y = 0; y < 8; y++) acc |= v[y].x | v[y].y | v[y].z | v[y].w;
+    if (sample) {
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        uint32_t rows = 0;
+#pragma unroll
+        for (int y = 0; y < 4; y++) rows |= row8_bits(v[4 * h + y]) << (8 * y);
+        q += square_counts(rows);
+      }
+    }
   }
   const uint32_t bits = __ballot_sync(kFull, acc != 0);
-  if (lane == 0) any[z] = bits;
+  if (sample) q = __reduce_add_sync(kFull, q);
+  if (lane == 0) {
+    any[z] = bits;
+    counts[z] = q;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
-    uint32_t m = 0;
+    uint32_t m = 0, n = 0;
 #pragma unroll
-    for (int k = 0; k < kDenseThreads / 32; k++) m |= any[k];
+    for (int k = 0; k < kDenseThreads / 32; k++) {
+      m |= any[k];
+      n += counts[k];
+    }
     occupied[blockIdx.x] = m;
+    if (sample) squares[blockIdx.x / step] = n;
   }
 }
 
@@ -734,21 +779,31 @@ __global__ void __launch_bounds__(kLevelThreads)
   }
 }
 
-// d_sub of `slots` consecutive pool slots, one thread each.
-__global__ void sub_kernel(const uint64_t* occ, uint64_t slots, uint64_t* sub) {
+// d_sub of `slots` consecutive pool slots, one thread each; their square_counts are
+// added to counts[0] and [1].
+__global__ void sub_kernel(const uint64_t* occ, uint64_t slots, uint64_t* sub, unsigned long long* counts) {
   const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= slots) return;
   const uint4* src = reinterpret_cast<const uint4*>(occ + p * 8);
   uint32_t w[16];
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    const uint4 v = src[k];
+    const uint4 v = p < slots ? src[k] : make_uint4(0, 0, 0, 0);
     w[4 * k] = v.x;
     w[4 * k + 1] = v.y;
     w[4 * k + 2] = v.z;
     w[4 * k + 3] = v.w;
   }
-  sub[p] = sub_mask(w);
+  uint32_t q = 0;
+  if (p < slots) {
+    sub[p] = sub_mask(w);
+#pragma unroll
+    for (int k = 0; k < 16; k++) q += square_counts(w[k]);
+  }
+  q = __reduce_add_sync(kFull, q);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(counts, (unsigned long long)(q & 0xFFFFu));
+    atomicAdd(counts + 1, (unsigned long long)(q >> 16));
+  }
 }
 
 // ---------------------------------------------------------------- scene API
@@ -871,11 +926,32 @@ meso_status rebuild_macro(meso_ctx* ctx, meso_scene* s, const uint32_t* d_cells,
   return MESO_OK;
 }
 
+// Of the squares of 2x2 voxels of z layers (all, or a sample) that are not solid
+// (`open`), `mixed` hold voxels.  A scene is rough if that is more than an eighth.
+// Its rays then walk step by step: so few regions are empty that leaving them one by
+// one costs more than the steps.  256^3 voxels, 1280x720 from outside, by region and
+// by steps: 2 % solid at random (0.08 of the squares) 225 and 249 us, 3 % (0.12) 185
+// and 182, 4 % (0.15) 158 and 146, 10 % (0.34) 87 and 69, 25 % (0.68) 48 and 35.
+// Terrains, caves, foliage and the generator's noise lie below 0.06.
+static void set_rough(meso_scene* s, uint64_t mixed, uint64_t open) { s->rough = 8 * mixed > open; }
+
 meso_status rebuild_sub(meso_ctx* ctx, meso_scene* s, uint64_t slots, cudaStream_t st) {
   if (slots == 0) return MESO_OK;
-  sub_kernel<<<(unsigned)((slots + 127) / 128), 128, 0, st>>>(s->d_occ, slots, s->d_sub);
-  ctx->launches.fetch_add(1);
-  MESO_CUDA_TRY(cudaGetLastError());
+  unsigned long long* d = nullptr;
+  unsigned long long counts[2] = {0, 0};
+  MESO_CUDA_TRY(dev_malloc_async(ctx, &d, sizeof(counts), st));
+  cudaError_t e = cudaMemsetAsync(d, 0, sizeof(counts), st);
+  if (e == cudaSuccess) {
+    sub_kernel<<<(unsigned)((slots + 127) / 128), 128, 0, st>>>(s->d_occ, slots, s->d_sub, d);
+    ctx->launches.fetch_add(1);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(counts, d, sizeof(counts), cudaMemcpyDeviceToHost, st);
+  cudaFreeAsync(d, st);
+  const cudaError_t e2 = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = e2;
+  if (e != cudaSuccess) return cuda_fail(e, "scene block masks");
+  set_rough(s, counts[0], counts[1] + (n_bricks_of(s) - slots) * 128);
   return MESO_OK;
 }
 
@@ -961,22 +1037,28 @@ static meso_status build_from_device_grid(meso_ctx* ctx, const T* d_grid, int32_
                                           uint64_t spare, cudaStream_t st, meso_scene** out) {
   const uint64_t nb = (uint64_t)nx * ny * nz / 512;
   const unsigned blocks = (unsigned)((nb + kDenseBricks - 1) / kDenseBricks);
-  uint32_t* d_occupied = nullptr;  // a word per block: which of its bricks hold anything; then their first slots, and the count
-  const cudaError_t ae = dev_malloc_async(ctx, &d_occupied, 8 * (size_t)blocks + 4, st);
+  // a word per block: which of its bricks hold anything; their first slots, and the
+  // count of bricks and of the sampled squares; the samples, about 1024
+  const uint32_t step = blocks / 1024u | 1u, n_squares = (blocks + step - 1) / step;
+  uint32_t* d_occupied = nullptr;
+  const cudaError_t ae = dev_malloc_async(ctx, &d_occupied, 8 * (size_t)blocks + 12 + 4 * (size_t)n_squares, st);
   if (ae != cudaSuccess) {
     cudaStreamSynchronize(st);
     return cuda_fail(ae, "dense scene: scratch allocation");
   }
   uint32_t* const d_base = d_occupied + blocks;
+  uint32_t* const d_total = d_base + blocks;
+  uint32_t* const d_squares = d_total + 3;
   const bool wide = (reinterpret_cast<uintptr_t>(d_grid) & (8 * sizeof(T) - 1)) == 0;
-  if (wide) dense_flag_kernel<T, true><<<blocks, kDenseThreads, 0, st>>>(d_grid, nx, ny, nb, d_occupied);
-  else dense_flag_kernel<T, false><<<blocks, kDenseThreads, 0, st>>>(d_grid, nx, ny, nb, d_occupied);
-  scan_words_kernel<<<1, kScanThreads, 0, st>>>(d_occupied, blocks, d_base, d_base + blocks);
+  if (wide) dense_flag_kernel<T, true><<<blocks, kDenseThreads, 0, st>>>(d_grid, nx, ny, nb, d_occupied, d_squares, step);
+  else dense_flag_kernel<T, false><<<blocks, kDenseThreads, 0, st>>>(d_grid, nx, ny, nb, d_occupied, d_squares, step);
+  scan_words_kernel<<<1, kScanThreads, 0, st>>>(d_occupied, blocks, d_base, d_total, d_squares, n_squares);
   ctx->launches.fetch_add(2);
-  uint32_t count = 0;
-  cudaError_t e = cudaMemcpyAsync(&count, d_base + blocks, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+  uint32_t totals[3] = {0, 0, 0};
+  cudaError_t e = cudaMemcpyAsync(totals, d_total, sizeof(totals), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   meso_status rc = e == cudaSuccess ? MESO_OK : cuda_fail(e, "dense scene build");
+  const uint32_t count = totals[0];
   meso_scene* s = nullptr;
   if (rc == MESO_OK) rc = alloc_sized(ctx, nx, ny, nz, count, spare, &s);
   if (rc == MESO_OK) {
@@ -987,6 +1069,7 @@ static meso_status build_from_device_grid(meso_ctx* ctx, const T* d_grid, int32_
       dense_fill_kernel<T, false><<<blocks, kDenseThreads, 0, st>>>(d_grid, nx, ny, nb, d_occupied, d_base, s->d_ptr, s->d_occ,
                                                                       s->d_mat, s->d_sub);
     ctx->launches.fetch_add(1);
+    set_rough(s, totals[1], totals[2]);
     rc = finish_pools(ctx, s, count, st);
   }
   cudaFreeAsync(d_occupied, st);
