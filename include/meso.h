@@ -285,9 +285,9 @@ typedef struct meso_hit {
  * Replaces the imposter draw (Samples/SimpleVoxel.cpp:374-393, vertex shader
  * :146-192).  light: normalised direction towards the light (MESO_RAY_SHADOW).
  * The walk is the two-level DDA (a coarse step per empty brick, a fine step
- * per voxel of an occupied brick); empty cells of 4^3, 16^3 and 64^3 bricks
- * are crossed in one jump whose result, step counts included, is that of the
- * brick-by-brick walk. */
+ * per voxel of an occupied brick).  Empty cubes of 2 voxels to 64 bricks on a
+ * side, and the space outside the bounds of what is occupied, are crossed in
+ * one step whose result, step counts included, is that of the walk. */
 meso_status meso_raymarch(meso_ctx* ctx, const meso_scene* const* scenes, const meso_camera* h_cams,
                           uint32_t n_views, const float light[3], uint32_t flags, meso_hit* d_hits,
                           void* stream);

@@ -55,7 +55,8 @@ constexpr int kArr = 32 * kS;
 constexpr int kFew = 2, kSome = 8;
 // Bytes per staged brick: two rows of each of four bricks side by side, what a
 // quarter of a warp loads at once, lie in 32 different banks (with 1040 one row
-// met another's: all chunks of the 1024^3 terrain 288.5 us, 283 now).
+// met another's: all chunks of the 1024^3 terrain 330 us, 324 so, back to back on
+// one box; 288 and 283 on a faster one).
 constexpr int kBrickSlot = 1056;
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 constexpr uint32_t kSideBytes = 32 * 32 * 16;  // the column of 16 bytes beside a grid chunk, for its X halo
@@ -953,7 +954,10 @@ meso_status launch_kind(meso_ctx* ctx, const MeshParams& base, const CUtensorMap
     // as soon as there are as many entries per CTA, and so: 4096 chunks at a
     // terrain's ground 209 and 170, 2500 of them 150 and 109, 1200 76 and 61, all
     // 8000 of a 640^3 terrain 130 and 104, all 32,768 of a 1024^3 one, 80 % of
-    // them air, 290 both; there tickets of 2, 4 and 16 take 311, 291 and 300.)
+    // them air, alike: 324, and with tickets of 2, 4 and 16 345, 328 and 333.  A
+    // list of nothing but air pays for its smaller tickets, 4096 entries 17 us
+    // after 8; larger ones after a ticket of air took a list of 4096 entries with
+    // one chunk in 20 from 37 to 43, with one in 5 from 60 to 68.)
     // 7919 and 104729 are primes, and no list of at most 2^20 entries is a
     // multiple of both, so t -> (t * perm_mul) mod n is a bijection
     const uint32_t b = n_chunks / (grid * 8u);
