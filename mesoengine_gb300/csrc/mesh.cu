@@ -55,8 +55,8 @@ constexpr int kArr = 32 * kS;
 constexpr int kFew = 2, kSome = 8;
 // Bytes per staged brick: two rows of each of four bricks side by side, what a
 // quarter of a warp loads at once, lie in 32 different banks (with 1040 one row
-// met another's: all chunks of the 1024^3 terrain 330 us, 324 so, back to back on
-// one box; 288 and 283 on a faster one).
+// met another's: all chunks of the 1024^3 terrain, launches back to back, 330 us
+// and 324 so; at another time 288 and 283).
 constexpr int kBrickSlot = 1056;
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 constexpr uint32_t kSideBytes = 32 * 32 * 16;  // the column of 16 bytes beside a grid chunk, for its X halo
